@@ -240,7 +240,7 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
 
     if (warp == 0) {
         // ------------------------------------------------------------------ weight stream
-        if (lane == 0) {
+        {
             ptx::prefetch_tensormap(&tm_packed);
             ptx::prefetch_tensormap(&tm_scale);
             if (DUAL) {
@@ -261,11 +261,13 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
                 while (hu < seg_end) {
                     const int cnt = (seg_end - hu) >= hps ? hps : 1;
                     ptx::mbar_wait(&empty_bar[stage], ph ^ 1u, s_abort, status, 0xA00u + (unsigned)stage);
-                    ptx::mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)(kPackedBytes + kScaleBytes) * cnt);
-                    for (int h = 0; h < cnt; ++h) {
-                        const int k0 = (kc + h) * kKC;
-                        ptx::tma_load_2d(s_w + (stage * hps + h) * kPackedBytes, mp, &full_bar[stage], k0 >> 1, row0, pol);
-                        ptx::tma_load_2d(s_raw + (stage * hps + h) * kScaleBytes, ms, &full_bar[stage], k0 >> 4, row0, pol);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)(kPackedBytes + kScaleBytes) * cnt);
+                        for (int h = 0; h < cnt; ++h) {
+                            const int k0 = (kc + h) * kKC;
+                            ptx::tma_load_2d(s_w + (stage * hps + h) * kPackedBytes, mp, &full_bar[stage], k0 >> 1, row0, pol);
+                            ptx::tma_load_2d(s_raw + (stage * hps + h) * kScaleBytes, ms, &full_bar[stage], k0 >> 4, row0, pol);
+                        }
                     }
                     hu += cnt;
                     kc += cnt;
@@ -276,21 +278,23 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
         }
     } else if (warp == 2) {
         // ------------------------------------------------------------------ resident activations (the pre-pass's output)
-        if (lane == 0 && !OWN) {
+        if (!OWN) {
             ptx::prefetch_tensormap(&tm_act);
             ptx::griddep_wait();
             const uint64_t pol = ptx::policy_evict_last();
-            ptx::mbar_arrive_expect_tx(&b_bar[0], (uint32_t)(p.slots * b_bytes));
-            const int kc0 = p.act_all ? 0 : kc_begin;
-            for (int j = 0; j < p.slots; ++j) {
-                int kc = kc0 + j;
-                if (kc >= p.kchunks) kc -= p.kchunks;
-                ptx::tma_load_2d(s_b + j * b_bytes, &tm_act, &b_bar[0], kc * (kKC / 2), 0, pol);
+            if (ptx::elect_one()) {
+                ptx::mbar_arrive_expect_tx(&b_bar[0], (uint32_t)(p.slots * b_bytes));
+                const int kc0 = p.act_all ? 0 : kc_begin;
+                for (int j = 0; j < p.slots; ++j) {
+                    int kc = kc0 + j;
+                    if (kc >= p.kchunks) kc -= p.kchunks;
+                    ptx::tma_load_2d(s_b + j * b_bytes, &tm_act, &b_bar[0], kc * (kKC / 2), 0, pol);
+                }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             const uint32_t idesc = fp4_idesc(p.NCp);
             ptx::mbar_wait(&b_bar[0], 0u, s_abort, status, 0xA10u);
             int stage = 0, acc = 0;
@@ -307,24 +311,26 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
                     const int cnt = (seg_end - hu) >= hps ? hps : 1;
                     ptx::mbar_wait(&sfa_bar[stage], ph, s_abort, status, 0xA30u + (unsigned)stage);
                     tc_fence_after();
-                    for (int h = 0; h < cnt; ++h) {
-                        const int slot = p.act_all ? kc + h : (hu - u_begin) + h;
-                        const uint32_t sfa_t = tmem_base + kSfCol + 32 * (uint32_t)(stage * hps + h), sfb_t = sfa_t + 16;
-                        const uint32_t a_addr = ptx::smem_u32(s_w + (stage * hps + h) * kPackedBytes);
-                        const uint32_t b_addr = ptx::smem_u32(s_b + slot * b_bytes);
+                    if (ptx::elect_one()) {
+                        for (int h = 0; h < cnt; ++h) {
+                            const int slot = p.act_all ? kc + h : (hu - u_begin) + h;
+                            const uint32_t sfa_t = tmem_base + kSfCol + 32 * (uint32_t)(stage * hps + h), sfb_t = sfa_t + 16;
+                            const uint32_t a_addr = ptx::smem_u32(s_w + (stage * hps + h) * kPackedBytes);
+                            const uint32_t b_addr = ptx::smem_u32(s_b + slot * b_bytes);
 #pragma unroll
-                        for (int s = 0; s < 4; ++s) {
-                            umma_fp4(d_tmem, umma_desc_sw128(a_addr + 32 * s), umma_desc_sw128(b_addr + 32 * s), idesc,
-                                     sfa_t + 4 * s, sfb_t + 4 * s, first ? 0u : 1u);
-                            first = false;
+                            for (int s = 0; s < 4; ++s) {
+                                umma_fp4(d_tmem, umma_desc_sw128(a_addr + 32 * s), umma_desc_sw128(b_addr + 32 * s), idesc,
+                                         sfa_t + 4 * s, sfb_t + 4 * s, (first && h == 0 && s == 0) ? 0u : 1u);
+                            }
                         }
+                        umma_commit(&empty_bar[stage]);        // the stage's codes and its scales in tensor memory are free once these MMAs have read them
                     }
-                    umma_commit(&empty_bar[stage]);        // the stage's codes and its scales in tensor memory are free once these MMAs have read them
+                    first = false;
                     hu += cnt;
                     kc += cnt;
                     if (++stage == stages) { stage = 0; ph ^= 1u; }
                 }
-                umma_commit(&tfull[acc]);
+                if (ptx::elect_one()) umma_commit(&tfull[acc]);
                 pt ^= 1u << acc;
                 acc ^= 1;
                 if (kc >= p.kchunks) kc = 0;

@@ -139,7 +139,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
 
     if (warp == 0) {
         // ------------------------------------------------------------------ weight stream
-        if (lane == 0) {
+        {
             ptx::prefetch_tensormap(&tm_packed);
             ptx::prefetch_tensormap(&tm_scale);
             const uint64_t pol = ptx::policy_evict_first();
@@ -153,11 +153,13 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
                 while (hu < seg_end) {
                     const int cnt = (seg_end - hu) >= hps ? hps : 1;
                     ptx::mbar_wait(&empty_bar[stage], ph ^ 1u, s_abort, status, 0xB00u + (unsigned)stage);
-                    ptx::mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)(kPackedBytes + kScaleBytes) * cnt);
-                    for (int h = 0; h < cnt; ++h) {
-                        const int k0 = (kc + h) * kKC;
-                        ptx::tma_load_2d(s_w + (stage * hps + h) * kPackedBytes, &tm_packed, &full_bar[stage], k0 >> 1, row0, pol);
-                        ptx::tma_load_2d(s_raw + (stage * hps + h) * kScaleBytes, &tm_scale, &full_bar[stage], k0 >> 4, row0, pol);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)(kPackedBytes + kScaleBytes) * cnt);
+                        for (int h = 0; h < cnt; ++h) {
+                            const int k0 = (kc + h) * kKC;
+                            ptx::tma_load_2d(s_w + (stage * hps + h) * kPackedBytes, &tm_packed, &full_bar[stage], k0 >> 1, row0, pol);
+                            ptx::tma_load_2d(s_raw + (stage * hps + h) * kScaleBytes, &tm_scale, &full_bar[stage], k0 >> 4, row0, pol);
+                        }
                     }
                     hu += cnt;
                     kc += cnt;
@@ -168,7 +170,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
         }
     } else if (warp == 2) {
         // ------------------------------------------------------------------ activation stream (the pre-pass's output, from L2)
-        if (lane == 0) {
+        {
             ptx::prefetch_tensormap(&tm_act);
             ptx::prefetch_tensormap(&tm_sfb);
             ptx::griddep_wait();                              // the pre-pass is the kernel before this one
@@ -182,10 +184,12 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
                 while (hu < seg_end) {
                     const int cnt = (seg_end - hu) >= hps ? hps : 1;
                     ptx::mbar_wait(&empty_bar[stage], ph ^ 1u, s_abort, status, 0xB10u + (unsigned)stage);
-                    ptx::mbar_arrive_expect_tx(&fullb_bar[stage], (uint32_t)(b_bytes + sfb_bytes) * cnt);
-                    for (int h = 0; h < cnt; ++h) {
-                        ptx::tma_load_2d(s_b + (stage * hps + h) * b_bytes, &tm_act, &fullb_bar[stage], (kc + h) * (kKC / 2), 0, pol);
-                        ptx::tma_load_2d(s_sfb + (stage * hps + h) * sfb_bytes, &tm_sfb, &fullb_bar[stage], 0, (kc + h) * p.groups, pol);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(&fullb_bar[stage], (uint32_t)(b_bytes + sfb_bytes) * cnt);
+                        for (int h = 0; h < cnt; ++h) {
+                            ptx::tma_load_2d(s_b + (stage * hps + h) * b_bytes, &tm_act, &fullb_bar[stage], (kc + h) * (kKC / 2), 0, pol);
+                            ptx::tma_load_2d(s_sfb + (stage * hps + h) * sfb_bytes, &tm_sfb, &fullb_bar[stage], 0, (kc + h) * p.groups, pol);
+                        }
                     }
                     hu += cnt;
                     kc += cnt;
@@ -196,7 +200,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             const uint32_t idesc = fp4_idesc(p.NCp);
             const uint32_t sf_col = 2u * (uint32_t)p.acc_stride;
             int stage = 0, acc = 0;
@@ -217,24 +221,26 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
                     ptx::mbar_wait(&full_bar[stage], ph, s_abort, status, 0xB30u + (unsigned)stage);
                     ptx::mbar_wait(&fullb_bar[stage], ph, s_abort, status, 0xB30u + (unsigned)stage);
                     tc_fence_after();
-                    for (int h = 0; h < cnt; ++h) {
-                        const int bslot = stage * hps + h;
-                        const uint32_t sfa_t = tmem_base + sf_col + 32 * (uint32_t)(stage * hps + h), sfb_t = sfa_t + 16;
-                        const uint32_t a_addr = ptx::smem_u32(s_w + (stage * hps + h) * kPackedBytes);
-                        const uint32_t b_addr = ptx::smem_u32(s_b + bslot * b_bytes);
+                    if (ptx::elect_one()) {
+                        for (int h = 0; h < cnt; ++h) {
+                            const int bslot = stage * hps + h;
+                            const uint32_t sfa_t = tmem_base + sf_col + 32 * (uint32_t)(stage * hps + h), sfb_t = sfa_t + 16;
+                            const uint32_t a_addr = ptx::smem_u32(s_w + (stage * hps + h) * kPackedBytes);
+                            const uint32_t b_addr = ptx::smem_u32(s_b + bslot * b_bytes);
 #pragma unroll
-                        for (int s = 0; s < 4; ++s) {
-                            umma_fp4(d_tmem, umma_desc_sw128(a_addr + 32 * s), umma_desc_sw128(b_addr + 32 * s), idesc,
-                                     sfa_t + 4 * s, sfb_t + 4 * s, first ? 0u : 1u);
-                            first = false;
+                            for (int s = 0; s < 4; ++s) {
+                                umma_fp4(d_tmem, umma_desc_sw128(a_addr + 32 * s), umma_desc_sw128(b_addr + 32 * s), idesc,
+                                         sfa_t + 4 * s, sfb_t + 4 * s, (first && h == 0 && s == 0) ? 0u : 1u);
+                            }
                         }
+                        umma_commit(&empty_bar[stage]);        // the stage's codes and its scales in tensor memory are free once these MMAs have read them
                     }
-                    umma_commit(&empty_bar[stage]);        // the stage's codes and its scales in tensor memory are free once these MMAs have read them
+                    first = false;
                     hu += cnt;
                     kc += cnt;
                     if (++stage == stages) { stage = 0; ph ^= 1u; }
                 }
-                umma_commit(&tfull[acc]);
+                if (ptx::elect_one()) umma_commit(&tfull[acc]);
                 pt ^= 1u << acc;
                 acc ^= 1;
                 if (kc >= p.kchunks) kc = 0;

@@ -224,7 +224,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             ptx::prefetch_tensormap(&tm_act);
             ptx::prefetch_tensormap(&tm_packed);
             ptx::prefetch_tensormap(&tm_scale);
@@ -238,22 +238,28 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 for (int ks = sg.ks0; ks < sg.ks1; ++ks) {
                     if (!DENSE) {
                         ptx::mbar_wait(&wempty[sw], pw ^ 1u, s_abort, p.status, 0x410u + sw);
-                        ptx::mbar_arrive_expect_tx(&wfull[sw], kWPackedBytes + kWScaleBytes);
-                        ptx::tma_load_2d(s_wp + sw * kWPackedBytes, &tm_packed, &wfull[sw], ks * (WK / 2), nt * BN, pol_w);
-                        ptx::tma_load_2d(s_ws + sw * kWScaleBytes, &tm_scale, &wfull[sw], ks * (WK / 16), nt * BN, pol_w);
+                        if (ptx::elect_one()) {
+                            ptx::mbar_arrive_expect_tx(&wfull[sw], kWPackedBytes + kWScaleBytes);
+                            ptx::tma_load_2d(s_wp + sw * kWPackedBytes, &tm_packed, &wfull[sw], ks * (WK / 2), nt * BN, pol_w);
+                            ptx::tma_load_2d(s_ws + sw * kWScaleBytes, &tm_scale, &wfull[sw], ks * (WK / 16), nt * BN, pol_w);
+                        }
                         if (++sw == kWStages) { sw = 0; pw ^= 1u; }
                     }
                     for (int j = 0; j < WK / BK; ++j) {
                         if (DENSE) {      // the B block of this 64-k step, as the tensor core wants it
                             ptx::mbar_wait(&bempty[sb], pb ^ 1u, s_abort, p.status, 0x410u + sb);
-                            ptx::mbar_arrive_expect_tx(&bfull[sb], kBBytes);
-                            ptx::tma_load_2d(s_b + sb * kBBytes, &tm_packed, &bfull[sb], ks * WK + j * BK, nt * BN, pol_w);
+                            if (ptx::elect_one()) {
+                                ptx::mbar_arrive_expect_tx(&bfull[sb], kBBytes);
+                                ptx::tma_load_2d(s_b + sb * kBBytes, &tm_packed, &bfull[sb], ks * WK + j * BK, nt * BN, pol_w);
+                            }
                             if (++sb == NB) { sb = 0; pb ^= 1u; }
                         }
                         for (int i = 0; i < sg.pair; ++i) {       // one activation tile per token tile of the pair
                             ptx::mbar_wait(&aempty[sa], pa ^ 1u, s_abort, p.status, 0x400u + sa);
-                            ptx::mbar_arrive_expect_tx(&afull[sa], kABytes);
-                            ptx::tma_load_2d(s_a + sa * kABytes, &tm_act, &afull[sa], ks * WK + j * BK, (mt + i) * BM, pol_a);
+                            if (ptx::elect_one()) {
+                                ptx::mbar_arrive_expect_tx(&afull[sa], kABytes);
+                                ptx::tma_load_2d(s_a + sa * kABytes, &tm_act, &afull[sa], ks * WK + j * BK, (mt + i) * BM, pol_a);
+                            }
                             if (++sa == kAStages) { sa = 0; pa ^= 1u; }
                         }
                     }
@@ -262,7 +268,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             // A pair of token tiles shares every dequantised B block: eight MMAs per 64-k block instead
             // of four for the same shared-memory fill, into both accumulators at once.  Single tiles
             // alternate between the two accumulators so that the epilogue of one overlaps the next.
@@ -284,19 +290,21 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                         ptx::mbar_wait(&afull[sa], pa, s_abort, p.status, 0x420u + sa);
                         const uint32_t a_addr = ptx::smem_u32(s_a + sa * kABytes);
                         const uint32_t d_tmem = tmem_base + (uint32_t)(acc0 + i) * BN;
+                        if (ptx::elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k) {
-                            umma_f16(d_tmem, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32),
-                                     (kb > 0 || k > 0) ? 1u : 0u, DENSE ? kInstrDescBf16 : kInstrDesc);
+                            for (int k = 0; k < BK / 16; ++k) {
+                                umma_f16(d_tmem, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32),
+                                         (kb > 0 || k > 0) ? 1u : 0u, DENSE ? kInstrDescBf16 : kInstrDesc);
+                            }
+                            umma_commit(&aempty[sa]);  // operand buffers are free once these MMAs have read them
                         }
-                        umma_commit(&aempty[sa]);  // operand buffers are free once these MMAs have read them
                         if (++sa == kAStages) { sa = 0; pa ^= 1u; }
                     }
-                    umma_commit(&bempty[sb]);
+                    if (ptx::elect_one()) umma_commit(&bempty[sb]);
                     if (++sb == NB) { sb = 0; pb ^= 1u; }
                 }
                 for (int i = 0; i < sg.pair; ++i) {
-                    umma_commit(&tfull[acc0 + i]);  // accumulator complete
+                    if (ptx::elect_one()) umma_commit(&tfull[acc0 + i]);  // accumulator complete
                     ptbits ^= 1u << (acc0 + i);
                 }
                 if (sg.pair == 1) next_acc ^= 1;

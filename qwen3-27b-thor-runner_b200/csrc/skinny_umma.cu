@@ -31,11 +31,10 @@
 // exact dequantised weights, BF16 activations, FP32 accumulation, one multiplication by
 // 1/global_scale, residual added in FP32 before the only rounding.
 //
-// Measured on B200 (gate_up 34816 x 5120): 43-50 us for 1..64 tokens, flat in M.  The issuing
-// thread sustains one tcgen05.mma with a TMEM A operand (128 x N x 16) per ~137 clocks whatever N
-// is, i.e. ~1.1 us per 128-row x 256-k stage, so the kernel streams weights at ~2.3 TB/s: slower
-// than the register-fed mma.sync GEMV for M <= 8 (26-30 us), faster than two GEMV launches or
-// the 128-token-tile GEMM between them.  kind::f16 takes both operands in ONE 16-bit format:
+// Measured on B200 (an MLP of 5120 x 17408, 40 tokens, norm + gate_up + SwiGLU + down): 72.1 us, 94.8 us while the MMAs
+// were issued behind `lane == 0`.  The issue rate was the bound: one tcgen05.mma (128 x N x 16) per ~111-137 clocks
+// whatever N is; behind elect.sync (ptx::elect_one) it is one per 51 clocks up to N = 64 (2048 weights, 6.4 TB/s of
+// packed weights over the chip) and 68 at N = 128.  kind::f16 takes both operands in ONE 16-bit format:
 // an instruction descriptor with A = FP16 and B = BF16 raises an illegal-instruction fault,
 // hence the FP16 activation copy.
 //
@@ -195,7 +194,7 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------------------------------------------ weight stream
-        if (lane == 0) {
+        {
             ptx::prefetch_tensormap(&tm_packed);
             ptx::prefetch_tensormap(&tm_scale);
             const uint64_t pol = ptx::policy_evict_first();
@@ -206,16 +205,18 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
             while (sched.next(sg)) {
                 for (int ks = sg.ks0; ks < sg.ks1; ++ks) {
                     ptx::mbar_wait(&wempty[sw], pw ^ 1u, s_abort, p.status, 0x510u + sw);
-                    ptx::mbar_arrive_expect_tx(&wfull[sw], kWPackedBytes + kWScaleBytes);
-                    ptx::tma_load_2d(s_wp + sw * kWPackedBytes, &tm_packed, &wfull[sw], ks * (WK / 2), sg.tile * TR, pol);
-                    ptx::tma_load_2d(s_ws + sw * kWScaleBytes, &tm_scale, &wfull[sw], ks * (WK / 16), sg.tile * TR, pol);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(&wfull[sw], kWPackedBytes + kWScaleBytes);
+                        ptx::tma_load_2d(s_wp + sw * kWPackedBytes, &tm_packed, &wfull[sw], ks * (WK / 2), sg.tile * TR, pol);
+                        ptx::tma_load_2d(s_ws + sw * kWScaleBytes, &tm_scale, &wfull[sw], ks * (WK / 16), sg.tile * TR, pol);
+                    }
                     if (++sw == p.w_stages) { sw = 0; pw ^= 1u; }
                 }
             }
         }
     } else if (warp == 2) {
         // ------------------------------------------------------------------ activation stream
-        if (lane == 0) {
+        {
             ptx::prefetch_tensormap(&tm_act);
             ptx::griddep_wait();           // the activations are the preceding kernel's output
             const uint64_t pol = ptx::policy_evict_last();
@@ -226,17 +227,19 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
             while (sched.next(sg)) {
                 for (int ks = sg.ks0; ks < sg.ks1; ++ks) {
                     ptx::mbar_wait(&xempty[sx], px ^ 1u, s_abort, p.status, 0x500u + sx);
-                    ptx::mbar_arrive_expect_tx(&xfull[sx], (uint32_t)xbytes);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(&xfull[sx], (uint32_t)xbytes);
 #pragma unroll
-                    for (int j = 0; j < WK / BK; ++j)
-                        ptx::tma_load_2d(s_x + sx * xbytes + j * (p.NT * 128), &tm_act, &xfull[sx], ks * WK + j * BK, 0, pol);
+                        for (int j = 0; j < WK / BK; ++j)
+                            ptx::tma_load_2d(s_x + sx * xbytes + j * (p.NT * 128), &tm_act, &xfull[sx], ks * WK + j * BK, 0, pol);
+                    }
                     if (++sx == p.x_stages) { sx = 0; px ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
             int sx = 0, au = 0, acc = 0;
             uint32_t px = 0, pa = 0, pt = 0;
             Schedule sched(p.sk_tiles, p.row_tiles, kstages);
@@ -253,20 +256,22 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
                         ptx::mbar_wait(&afull[au], pa, s_abort, p.status, 0x530u + au);
                         tc_fence_after();
                         const uint32_t a_tmem = tmem_base + (uint32_t)(p.a_col0 + au * kAUnitCols);
+                        if (ptx::elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < kAUnitK / 16; ++k) {
-                            const int kk = h * (kAUnitK / 16) + k;      // 16-k step inside the stage
-                            // 64-k block kk/4 of the stage (NT x 128 B each), 32 bytes per step inside it
-                            const uint64_t bdesc = xdesc + (uint64_t)(((kk >> 2) * (p.NT * 128) + (kk & 3) * 32) >> 4);
-                            umma_f16_ts(d_tmem, a_tmem + k * 8, bdesc, p.idesc, (ks > sg.ks0 || kk > 0) ? 1u : 0u);
+                            for (int k = 0; k < kAUnitK / 16; ++k) {
+                                const int kk = h * (kAUnitK / 16) + k;      // 16-k step inside the stage
+                                // 64-k block kk/4 of the stage (NT x 128 B each), 32 bytes per step inside it
+                                const uint64_t bdesc = xdesc + (uint64_t)(((kk >> 2) * (p.NT * 128) + (kk & 3) * 32) >> 4);
+                                umma_f16_ts(d_tmem, a_tmem + k * 8, bdesc, p.idesc, (ks > sg.ks0 || kk > 0) ? 1u : 0u);
+                            }
+                            umma_commit(&aempty[au]);  // the A unit is free once these MMAs have read it
                         }
-                        umma_commit(&aempty[au]);  // the A unit is free once these MMAs have read it
                         if (++au == p.a_units) { au = 0; pa ^= 1u; }
                     }
-                    umma_commit(&xempty[sx]);
+                    if (ptx::elect_one()) umma_commit(&xempty[sx]);
                     if (++sx == p.x_stages) { sx = 0; px ^= 1u; }
                 }
-                umma_commit(&tfull[acc]);
+                if (ptx::elect_one()) umma_commit(&tfull[acc]);
                 if (++acc == kAccs) { acc = 0; pt ^= 1u; }
             }
         }
