@@ -11,11 +11,14 @@
 namespace nvfp4 {
 namespace {
 
-// One CTA per token.
+constexpr int kHeld = 4;       // 16-byte vectors a thread keeps between the two steps
+
+// One CTA per token.  Latency-bound: the row is read once (all loads of a thread in flight together) and stays in registers
+// between the row maximum and the conversion; rows beyond kHeld x blockDim vectors are read again for the rest.
 __global__ void __launch_bounds__(1024)
 act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out, float* __restrict__ unscale, int K) {
     __shared__ unsigned int s_max;
-    const int m = blockIdx.x;
+    const int m = blockIdx.x, nv = K / 8;
     const uint4* src = reinterpret_cast<const uint4*>(A + (size_t)m * K);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)m * K);
     if (threadIdx.x == 0) s_max = 0u;
@@ -23,12 +26,20 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
     ptx::griddep_wait();                   // A is the output of the kernel before this one
     __syncthreads();
     unsigned int amax = 0;
-    for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-        const uint4 x = __ldg(src + i);
+    auto largest = [&](const uint4& x) {
         const uint32_t v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) amax = max(amax, max(v[q] & 0x7FFFu, (v[q] >> 16) & 0x7FFFu));
+    };
+    uint4 held[kHeld];
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        held[j] = i < nv ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
     }
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) largest(held[j]);
+    for (int i = threadIdx.x + kHeld * blockDim.x; i < nv; i += blockDim.x) largest(__ldg(src + i));
     amax = __reduce_max_sync(0xffffffffu, amax);
     if ((threadIdx.x & 31) == 0 && amax) atomicMax(&s_max, amax);
     __syncthreads();
@@ -36,15 +47,20 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
     se = se < 1 ? 1 : (se > 254 ? 254 : se);
     const float sc = __uint_as_float((uint32_t)se << 23);
     if (threadIdx.x == 0) unscale[m] = __uint_as_float((uint32_t)(254 - se) << 23);
-    for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-        const uint4 x = __ldg(src + i);
+    auto convert = [&](const uint4& x, int i) {
         const uint32_t v[4] = {x.x, x.y, x.z, x.w};
         uint32_t y[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             y[q] = ptx::pack_f16x2(__uint_as_float(v[q] << 16) * sc, __uint_as_float(v[q] & 0xFFFF0000u) * sc);
         dst[i] = make_uint4(y[0], y[1], y[2], y[3]);
+    };
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < nv) convert(held[j], i);
     }
+    for (int i = threadIdx.x + kHeld * blockDim.x; i < nv; i += blockDim.x) convert(__ldg(src + i), i);
 }
 
 }  // namespace
@@ -52,7 +68,10 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
 cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(M);
-    cfg.blockDim = dim3(M <= 32 ? 1024 : 256);     // few tokens: latency matters, use the whole SM
+    // as many threads as hold the row in kHeld vectors each; few tokens: half as many vectors (latency, SMs to spare)
+    const int per = M <= 148 ? kHeld / 2 : kHeld;
+    int threads = ((K / 8 + per - 1) / per + 31) / 32 * 32;
+    cfg.blockDim = dim3(threads < 64 ? 64 : (threads > 1024 ? 1024 : threads));
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
