@@ -62,6 +62,7 @@ struct nvfp4_device_info {
     int skinny_split_cost = 12;  // stage-times charged to splitting row tiles by k in the few-token kernel
     int fp4_own_quant = 1;       // one or two tokens: the tensor-core GEMV expands its activations itself, no pre-pass launch
     size_t gemv_pairs_offset = 6u << 20;   // where the 8-token GEMV's {value, epoch} partial pairs start in its scratch
+    int max_pairs = 0;                     // CTA pairs of the prefill kernel the device can hold at once (set at creation)
     TensorMapCache* maps = nullptr;        // null: encode every time
 };
 
@@ -101,7 +102,7 @@ struct DenseArgs {
 bool dense_gemv_supported(const DenseArgs& a, const nvfp4_device_info& dev);
 cudaError_t configure_dense_gemv();
 cudaError_t launch_dense_gemv(const DenseArgs& a, nvfp4_device_info& dev, void* scratch, int* launches, cudaStream_t s);
-// --- prefill_umma.cu, BF16 weights: the tcgen05 GEMM without the dequantisation (K % 256 == 0, N % 8 == 0).
+// --- prefill_pair.cu, BF16 weights: the tcgen05 GEMM without the dequantisation (K % 256 == 0, N % 8 == 0).
 bool dense_umma_supported(const DenseArgs& a);
 size_t dense_umma_scratch_bytes();
 cudaError_t launch_dense_umma(const DenseArgs& a, nvfp4_device_info& dev, void* scratch, size_t scratch_bytes, size_t offset,
@@ -177,7 +178,7 @@ cudaError_t launch_decode_fp4_stream(const LinearArgs& a, nvfp4_device_info& dev
 // --- act_f16.cu: BF16 activations -> FP16 copy with an exact per-token power-of-two scale; unscale[m] = 1/scale.
 cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, cudaStream_t s);
 
-// --- prefill_umma.cu: fused dequant + tcgen05 BF16 GEMM with TMEM accumulators.
+// --- prefill_pair.cu: fused dequant + tcgen05 GEMM on pairs of SMs, weights expanded into tensor memory.
 bool prefill_umma_supported(const LinearArgs& a);
 size_t prefill_umma_reserved_bytes();   // flags + partial tiles at the start of the kernel's scratch
 size_t prefill_umma_scratch_bytes(int max_M, int max_N, int max_K);
@@ -199,6 +200,6 @@ cudaError_t configure_skinny_umma();
 cudaError_t launch_skinny_umma(const LinearArgs& a, nvfp4_device_info& dev, void* scratch, size_t scratch_bytes,
                                size_t offset, int* launches, cudaStream_t s);
 
-cudaError_t configure_kernels(const nvfp4_device_info& dev);
+cudaError_t configure_kernels(nvfp4_device_info& dev);
 
 }  // namespace nvfp4

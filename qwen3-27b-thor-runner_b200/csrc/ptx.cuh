@@ -64,6 +64,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+// One look, never suspends.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait.  `abort_flag` lives in shared memory: once any thread of the CTA has timed
 // out, every later wait returns at once.  Budget ~2e9 clocks (about a second).
 constexpr long long kWaitBudgetClocks = 2000000000LL;
@@ -104,6 +117,39 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, ui
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
         "[%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_u32(smem_dst)),
         "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(policy)
+        : "memory");
+}
+
+// ---------------------------------------------------------------- CTA pairs (clusters of two)
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Every thread of both CTAs arrives and waits; ends whatever the other side does, since no thread skips it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The shared::cluster address of this CTA's shared-memory address `addr` in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
+    uint32_t d;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
+    return d;
+}
+// Arrives on a barrier of either CTA of the cluster.  No memory of the generic proxy is handed over with it (what the two
+// CTAs share is tensor memory, ordered by the tcgen05 fences and waits, and what TMA wrote), so the default scope is
+// enough; release / acquire at cluster scope cost a fence per arrival and wait: 2000 instead of 500 clocks per
+// dequantised 64-k block, measured.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Tiled load into this CTA's shared memory that reports to a barrier of either CTA of the pair (no multicast).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int x, int y,
+                                                 uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint "
+        "[%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_u32(smem_dst)),
+        "l"(tmap), "r"(bar_cluster_addr), "r"(x), "r"(y), "l"(policy)
         : "memory");
 }
 

@@ -13,41 +13,21 @@ namespace nvfp4 {
 namespace umma {
 
 // Work of one CTA: first its share of the stream-K region (tiles [0, sk_tiles), cut into
-// (tile, stage) units and split evenly over the CTAs), then whole tiles (or pairs of tiles)
-// blockIdx.x + i * gridDim.x behind that region.  The interleaved order keeps the CTAs that share
-// a weight tile in step, so the tile is fetched from HBM once and read from L2 by the others.
-// Every role walks the same list.
+// (tile, stage) units and split evenly over the CTAs), then whole tiles blockIdx.x + i * gridDim.x
+// behind that region.  Every role walks the same list.
 struct Segment {
     int tile, ks0, ks1;
-    int pair;     // 1, or 2: tiles `tile` and `tile + 1` (same weight rows, consecutive token tiles) over the whole k range
 };
 struct Schedule {
     long long u, u_end;
     int dp, dp_end, kstages;
-    int m_tiles, pairs_per_nt;        // pairs_per_nt == 0: whole tiles are handed out one by one
-    // Whole tiles one by one: tiles [0, sk_tiles) are the stream-K region.
     __device__ __forceinline__ Schedule(int sk_tiles, int tiles, int kst) {
-        init_sk(sk_tiles, kst);
-        dp = sk_tiles + blockIdx.x;
-        dp_end = tiles;
-        m_tiles = 1;
-        pairs_per_nt = 0;
-    }
-    // Whole tiles in pairs of consecutive token tiles of one weight tile (the last pair of a
-    // weight tile is a single when m_tiles is odd); the pairs [0, sk_pairs) -- tiles [0, sk_tiles)
-    // -- are the stream-K region, handled tile by tile.
-    __device__ __forceinline__ Schedule(int sk_tiles, int sk_pairs, int m_tiles_, int n_tiles, int kst) {
-        init_sk(sk_tiles, kst);
-        m_tiles = m_tiles_;
-        pairs_per_nt = (m_tiles_ + 1) / 2;
-        dp = sk_pairs + blockIdx.x;
-        dp_end = n_tiles * pairs_per_nt;
-    }
-    __device__ __forceinline__ void init_sk(int sk_tiles, int kst) {
         const long long sk_units = (long long)sk_tiles * kst;
         u = (long long)blockIdx.x * sk_units / gridDim.x;
         u_end = (long long)(blockIdx.x + 1) * sk_units / gridDim.x;
         kstages = kst;
+        dp = sk_tiles + blockIdx.x;
+        dp_end = tiles;
     }
     __device__ __forceinline__ bool next(Segment& s) {
         if (u < u_end) {
@@ -55,19 +35,11 @@ struct Schedule {
             s.ks0 = (int)(u % kstages);
             const long long room = u_end - u;
             s.ks1 = (kstages - s.ks0) < room ? kstages : s.ks0 + (int)room;
-            s.pair = 1;
             u += s.ks1 - s.ks0;
             return true;
         }
         if (dp < dp_end) {
-            if (pairs_per_nt == 0) {
-                s.tile = dp;
-                s.pair = 1;
-            } else {
-                const int nt = dp / pairs_per_nt, mp = dp - nt * pairs_per_nt;
-                s.tile = nt * m_tiles + 2 * mp;
-                s.pair = m_tiles - 2 * mp >= 2 ? 2 : 1;
-            }
+            s.tile = dp;
             s.ks0 = 0;
             s.ks1 = kstages;
             dp += gridDim.x;
@@ -94,19 +66,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ void tmem_alloc_512(uint32_t* smem_slot) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  ::"r"(ptx::smem_u32(smem_slot)), "r"(512) : "memory");

@@ -1,0 +1,83 @@
+"""The prefill GEMM on pairs of SMs: sizes at the edges of its token tiles (multiples of 32 up to 192), row tiles (256 per
+pair, an odd number of them leaves half an item), 256-k stages and split tiles, through every output form."""
+import numpy as np
+import pytest
+
+import oracle_binding as ob
+import util
+
+pytestmark = pytest.mark.gpu
+
+# Relative Frobenius error against the oracle's exact-weight arithmetic (GEMV mode): both round the same FP32 sums once, in
+# another order.  (Its GEMM mode rounds weights / global_scale to BF16, 2^-9 each: 1.5e-3 and more when the scale is not 1.)
+TOL = 1e-3
+
+
+def run(h, A, packed, scale, gs, residual=None):
+    import torch
+    M, K = A.shape
+    N = packed.shape[0]
+    dC = torch.full((M, N), 0x7FC0, dtype=torch.int16, device="cuda")   # NaN canary
+    dR = util.to_dev(residual) if residual is not None else None
+    h.linear(util.to_dev(A), M, util.to_dev(packed), util.to_dev(scale), gs, N, K, dC, residual=dR)
+    torch.cuda.synchronize()
+    return util.to_host_u16(dC)
+
+
+@pytest.mark.parametrize("M,N,K,res", [
+    (65, 8, 256, True),           # one short row tile, one stage: every wait is a first phase
+    (96, 264, 512, False),        # two row tiles, the second of 8 rows
+    (97, 768, 256, True),         # three row tiles
+    (160, 5376, 512, False),      # 21 row tiles: the last item has one
+    (161, 1280, 1024, True),      # one token in the last tile
+    (193, 2048, 2816, False),     # split along k
+    (385, 520, 4352, True),       # ragged rows, split tiles of a few tokens
+    (2500, 2816, 256, False),     # many items of one stage: the rings run across items
+    (1300, 5120, 768, True),      # whole items behind split ones
+])
+def test_pair_kernel_vs_oracle(handle, M, N, K, res):
+    packed, scale = util.make_weight(N, K, seed=M + N, sigma=0.14)
+    A = util.make_bf16((M, K), seed=M + 5)
+    R = util.make_bf16((M, N), seed=N + 6) if res else None
+    got = run(handle, A, packed, scale, 1.7, residual=R)
+    for _ in range(3):
+        assert np.array_equal(got, run(handle, A, packed, scale, 1.7, residual=R))   # fixed summation order
+    assert ob.rel_frobenius(got, ob.linear(A, packed, scale, 1.7, residual=R, mode=ob.GEMV, threads=8)) <= TOL
+    assert handle.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 96, 256), (150, 5120, 2560), (333, 1024, 4352)])
+def test_swiglu_output_equals_linear_and_swiglu(handle, M, N, K):
+    """Interleaved rows (8 gate, 8 up): the SwiGLU of the plain call's rounded outputs, also across split tiles."""
+    import torch
+    packed, scale = util.make_weight(N, K, seed=M, sigma=0.14)
+    A = util.make_bf16((M, K), seed=M + 1)
+    dA, dp, ds = util.to_dev(A), util.to_dev(packed), util.to_dev(scale)
+    plain = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    out = torch.empty((M, N // 2), dtype=torch.bfloat16, device="cuda")
+    handle.linear(dA, M, dp, ds, 1.0, N, K, plain)
+    handle.linear_ex(dA, M, dp, ds, 1.0, N, K, out, swiglu_epilogue=True)
+    slabs = plain.float().view(M, N // 16, 2, 8)
+    gate, up = slabs[:, :, 0].reshape(M, -1), slabs[:, :, 1].reshape(M, -1)
+    want = (gate / (1 + torch.exp(-gate)) * up).to(torch.bfloat16)
+    # same sums, so at most one BF16 step where the two exponentials round differently: 2^-8 of the value
+    assert torch.allclose(out.float(), want.float(), rtol=2 ** -7, atol=1e-30)
+    assert handle.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 8, 256), (33, 776, 256), (161, 2816, 512), (512, 5120, 1280), (700, 264, 2560)])
+def test_bf16_weights_vs_oracle(handle, M, N, K):
+    import torch
+    W = util.make_bf16((N, K), seed=N + 1, std=0.05)
+    A = util.make_bf16((M, K), seed=M + 3)
+    dA, dW = util.to_dev(A), util.to_dev(W)
+    outs = []
+    for _ in range(8):
+        dC = torch.full((M, N), 0x7FC0, dtype=torch.int16, device="cuda")
+        handle.linear_bf16(dA, M, dW, N, K, dC)
+        outs.append(dC)
+    torch.cuda.synchronize()
+    got = util.to_host_u16(outs[0])
+    assert all(np.array_equal(got, util.to_host_u16(o)) for o in outs[1:])
+    assert ob.rel_frobenius(got, ob.dense_linear(A, W)) <= TOL
+    assert handle.device_status() == 0
