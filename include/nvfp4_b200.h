@@ -63,7 +63,9 @@ typedef struct nvfp4_quantized_weight {
  * device, workspace sized once at creation. */
 int nvfp4_create(int device, size_t workspace_bytes, nvfp4_handle** out);
 int nvfp4_destroy(nvfp4_handle* h);
-/* Workspace needed so that every call with M<=max_M, N<=max_N, K<=max_K succeeds. */
+/* Workspace needed so that every call with M<=max_M, N<=max_N, K<=max_K succeeds.  For max_M <= 16 it leaves out
+ * the ~40 MB of the tcgen05 GEMM, which so few tokens reach only through options ("gemm_weight_rounding" = 1, or a
+ * "decode_max_m" below their count): such a call returns NVFP4_E_WORKSPACE.  Ask for max_M = 17 to make room for it. */
 int nvfp4_workspace_bytes(int max_M, int max_N, int max_K, size_t* bytes);
 const char* nvfp4_status_string(int status);
 

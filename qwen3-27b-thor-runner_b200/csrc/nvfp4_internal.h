@@ -181,7 +181,7 @@ cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float*
 // --- prefill_pair.cu: fused dequant + tcgen05 GEMM on pairs of SMs, weights expanded into tensor memory.
 bool prefill_umma_supported(const LinearArgs& a);
 size_t prefill_umma_reserved_bytes();   // flags + partial tiles at the start of the kernel's scratch
-size_t prefill_umma_scratch_bytes(int max_M, int max_N, int max_K);
+size_t prefill_umma_scratch_bytes(int M, int N, int K);   // all a launch writes behind its offset
 // scratch[0] is the handle's status word; the FP16 activation copy lives at scratch + offset.
 cudaError_t launch_prefill_umma(const LinearArgs& a, nvfp4_device_info& dev, void* scratch,
                                 size_t scratch_bytes, size_t offset, int* launches, cudaStream_t s);

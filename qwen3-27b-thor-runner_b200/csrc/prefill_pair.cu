@@ -843,10 +843,10 @@ bool prefill_umma_supported(const LinearArgs& a) {
 size_t prefill_umma_reserved_bytes() { return kStreamKBytes; }
 
 // Stream-K flags and partial tiles (fixed place, so a flag word only ever holds launch tags),
-// then the FP16 copy of the activations and one FP32 per token.
-size_t prefill_umma_scratch_bytes(int max_M, int /*max_N*/, int max_K) {
-    if (max_M <= 16) return 0;
-    return kStreamKBytes + act_bytes(max_M, max_K) + ((size_t)max_M * 4 + 255) / 256 * 256;
+// then the FP16 copy of the activations and one FP32 per token.  What a launch writes, whatever M is: options send
+// calls of 16 tokens and fewer here too.
+size_t prefill_umma_scratch_bytes(int M, int /*N*/, int K) {
+    return kStreamKBytes + act_bytes(M, K) + ((size_t)M * 4 + 255) / 256 * 256;
 }
 
 cudaError_t configure_prefill_umma(nvfp4_device_info& dev) {

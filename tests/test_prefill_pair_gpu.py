@@ -1,8 +1,11 @@
 """The prefill GEMM on pairs of SMs: sizes at the edges of its token tiles (multiples of 32 up to 192), row tiles (256 per
 pair, an odd number of them leaves half an item), 256-k stages and split tiles, through every output form."""
+import ctypes
+
 import numpy as np
 import pytest
 
+import nvfp4
 import oracle_binding as ob
 import util
 
@@ -81,3 +84,35 @@ def test_bf16_weights_vs_oracle(handle, M, N, K):
     assert all(np.array_equal(got, util.to_host_u16(o)) for o in outs[1:])
     assert ob.rel_frobenius(got, ob.dense_linear(A, W)) <= TOL
     assert handle.device_status() == 0
+
+
+@pytest.mark.parametrize("option,value,M", [("gemm_weight_rounding", 1, 9), ("gemm_weight_rounding", 1, 16), ("decode_max_m", 0, 1),
+                                            ("decode_max_m", 8, 12)])
+def test_few_tokens_need_the_kernels_whole_scratch(option, value, M):
+    """Options send 16 tokens and fewer to the pair kernel: a workspace sized for the GEMV kernels alone is refused before
+    anything is launched, through the host-buffer call too; one sized for 17 tokens takes the call."""
+    import torch
+    N, K = 512, 1024
+    lib = nvfp4.load()
+    packed, scale = util.make_weight(N, K, seed=M, sigma=0.14)
+    A = util.make_bf16((M, K), seed=M + 1)
+    dA, dp, ds = util.to_dev(A), util.to_dev(packed), util.to_dev(scale)
+    dC = torch.full((M, N), 0x7FC0, dtype=torch.int16, device="cuda")
+    hA, hC = torch.from_numpy(A.view(np.int16)), torch.zeros((M, N), dtype=torch.int16)
+    for max_m in (16, 17):
+        need = ctypes.c_size_t()
+        assert lib.nvfp4_workspace_bytes(max_m, N, K, ctypes.byref(need)) == 0
+        h = nvfp4.Handle(0, need.value)
+        h.set_option(option, value)
+        before = h.launch_count()
+        st = h.linear(dA, M, dp, ds, 1.0, N, K, dC, check=False)
+        if max_m == 16:
+            assert st == -4
+            assert lib.nvfp4_linear_host(h.h, hA.data_ptr(), M, dp.data_ptr(), ds.data_ptr(), 1.0, N, K, None, hC.data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream) == -4
+            assert h.launch_count() == before
+        else:
+            assert st == 0 and h.launch_count() == before + 2
+            assert ob.rel_frobenius(util.to_host_u16(dC), ob.linear(A, packed, scale, 1.0, mode=ob.GEMV, threads=8)) <= TOL
+            assert h.device_status() == 0
+        h.close()
