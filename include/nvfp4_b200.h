@@ -120,7 +120,12 @@ int nvfp4_get_option(nvfp4_handle* h, const char* name, int* value);
  *   invoke_fp4_gemm      (:539-584)                          residual NULL
  *   invoke_fp4_gemm_add  (:586-632)
  * Requirements: K % 16 == 0; A, C, residual 16-byte aligned; packed 16-byte
- * aligned; K % 32 == 0 for the fast paths (other K take the scalar path). */
+ * aligned; K % 32 == 0 for the fast paths (other K take the scalar path).
+ * Order: A, residual and C follow the stream.  So do the weights above 64 tokens.  Up to 64
+ * tokens the kernels start to read packed and scale while the kernel before them in the stream
+ * may still be running: weights written on the device (not loaded long before) must be complete,
+ * by a synchronisation with whatever wrote them, before such a call is issued.  The same holds
+ * for the other entry points that take packed and scale. */
 int nvfp4_linear(nvfp4_handle* h, const void* A_bf16, int M,
                  const uint8_t* packed, const uint8_t* scale_ue4m3, float global_scale,
                  int N, int K, const void* residual_bf16_or_null, void* C_bf16,

@@ -428,6 +428,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
             }
         } else {
             ptx::prefetch_tensormap(&tm_scale);
+            // No wait here: the pre-pass lets this kernel start only when everything older than itself has completed, so the
+            // stream orders the weights as for any kernel while their ring fills beside the pre-pass.
             while (work.next(p, it)) {
                 for (int ks = it.ks0; ks < it.ks1; ++ks) {
                     for (int r = 0; r < it.rows; ++r) {
@@ -896,7 +898,7 @@ cudaError_t launch_prefill_umma(const LinearArgs& a, nvfp4_device_info& dev, voi
         !make_map_cached(dev.maps, &tms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.scale, (uint64_t)a.K / 16, (uint64_t)a.N, 16, TR,
                   CU_TENSOR_MAP_SWIZZLE_NONE))
         return cudaErrorInvalidValue;
-    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, ah, unscale, s);
+    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, ah, unscale, true, s);
     if (e != cudaSuccess) return e;
     p.residual = static_cast<const __nv_bfloat16*>(a.residual);
     p.C = static_cast<__nv_bfloat16*>(a.C);

@@ -116,3 +116,43 @@ def test_few_tokens_need_the_kernels_whole_scratch(option, value, M):
             assert ob.rel_frobenius(util.to_host_u16(dC), ob.linear(A, packed, scale, 1.0, mode=ob.GEMV, threads=8)) <= TOL
             assert h.device_status() == 0
         h.close()
+
+
+@pytest.mark.parametrize("M", [65, 300])
+def test_weights_follow_the_stream(handle, M):
+    """A weight written by the work right before the call, again and again into the same buffers: by a copy, and by a call of
+    this library whose BF16 output serves as the codes (that kernel lets the next one start early)."""
+    import torch
+    N, K = 2048, 1024                                    # the second weight is the first call's [T, 256] output: N * K / 2 bytes
+    T, K1 = 2048, 2560
+    A = util.to_dev(util.make_bf16((M, K), seed=M))
+    A1 = util.to_dev(util.make_bf16((T, K1), seed=M + 1))
+    w1 = [util.make_weight(256, K1, seed=M + 2 + i, sigma=0.14) for i in range(4)]
+    w1 = [(util.to_dev(p), util.to_dev(s)) for p, s in w1]
+    source = [util.make_weight(N, K, seed=M + 20 + i, sigma=0.14) for i in range(4)]
+    source = [(util.to_dev(p), util.to_dev(s)) for p, s in source]
+    made = torch.empty((T, 256), dtype=torch.int16, device="cuda")
+    packed, scale = torch.empty_like(source[0][0]), torch.empty_like(source[0][1])
+    codes = made.view(torch.uint8).view(N, K // 2)
+
+    def step(i, out, wait):
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        packed.copy_(source[i][0])
+        scale.copy_(source[i][1])
+        sync()
+        handle.linear(A, M, packed, scale, 1.0, N, K, out[0])
+        sync()
+        handle.linear(A1, T, w1[i][0], w1[i][1], 1.0, 256, K1, made)
+        sync()
+        handle.linear(A, M, codes, scale, 1.0, N, K, out[1])
+        sync()
+
+    buffers = lambda: [torch.empty((M, N), dtype=torch.int16, device="cuda") for _ in range(2)]
+    want = [buffers() for _ in range(4)]
+    for i in range(4):
+        step(i, want[i], True)
+    for r in range(40):
+        got = buffers()
+        step(r % 4, got, False)
+        assert all(torch.equal(g, w) for g, w in zip(got, want[r % 4])), r
+    assert handle.device_status() == 0
