@@ -497,8 +497,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 const int turns = (it.ks1 - it.ks0) * (WK / XK) / (one ? 2 : 1);
                 const uint32_t d = tmem_base + (uint32_t)(t.i * p.T);
                 ok = ptx::mbar_wait(&tempty[t.i], t.phase ^ 1u, s_abort, p.status, 0x440u + t.i);
-                for (int turn = 0; ok && turn < turns; ++turn) {
-                    if (!xready) ok = ptx::mbar_wait(&xfull[x.i], x.phase, s_abort, p.status, 0x420u + x.i);
+                for (int turn = 0; turn < turns; ++turn) {
+                    if (!xready) ok = ok && ptx::mbar_wait(&xfull[x.i], x.phase, s_abort, p.status, 0x420u + x.i);
                     const uint32_t xa = (uint32_t)x.i;
                     x.advance(1);
                     uint32_t xb = xa;
@@ -508,6 +508,9 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                         x.advance(1);
                     }
                     if (!aready) ok = ok && ptx::mbar_wait(&afull[u.i], u.phase, s_abort, p.status, 0x430u + u.i);
+                    // One decision for the warp: where a wait runs out in some lanes only, those would leave and the others
+                    // stay for ever in the elections of the MMAs and commits below.
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t ui = (uint32_t)u.i;
