@@ -42,48 +42,28 @@
 
 #include "nvfp4_format.cuh"
 #include "nvfp4_internal.h"
+#include "pair_plan.h"
 #include "ptx.cuh"
 #include "umma.cuh"
 
 namespace nvfp4 {
 namespace {
 
+using namespace pair;
 using namespace umma;
 
-constexpr int TR = 128;                        // weight rows per CTA and row tile (TMEM lanes); 256 per pair
-constexpr int BK = 64;                         // k per operand block (128 bytes of 16-bit elements: one swizzle row)
-constexpr int WK = 256;                        // k per raw weight stage and per scheduling unit
-constexpr int kBlocks = WK / BK;
-constexpr int kWPackedBytes = TR * WK / 2;     // 16 KB
-constexpr int kWScaleBytes = TR * WK / 16;     // 2 KB
-constexpr int kWStageBytes = kWPackedBytes + kWScaleBytes;
-constexpr int XK = 128;                        // k per token stage and A unit (two operand blocks)
-constexpr int kDenseBlockBytes = TR * BK * 2;  // 16 KB
-constexpr int kDenseUnitBytes = 2 * kDenseBlockBytes;
-constexpr int kUnitCols = XK / 2;              // 64 TMEM columns of FP16 pairs per A unit (128 rows x 128 k)
-constexpr int kMaxUnits = 8, kMaxX = 8, kMaxW = 8, kMaxAccs = 4;
 constexpr int kThreads = 640;
 constexpr int kGroupWarps = 4, kEpiWarps = 4;  // two dequantising groups of four warps (one per TMEM lane quarter)
-constexpr int kBarBytes = 2048;     // barriers, token factors, a few words
-constexpr int kSmemMax = 225 * 1024;
 constexpr int kMaxT = 256;                     // columns a partial slot has room for
 constexpr int kSlotFloats = TR * kMaxT;        // one FP32 partial: [token][row]
-constexpr int kRaster = 8;                     // token tiles that consecutive items share a row group over
 
-struct PairParams {
+struct PairParams : Plan {
     const __nv_bfloat16* residual;
     __nv_bfloat16* C;
     const float* unscale;      // per token: 1 / activation scale (null: BF16 weights)
     unsigned int* status;
     float* partials;           // [grid][2][kSlotFloats]
     unsigned int* flags;       // [grid][2], the launch's tag once that partial is stored
-    int M, N, K;
-    int T;                     // tokens per tile
-    int m_tiles, row_tiles;    // row tiles of 256
-    int R;                     // row tiles per item
-    int items, dp_items;       // items [0, dp_items) run whole, the rest is split by k, one row tile at a time
-    int sk_tiles;              // (items - dp_items) * R
-    int w_stages, x_stages, units, accs, a_col0;
     uint32_t idesc;
     float inv_gs;
     float out_mul;             // what the epilogue multiplies the sums by besides the token factor: 2^8 / gs, or 1 / wshift
@@ -93,60 +73,6 @@ struct PairParams {
 };
 
 enum Mode { kExact = 0, kRounded = 1, kDense = 2 };
-
-// ---------------------------------------------------------------- work list
-struct Item {
-    int rt, rows;      // first row tile, number of row tiles (1 or 2)
-    int mt;            // token tile
-    int ks0, ks1;      // 256-k stages
-    int sk;            // split tile index, -1 = whole
-};
-struct Work {
-    long long u, u_end;
-    int dp, kst, pairs;
-    __device__ __forceinline__ Work(const PairParams& p, int kstages) {
-        pairs = gridDim.x >> 1;
-        const int id = blockIdx.x >> 1;
-        const long long units = (long long)p.sk_tiles * kstages;
-        u = (long long)id * units / pairs;
-        u_end = (long long)(id + 1) * units / pairs;
-        dp = id;
-        kst = kstages;
-    }
-    // item index -> first row tile and token tile: blocks of kRaster token tiles, row groups outside them
-    __device__ __forceinline__ void place(const PairParams& p, int item, int& rg, int& mt) const {
-        const int groups = (p.row_tiles + p.R - 1) / p.R;
-        const int blk = item / (kRaster * groups), rem = item - blk * (kRaster * groups);
-        const int width = min(kRaster, p.m_tiles - blk * kRaster);
-        rg = rem / width;
-        mt = blk * kRaster + rem - rg * width;
-    }
-    __device__ __forceinline__ bool next(const PairParams& p, Item& t) {
-        int rg;
-        if (u < u_end) {
-            t.sk = (int)(u / kst);
-            t.ks0 = (int)(u % kst);
-            const long long room = u_end - u;
-            t.ks1 = (kst - t.ks0) < room ? kst : t.ks0 + (int)room;
-            u += t.ks1 - t.ks0;
-            place(p, p.dp_items + t.sk / p.R, rg, t.mt);
-            t.rt = rg * p.R + t.sk % p.R;
-            t.rows = 1;
-            return true;
-        }
-        if (dp < p.dp_items) {
-            place(p, dp, rg, t.mt);
-            t.rt = rg * p.R;
-            t.rows = min(p.R, p.row_tiles - t.rt);
-            t.ks0 = 0;
-            t.ks1 = kst;
-            t.sk = -1;
-            dp += pairs;
-            return true;
-        }
-        return false;
-    }
-};
 
 // Position in a ring of buffers and the phase its barriers are in.
 struct Ring {
@@ -247,22 +173,12 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
     *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
-// Pairs first..last hold the parts of split tile `tile`; the first one holds its head (slot 1), the others a middle or tail (slot 0).
-__device__ __forceinline__ void participants(const PairParams& p, int kstages, int tile, int& first, int& last) {
-    const int pairs = gridDim.x >> 1;
-    const long long units = (long long)p.sk_tiles * kstages;
-    const long long b = (long long)tile * kstages, e = b + kstages;
-    first = last = blockIdx.x >> 1;
-    while (first > 0 && (long long)first * units / pairs > b) --first;
-    while (last + 1 < pairs && (long long)(last + 1) * units / pairs < e) ++last;
-}
-
 // Every participant calls this once its own parts are stored: it waits (bounded) for the parts of the others -- the CTAs of
 // the same rank in their pairs, which hold the same 128 rows -- and sums its own 1/P of the tile in pair order.
 __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int epoch, int tile, int kstages, int t, int nthreads,
                                              volatile int* s_abort) {
     int first, last;
-    participants(p, kstages, tile, first, last);
+    participants(p, kstages, gridDim.x >> 1, blockIdx.x >> 1, tile, first, last);
     const int rank = blockIdx.x & 1;
     {
         const long long t0 = clock64();
@@ -280,9 +196,8 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
         __syncwarp();
         if (*s_abort) return;
     }
-    Work w(p, kstages);
     int rg, mt;
-    w.place(p, p.dp_items + tile / p.R, rg, mt);
+    Work::place(p, p.dp_items + tile / p.R, rg, mt);
     const int n0 = (rg * p.R + tile % p.R) * 2 * TR + rank * TR, m0 = mt * p.T;
     const int tokens = min(p.T, p.M - m0);
     const int P = last - first + 1, me = (int)(blockIdx.x >> 1) - first;
@@ -392,7 +307,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const uint32_t tmem_base = *s_tmem;
     ptx::griddep_launch_dependents();      // the next kernel in the stream may start its own prologue
 
-    Work work(p, kstages);
+    Work work(p, kstages, gridDim.x >> 1, blockIdx.x >> 1);
     Item it;
     if (warp == 0) {
         // ------------------------------------------------------------------ weight stream
@@ -755,64 +670,14 @@ constexpr size_t kPartialBytes = (size_t)kSlotFloats * 4;
 constexpr int kMaxPrefillGrid = 160;
 constexpr size_t kStreamKBytes = 4096 + 2 * kMaxPrefillGrid * kPartialBytes;
 
-// Fills the tile plan of one launch; returns the grid, and the dynamic shared memory in *smem.
+// The tile plan of one launch and what follows from it; returns the grid, and the dynamic shared memory in *smem.
 int plan_pair(PairParams& p, const nvfp4_device_info& dev, bool dense, int* smem) {
     int pairs = (dev.sm_count < kMaxPrefillGrid ? dev.sm_count : kMaxPrefillGrid) / 2;
     if (dev.max_pairs > 0 && dev.max_pairs < pairs) pairs = dev.max_pairs;
-    const int kst = p.K / WK;
-    p.row_tiles = (p.N + 2 * TR - 1) / (2 * TR);
-    // T up to 192: two accumulators and two 64-column A units fill tensor memory; BF16 weights up to 160, where four 32 KB A
-    // units still leave three token stages.  Every (T, row tiles per item, split or not) is priced in clocks, with constants
-    // fitted to all plans of 19 shapes (65 to 8192 tokens, K 5120 to 17408): the choice is the best plan measured or within
-    // 5 % of it.  One MMA costs at least 87 clocks here (alone 65: the issuing warps share their schedulers with the
-    // dequantising ones), the operand streams bring 36 bytes a clock and SM; splitting costs 23,500 clocks and 49 a token
-    // (parts stored, flags, reduction), 7900 where whole items hide the reduction.
-    const int t_max = dense ? 160 : 192;
-    double best = 1e30;
-    for (int T = 32; T <= t_max; T += 32) {
-        const int mt = (p.M + T - 1) / T;
-        for (int R = 1; R <= 2; ++R) {
-            const long long items = (long long)((p.row_tiles + R - 1) / R) * mt;
-            // clocks of one 64-k block: the MMAs of a row tile, or the bytes of both streams
-            const double mma = 4.0 * (T / 2 > 87 ? T / 2 : 87), w_bytes = dense ? 16384.0 : 4608.0;
-            const double blk = std::fmax(R * mma, (T * 64.0 + R * w_bytes) / 36.0), blk1 = std::fmax(mma, (T * 64.0 + w_bytes) / 36.0);
-            const long long full = items / pairs, left = items % pairs;
-            const double epi = 8.0 * T * R, item = kst * kBlocks * blk + 0.25 * epi;
-            for (int split = 0; split < 2; ++split) {
-                if (split && (!left || !dev.prefill_stream_k || left * R * kst < pairs)) continue;
-                const double cost = split ? full * item + (double)((left * R * kst + pairs - 1) / pairs) * kBlocks * blk1 +
-                                                (full ? 7900.0 : 23500.0) + 49.0 * T
-                                          : (full + (left ? 1 : 0)) * item + epi;
-                if (cost < best) {
-                    best = cost;
-                    p.T = T; p.R = R; p.m_tiles = mt;
-                    p.items = (int)items;
-                    p.dp_items = split ? (int)(full * pairs) : (int)items;
-                    p.sk_tiles = split ? (int)(left * R) : 0;
-                }
-            }
-        }
-    }
-    const int xbytes = p.T / 2 * (XK * 2);
-    if (dense) {
-        p.accs = p.T <= 128 ? 4 : 2;
-        p.units = 4;
-        p.w_stages = 0;
-    } else {
-        p.accs = p.T <= 64 ? 4 : 2;
-        p.units = (512 - p.accs * p.T) / kUnitCols / 2 * 2;
-        if (p.units > kMaxUnits) p.units = kMaxUnits;
-        p.w_stages = p.T <= 64 ? 8 : 6;
-        p.a_col0 = 512 - p.units * kUnitCols;
-    }
-    const int wbytes = dense ? p.units * kDenseUnitBytes : p.w_stages * kWStageBytes;
-    p.x_stages = (kSmemMax - 1024 - kBarBytes - wbytes) / xbytes;
-    if (p.x_stages > kMaxX) p.x_stages = kMaxX;
-    *smem = 1024 + p.x_stages * xbytes + wbytes + kBarBytes;
+    pairs = make_plan(p, pairs, dev.prefill_stream_k != 0, dense, smem);
     p.idesc = (1u << 4) | ((uint32_t)(p.T >> 3) << 17) | ((uint32_t)(2 * TR >> 4) << 24);
     if (dense) p.idesc |= (1u << 7) | (1u << 10);         // A and B formats: BF16 instead of FP16
-    const long long work = p.dp_items ? p.items : (long long)p.sk_tiles * kst;
-    return 2 * (int)(work < pairs ? work : pairs);
+    return 2 * pairs;
 }
 
 template <int MODE>

@@ -1,0 +1,63 @@
+// The prefill kernel's plan and work list (csrc/pair_plan.h) for a test on the CPU.
+#include <vector>
+
+#include "pair_plan.h"
+
+using namespace nvfp4::pair;
+
+extern "C" {
+
+// out: T, R, m_tiles, row_tiles, items, dp_items, sk_tiles, w_stages, x_stages, units, accs, a_col0, smem, pairs used
+void pair_plan(int M, int N, int K, int pairs, int stream_k, int dense, int* out) {
+    Plan p{};
+    p.M = M; p.N = N; p.K = K;
+    int smem = 0;
+    const int used = make_plan(p, pairs, stream_k != 0, dense != 0, &smem);
+    const int v[] = {p.T, p.R, p.m_tiles, p.row_tiles, p.items, p.dp_items, p.sk_tiles, p.w_stages, p.x_stages, p.units, p.accs, p.a_col0, smem, used};
+    for (int i = 0; i < (int)(sizeof v / sizeof v[0]); ++i) out[i] = v[i];
+}
+
+// Walks all pairs' lists.  0: every (row tile, token tile, k stage) that holds outputs is worked on exactly once, no pair writes a
+// partial slot twice, and every holder of a split tile's part names the same holders, whose slots hold it.
+int pair_walk(int M, int N, int K, int pairs, int stream_k, int dense) {
+    Plan p{};
+    p.M = M; p.N = N; p.K = K;
+    int smem = 0;
+    const int used = make_plan(p, pairs, stream_k != 0, dense != 0, &smem), kst = K / WK;
+    if (used < 1 || used > pairs) return 1;
+    std::vector<unsigned char> seen((size_t)p.row_tiles * p.m_tiles * kst, 0);
+    std::vector<std::vector<int>> slot(used, std::vector<int>{-1, -1});      // split tile in the pair's slots (tail or middle, head)
+    for (int id = 0; id < used; ++id) {
+        Work w(p, kst, used, id);
+        Item t;
+        while (w.next(p, t)) {
+            if (t.rows < 1 || t.rows > 2 || t.mt < 0 || t.mt >= p.m_tiles || t.ks0 < 0 || t.ks1 > kst || t.ks0 >= t.ks1) return 2;
+            for (int r = 0; r < t.rows; ++r) {
+                if (t.rt + r >= p.row_tiles) {
+                    if (t.sk < 0 || p.R != 2) return 3;
+                    continue;
+                }
+                for (int k = t.ks0; k < t.ks1; ++k)
+                    if (seen[((size_t)(t.rt + r) * p.m_tiles + t.mt) * kst + k]++) return 4;
+            }
+            if (t.sk >= 0 && (t.ks0 || t.ks1 < kst)) {
+                int& s = slot[id][t.ks0 == 0];
+                if (s >= 0) return 5;
+                s = t.sk;
+            }
+        }
+    }
+    for (unsigned char c : seen) if (!c) return 6;
+    for (int id = 0; id < used; ++id)
+        for (int which = 0; which < 2; ++which)
+            if (slot[id][which] >= 0) {
+                int first, last;
+                participants(p, kst, used, id, slot[id][which], first, last);
+                if (first == last || id < first || id > last) return 7;
+                for (int c = first; c <= last; ++c)
+                    if (slot[c][c == first] != slot[id][which]) return 8;
+            }
+    return 0;
+}
+
+}  // extern "C"

@@ -1,5 +1,5 @@
-"""The prefill GEMM on pairs of SMs: sizes at the edges of its token tiles (multiples of 32 up to 192), row tiles (256 per
-pair, an odd number of them leaves half an item), 256-k stages and split tiles, through every output form."""
+"""The prefill GEMM on pairs of SMs: every form of its work (pair_forms.py: tokens per tile, row tiles per item, whole and split
+items) through every output form, and sizes at the edges of its tiles (256 rows a pair, 256-k stages)."""
 import ctypes
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 
 import nvfp4
 import oracle_binding as ob
+import pair_forms
 import util
 
 pytestmark = pytest.mark.gpu
@@ -27,16 +28,128 @@ def run(h, A, packed, scale, gs, residual=None):
     return util.to_host_u16(dC)
 
 
+def sample(N):
+    """Weight rows at the edges of row tiles and CTAs, and some between."""
+    edges = [0, 7, 8, 127, 128, 255, 256, 383, 384, N // 256 * 256 - 1, N // 256 * 256, N - 8, N - 1]
+    return np.unique([r for r in edges if 0 <= r < N] + list(np.random.default_rng(N).integers(0, N, 48)))
+
+
+def swiglu_of(plain, N):
+    import torch
+    slabs = plain.float().view(plain.shape[0], N // 16, 2, 8)
+    gate, up = slabs[:, :, 0].reshape(plain.shape[0], -1), slabs[:, :, 1].reshape(plain.shape[0], -1)
+    return (gate / (1 + torch.exp(-gate)) * up).to(torch.bfloat16)
+
+
+@pytest.fixture
+def pair_only(handle):
+    """17 to 64 tokens to the pair kernel too."""
+    handle.set_option("skinny_max_m", 0)
+    yield handle
+    handle.set_option("skinny_max_m", 64)
+    handle.set_option("gemm_weight_rounding", 0)
+
+
+@pytest.mark.parametrize("M,N,K,T,R,how", pair_forms.FP4)
+def test_every_form_through_every_output(pair_only, M, N, K, T, R, how):
+    import torch
+    h, gs = pair_only, 1.7
+    packed, scale = util.make_weight(N, K, seed=M + N, sigma=0.14)
+    A, residual = util.make_bf16((M, K), seed=M + 5), util.make_bf16((M, N), seed=N + 6)
+    dA, dp, ds, dR = (util.to_dev(x) for x in (A, packed, scale, residual))
+    rows = sample(N)
+    at = torch.from_numpy(rows).cuda()
+    p_s, s_s, r_s = (np.ascontiguousarray(x) for x in (packed[rows], scale[rows], residual[:, rows]))
+
+    def call(res=None, out=None):
+        out = torch.full((M, N), 0x7FC0, dtype=torch.int16, device="cuda") if out is None else out      # NaN canary
+        h.linear(dA, M, dp, ds, gs, N, K, out, residual=res)
+        return out
+
+    def error(out, **how_):
+        return ob.rel_frobenius(util.to_host_u16(out[:, at]), ob.linear(A, p_s, s_s, gs, threads=8, **how_))
+
+    plain = call()
+    assert error(plain, mode=ob.GEMV) <= TOL
+    assert torch.isfinite(plain.view(torch.bfloat16).float()).all()
+    added = call(dR)
+    assert error(added, residual=r_s, mode=ob.GEMV) <= TOL
+    for _ in range(3):
+        assert torch.equal(plain, call()) and torch.equal(added, call(dR))           # fixed summation order
+    alias = dR.clone()
+    assert torch.equal(added, call(alias, alias))                                    # C as its own residual
+    f32 = torch.full((M, N), float("nan"), device="cuda")
+    h.linear_f32(dA, M, dp, ds, gs, N, K, f32)
+    assert torch.equal(f32.to(torch.bfloat16).view(torch.int16), plain)              # the same sums, not rounded
+    if N % 32 == 0:
+        out = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device="cuda")
+        h.linear_ex(dA, M, dp, ds, gs, N, K, out, swiglu_epilogue=True)
+        # same sums, so at most one BF16 step where the two exponentials round differently: 2^-8 of the value
+        assert torch.allclose(out.float(), swiglu_of(plain.view(torch.bfloat16), N).float(), rtol=2 ** -7, atol=1e-30)
+    h.set_option("gemm_weight_rounding", 1)
+    rounded = call(dR)
+    assert torch.equal(rounded, call(dR))
+    assert error(rounded, residual=r_s, mode=ob.GEMM) <= TOL
+    assert h.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,T,R,how", [f for f in pair_forms.FP4 if f[3:] in ((160, 2, "whole"), (128, 1, "parts"), (160, 2, "tail"))])
+def test_non_finite_tokens_keep_to_themselves(pair_only, M, N, K, T, R, how):
+    """Tokens are columns of shared accumulators: an infinity or a NaN in one of them reaches no other."""
+    import torch
+    packed, scale = util.make_weight(N, K, seed=M, sigma=0.14)
+    dA = util.to_dev(util.make_bf16((M, K), seed=M + 1))
+    dp, ds = util.to_dev(packed), util.to_dev(scale)
+    clean, got = (torch.empty((M, N), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    pair_only.linear(dA, M, dp, ds, 1.0, N, K, clean)
+    bad = {0: 0x7F80, M // 2: 0x7FC0, M - 1: 0xFF80 - 0x10000}      # +inf, NaN, -inf
+    for m, bits in bad.items():
+        dA[m, (37 * m + 5) % K] = bits
+    pair_only.linear(dA, M, dp, ds, 1.0, N, K, got)
+    finite = torch.ones(M, dtype=torch.bool, device="cuda")
+    finite[list(bad)] = False
+    assert torch.equal(got[finite], clean[finite])
+    assert not torch.isfinite(got[~finite].float()).any()
+    assert pair_only.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,T,R,how", pair_forms.BF16)
+def test_every_form_on_bf16_weights(handle, M, N, K, T, R, how):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    W = (0.05 * torch.randn((N, K), device="cuda", generator=gen)).to(torch.bfloat16)
+    A, residual = util.make_bf16((M, K), seed=M + 3), util.make_bf16((M, N), seed=N + 4)
+    dA, dR = util.to_dev(A), util.to_dev(residual)
+    rows = sample(N)
+    at = torch.from_numpy(rows).cuda()
+    W_s = util.to_host_u16(W[at])
+
+    def call(res=None, out=None):
+        out = torch.full((M, N), 0x7FC0, dtype=torch.int16, device="cuda") if out is None else out
+        handle.linear_bf16(dA, M, W, N, K, out, residual=res)
+        return out
+
+    plain, added = call(), call(dR)
+    assert ob.rel_frobenius(util.to_host_u16(plain[:, at]), ob.dense_linear(A, W_s)) <= TOL
+    assert ob.rel_frobenius(util.to_host_u16(added[:, at]), ob.dense_linear(A, W_s, residual=np.ascontiguousarray(residual[:, rows]))) <= TOL
+    assert torch.isfinite(plain.view(torch.bfloat16).float()).all()
+    for _ in range(3):
+        assert torch.equal(plain, call()) and torch.equal(added, call(dR))
+    alias = dR.clone()
+    assert torch.equal(added, call(alias, alias))
+    assert handle.device_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K,res", [
     (65, 8, 256, True),           # one short row tile, one stage: every wait is a first phase
     (96, 264, 512, False),        # two row tiles, the second of 8 rows
-    (97, 768, 256, True),         # three row tiles
-    (160, 5376, 512, False),      # 21 row tiles: the last item has one
+    (97, 768, 256, True),         # three row tiles, one token in the last tile
+    (160, 5376, 512, False),      # 21 row tiles, two stages
     (161, 1280, 1024, True),      # one token in the last tile
-    (193, 2048, 2816, False),     # split along k
-    (385, 520, 4352, True),       # ragged rows, split tiles of a few tokens
+    (193, 2048, 2816, False),     # one token in the last tile, eleven stages
+    (385, 520, 4352, True),       # ragged rows, one token in the last tile, split
     (2500, 2816, 256, False),     # many items of one stage: the rings run across items
-    (1300, 5120, 768, True),      # whole items behind split ones
+    (1300, 5120, 768, True),      # items of two row tiles, three stages each
 ])
 def test_pair_kernel_vs_oracle(handle, M, N, K, res):
     packed, scale = util.make_weight(N, K, seed=M + N, sigma=0.14)
@@ -51,7 +164,7 @@ def test_pair_kernel_vs_oracle(handle, M, N, K, res):
 
 @pytest.mark.parametrize("M,N,K", [(70, 96, 256), (150, 5120, 2560), (333, 1024, 4352)])
 def test_swiglu_output_equals_linear_and_swiglu(handle, M, N, K):
-    """Interleaved rows (8 gate, 8 up): the SwiGLU of the plain call's rounded outputs, also across split tiles."""
+    """Interleaved rows (8 gate, 8 up): the SwiGLU of the plain call's rounded outputs."""
     import torch
     packed, scale = util.make_weight(N, K, seed=M, sigma=0.14)
     A = util.make_bf16((M, K), seed=M + 1)
@@ -60,9 +173,7 @@ def test_swiglu_output_equals_linear_and_swiglu(handle, M, N, K):
     out = torch.empty((M, N // 2), dtype=torch.bfloat16, device="cuda")
     handle.linear(dA, M, dp, ds, 1.0, N, K, plain)
     handle.linear_ex(dA, M, dp, ds, 1.0, N, K, out, swiglu_epilogue=True)
-    slabs = plain.float().view(M, N // 16, 2, 8)
-    gate, up = slabs[:, :, 0].reshape(M, -1), slabs[:, :, 1].reshape(M, -1)
-    want = (gate / (1 + torch.exp(-gate)) * up).to(torch.bfloat16)
+    want = swiglu_of(plain, N)
     # same sums, so at most one BF16 step where the two exponentials round differently: 2^-8 of the value
     assert torch.allclose(out.float(), want.float(), rtol=2 ** -7, atol=1e-30)
     assert handle.device_status() == 0
