@@ -16,17 +16,14 @@ constexpr int kHeld = 4;       // 16-byte vectors a thread keeps between the two
 // One CTA per token.  Latency-bound: the row is read once (all loads of a thread in flight together) and stays in registers
 // between the row maximum and the conversion; rows beyond kHeld x blockDim vectors are read again for the rest.
 __global__ void __launch_bounds__(1024)
-act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out, float* __restrict__ unscale, int K, bool ordered) {
+act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out, float* __restrict__ unscale, int K) {
     __shared__ unsigned int s_max;
     const int m = blockIdx.x, nv = K / 8;
     const uint4* src = reinterpret_cast<const uint4*>(A + (size_t)m * K);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)m * K);
     if (threadIdx.x == 0) s_max = 0u;
-    // The GEMM behind this kernel may set itself up and start streaming weights: at once, or (`ordered`) only when all that the
-    // stream holds before this call has completed, so that a weight written there is read as written.
-    if (!ordered) ptx::griddep_launch_dependents();
+    ptx::griddep_launch_dependents();      // the GEMM behind this kernel may set itself up (few tokens: start streaming weights)
     ptx::griddep_wait();                   // A is the output of the kernel before this one
-    if (ordered) ptx::griddep_launch_dependents();
     __syncthreads();
     unsigned int amax = 0;
     auto largest = [&](const uint4& x) {
@@ -68,7 +65,7 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
 
 }  // namespace
 
-cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, bool ordered, cudaStream_t s) {
+cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(M);
     // as many threads as hold the row in kHeld vectors each; few tokens: half as many vectors (latency, SMs to spare)
@@ -83,7 +80,7 @@ cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float*
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, act_to_f16_kernel, static_cast<const __nv_bfloat16*>(A), static_cast<__half*>(out_f16),
-                              unscale, K, ordered);
+                              unscale, K);
 }
 
 }  // namespace nvfp4

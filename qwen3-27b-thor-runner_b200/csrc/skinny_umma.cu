@@ -481,7 +481,7 @@ cudaError_t launch_skinny_umma(const LinearArgs& a, nvfp4_device_info& dev, void
         !make_map_cached(dev.maps, &tms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.scale, (uint64_t)a.K / 16, (uint64_t)a.N, 16, TR,
                   CU_TENSOR_MAP_SWIZZLE_NONE))
         return cudaErrorInvalidValue;
-    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, base, unscale, false, s);
+    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, base, unscale, s);
     if (e != cudaSuccess) return e;
     pl.p.unscale = unscale;
     pl.p.residual = static_cast<const __nv_bfloat16*>(a.residual);
