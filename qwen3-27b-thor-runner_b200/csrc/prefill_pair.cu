@@ -582,11 +582,15 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                         f[i + 3] = __uint_as_float(v[i + 3]) * k4.w;
                     }
                     if (p.swiglu_out) {
-                        __nv_bfloat16* dst = p.C + (size_t)(m0 + c0) * (p.N / 2) + 8 * (n >> 4) + (n & 7);
+                        // A gate lane and its up lane (eight rows on) hold both halves of sixteen outputs: the gate lane finishes
+                        // the first eight tokens, the up lane the others, one exchange and one SiLU each.
+                        const int late = n & 8;
+                        __nv_bfloat16* dst = p.C + (size_t)(m0 + c0 + late) * (p.N / 2) + 8 * (n >> 4) + (n & 7);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float up = __shfl_xor_sync(0xffffffffu, f[i], 8);
-                            if (i < cnt && !(n & 8) && n < p.N) dst[(size_t)i * (p.N / 2)] = __float2bfloat16_rn(silu_pair(f[i], up));
+                        for (int i = 0; i < 8; ++i) {
+                            const float other = __shfl_xor_sync(0xffffffffu, late ? f[i] : f[i + 8], 8);
+                            const float y = silu_pair(late ? other : f[i], late ? f[i + 8] : other);
+                            if (late + i < cnt && n < p.N) dst[(size_t)i * (p.N / 2)] = __float2bfloat16_rn(y);
                         }
                         continue;
                     }
