@@ -549,6 +549,11 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
             // Both groups wait for and free both accumulators (accs is even: a pair never wraps).
             const int begin = two ? 0 : eg * (p.T / 2), end = two ? tokens : min(tokens, (eg + 1) * (p.T / 2));
             const int n = ((it.rt + (two ? eg : 0)) * 2 + rank) * TR + te;
+            if (p.residual && complete && n - lane < p.N) {    // its way from memory goes behind the MMAs: 64 bytes a token and warp into L2
+                const __nv_bfloat16* src = p.residual + (size_t)m0 * p.N;
+                for (int i = 2 * begin + lane; i < 2 * end; i += 32)
+                    ptx::prefetch_l2(src + (size_t)(i >> 1) * p.N + min(n - lane + 16 * (i & 1), p.N - 1));
+            }
             for (int i = t.i; i < t.i + 2; ++i)
                 if (ptx::mbar_wait(&tfull[i], t.phase, s_abort, p.status, 0x470u + i) && rank == 0 && tt == 0) relay(&tfull[i]);
             __syncwarp();
