@@ -30,8 +30,6 @@ struct nvfp4_handle {
     int gemm_weight_rounding = 0;                // above 8 tokens: the reference's BF16-rounded weights (its GEMM branch)
     unsigned long long launches = 0;
     int host_direct_out = 1;                     // nvfp4_linear_host: kernels store into a pinned, device-mapped C_host themselves
-    const void* host_out_seen = nullptr;         // the last C_host looked up, and its device address (null: not pinned)
-    void* host_out_dev = nullptr;
     // scale tensors in which nvfp4_scan_scales found a byte 0x7F / 0xFF: the tensor core reads those as NaN, so
     // these weights stay on the kernels that decode the scale themselves
     std::vector<const void*> nan_scales;
@@ -709,16 +707,12 @@ int nvfp4_linear_host(nvfp4_handle* h, const void* A_host, int M, const uint8_t*
     // that overlap the kernel's tail) and the copy back, with its own start-up latency, is not needed.
     void* out = dC;
     if (h->host_direct_out && !residual_host && aligned16(C_host) && (size_t)M * N * 2 <= (2u << 20)) {
-        if (C_host != h->host_out_seen) {
-            cudaPointerAttributes at{};
-            h->host_out_seen = C_host;
-            h->host_out_dev = nullptr;
-            if (cudaPointerGetAttributes(&at, C_host) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
-                h->host_out_dev = at.devicePointer;
-            else
-                cudaGetLastError();
-        }
-        if (h->host_out_dev) out = h->host_out_dev;
+        // asked on every call: the address may be other memory by now, or no longer pinned
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, C_host) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
+            out = at.devicePointer;
+        else
+            cudaGetLastError();
     }
     // The kernels see the workspace without the staging area, so their scratch never reaches it.
     LinearArgs a{dA, packed, scale, 1.0f / global_scale, dR, out, M, N, K};

@@ -510,6 +510,31 @@ def test_linear_host_direct_output_equals_staged(handle, M, N, K):
     assert handle.device_status() == 0
 
 
+def test_linear_host_output_that_is_no_longer_pinned(handle):
+    """One address, pinned for the first call and ordinary memory for the second: nothing may be kept about it."""
+    import mmap
+    import torch
+    M, N, K = 2, 1024, 1024
+    packed, scale = util.make_weight(N, K, seed=90)
+    dp, ds = util.to_dev(packed), util.to_dev(scale)
+    hA = torch.from_numpy(util.make_bf16((M, K), seed=91).view(np.int16)).pin_memory()
+    memory = mmap.mmap(-1, M * N * 2)
+    out = np.frombuffer(memory, dtype=np.int16).reshape(M, N)
+    cudart = torch.cuda.cudart()
+    got = []
+    for pinned in (True, False):
+        if pinned:
+            assert int(cudart.cudaHostRegister(out.ctypes.data, out.nbytes, 0)) == 0
+        out[:] = 0x7FC0
+        handle.linear_host(hA, M, dp, ds, 1.0, N, K, torch.from_numpy(out))
+        got.append(out.copy())
+        if pinned:
+            assert int(cudart.cudaHostUnregister(out.ctypes.data)) == 0
+    assert np.array_equal(got[0], got[1])
+    want = ob.linear(hA.numpy().view(np.uint16), packed, scale, 1.0, mode=ob.GEMV)
+    assert ob.rel_frobenius(got[1].view(np.uint16), want) <= TOL
+
+
 def test_linear_host_odd_workspace_size():
     """A workspace size that is not a multiple of 16: the staging buffers at its end stay aligned."""
     import torch
