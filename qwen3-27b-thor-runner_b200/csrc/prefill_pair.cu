@@ -472,19 +472,28 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                     const uint32_t scw = mask_scale_bytes(*reinterpret_cast<const uint32_t*>(ws + 4 * j));
                     const uint32_t q[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
                     uint32_t o[2][16];
+                    uint32_t one = 0u, more = 0u;          // kRounded: what a block's 1.0 comes to, and twice what 1.5 has over it
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {          // 8 consecutive k = one 32-bit word of codes
                         uint32_t e[4];
                         ptx::cvt_e2m1x8_to_f16x2(q[c], e);
                         if (MODE == kRounded) {
-                            // the reference's dequantisation, operation for operation: FP32 block scale times 1/gs, FP32
-                            // product with the code's value, one rounding to BF16; then a power of two into FP16 (exact)
-                            const float bs = ue4m3_to_float((scw >> (8 * (c >> 1))) & 0xFFu) * p.inv_gs;
+                            // The bits of the reference's dequantisation: FP32 block scale times 1/gs, FP32 product with the code's
+                            // value, one rounding to BF16; then a power of two into FP16 (exact).  A code is p or 1.5 p, p a power
+                            // of two, which commutes with the roundings, so a block takes two of them, and an element is
+                            // p * one + (code - p) * more, exact in FP16 (one and 1.5's value have eight bits each).  One rounding
+                            // an element bound the kernel: 34816 x 5120 at 256 / 2048 tokens 164 / 832 us, 125 / 644 so.
+                            if (!(c & 1)) {
+                                const float bs = ue4m3_to_float((scw >> (8 * (c >> 1))) & 0xFFu) * p.inv_gs;
+                                const float2 b = __bfloat1622float2(__floats2bfloat162_rn(bs, 1.5f * bs));
+                                const float x = b.x * p.wshift, y = 2.0f * (b.y - b.x) * p.wshift;
+                                one = ptx::pack_f16x2(x, x);
+                                more = ptx::pack_f16x2(y, y);
+                            }
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
-                                const float2 l = __half22float2(*reinterpret_cast<const __half2*>(&e[i]));
-                                const float2 b = __bfloat1622float2(__floats2bfloat162_rn(l.x * bs, l.y * bs));
-                                o[c >> 2][(c & 3) * 4 + i] = ptx::pack_f16x2(b.x * p.wshift, b.y * p.wshift);
+                                const uint32_t pow2 = e[i] & 0xFDFFFDFFu;           // without FP16's top mantissa bit, set in 1.5, 3 and 6
+                                o[c >> 2][(c & 3) * 4 + i] = ptx::fma_f16x2(ptx::sub_f16x2(e[i], pow2), more, ptx::mul_f16x2(pow2, one));
                             }
                         } else {
                             const uint32_t S = scale_byte_to_f16x2(scw, c >> 1);     // scale / 2^8, undone in the epilogue

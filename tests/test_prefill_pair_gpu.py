@@ -93,6 +93,27 @@ def test_every_form_through_every_output(pair_only, M, N, K, T, R, how):
     assert h.device_status() == 0
 
 
+@pytest.mark.parametrize("gs", [1.0, 0.37, 2688.0, 3.0e-20, 7.0e25])
+def test_rounded_weights_are_the_dequantised_matrix(handle, gs):
+    """One-hot tokens pick single weights out: with gemm_weight_rounding each is the bits that nvfp4_dequant_bf16 stores (the
+    reference's), over all codes and finite block scales."""
+    import torch
+    N, K = 2048, 256
+    rng = np.random.default_rng(11)
+    packed = util.to_dev(rng.integers(0, 256, (N, K // 2), dtype=np.uint8))
+    scale = util.to_dev((np.arange(N * K // 16, dtype=np.int64) * 31 % 127).astype(np.uint8).reshape(N, K // 16))      # 0 .. 126, all of them
+    want = torch.empty((N, K), dtype=torch.bfloat16, device="cuda")
+    handle.dequant(packed, scale, gs, N, K, want)
+    out = torch.full((K, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    handle.set_option("gemm_weight_rounding", 1)
+    try:
+        handle.linear(torch.eye(K, dtype=torch.bfloat16, device="cuda"), K, packed, scale, gs, N, K, out)
+    finally:
+        handle.set_option("gemm_weight_rounding", 0)
+    assert torch.equal(out.T.float(), want.float())                    # by value: -0 and 0 are alike
+    assert torch.isfinite(want.float()).all() and handle.device_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K,T,R,how", [f for f in pair_forms.FP4 if f[3:] in ((160, 2, "whole"), (128, 1, "parts"), (160, 2, "tail"))])
 def test_non_finite_tokens_keep_to_themselves(pair_only, M, N, K, T, R, how):
     """Tokens are columns of shared accumulators: an infinity or a NaN in one of them reaches no other."""
