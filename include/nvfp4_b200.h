@@ -85,7 +85,7 @@ const char* nvfp4_status_string(int status);
  *   "gemm_weight_rounding": 0 (default) = every kernel multiplies the exact block-scaled weights and applies
  *                   1 / global_scale once, in FP32 (the reference's arithmetic up to 8 tokens,
  *                   dense_gemm_fp4_sm110.cu:96-141).  1 = above 8 tokens the weights are rounded to BF16
- *                   after the global scale, bf16(e2m1 * (ue4m3 * 1/gs)), operation for operation what the
+ *                   after the global scale, bf16(e2m1 * (ue4m3 * 1/gs)), the bits of what the
  *                   reference's GEMM branch does (:444-467, 558-583); with a global scale that is not a
  *                   power of two the two forms lie 2.7e-3 apart.  Plain calls with N % 8 == 0 and
  *                   K % 256 == 0 only (NVFP4_E_LIMIT otherwise); slower (the tcgen05 GEMM with a longer

@@ -65,11 +65,11 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
 
 }  // namespace
 
-cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, cudaStream_t s) {
+cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, int sm_count, cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(M);
     // as many threads as hold the row in kHeld vectors each; few tokens: half as many vectors (latency, SMs to spare)
-    const int per = M <= 148 ? kHeld / 2 : kHeld;
+    const int per = M <= sm_count ? kHeld / 2 : kHeld;
     int threads = ((K / 8 + per - 1) / per + 31) / 32 * 32;
     cfg.blockDim = dim3(threads < 64 ? 64 : (threads > 1024 ? 1024 : threads));
     cfg.dynamicSmemBytes = 0;

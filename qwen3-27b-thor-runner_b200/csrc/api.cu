@@ -110,7 +110,7 @@ int run_linear(nvfp4_handle* h, const LinearArgs& a, cudaStream_t s, size_t ws_b
         return cuda_status(e);
     }
     if (a.out_f32 && a.M > 16) {
-        // unrounded FP32 sums beyond the GEMV kernels: the 128-token-tile tcgen05 kernel's FP32 epilogue
+        // unrounded FP32 sums beyond the GEMV kernels: the FP32 epilogue of the tcgen05 GEMM on pairs of SMs
         if (a.swiglu_up || a.a_stride || a.k_valid || a.norm_w || a.px || a.swiglu_out) return NVFP4_E_LIMIT;
         if (h->prefill_impl == 1 || !prefill_umma_supported(a)) return NVFP4_E_LIMIT;
         if (kDecodeScratchBytes + prefill_umma_scratch_bytes(a.M, a.N, a.K) > ws_bytes) return NVFP4_E_WORKSPACE;
@@ -120,7 +120,7 @@ int run_linear(nvfp4_handle* h, const LinearArgs& a, cudaStream_t s, size_t ws_b
         return cuda_status(e);
     }
     if (a.swiglu_out && !other_options && !a.px && a.M > 16) {
-        // beyond the GEMV kernels only the 128-token-tile tcgen05 kernel has the SwiGLU epilogue
+        // beyond the GEMV kernels only the tcgen05 GEMM on pairs of SMs has the SwiGLU epilogue
         if (h->prefill_impl == 1 || !prefill_umma_supported(a)) return NVFP4_E_LIMIT;
         if (kDecodeScratchBytes + prefill_umma_scratch_bytes(a.M, a.N, a.K) > ws_bytes) return NVFP4_E_WORKSPACE;
         int nl = 0;

@@ -424,7 +424,7 @@ cudaError_t launch_decode_wide(const LinearArgs& a, nvfp4_device_info& dev, void
         !umma::make_map_cached(dev.maps, &tms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.scale, (uint64_t)a.K / 16, (uint64_t)a.N, 16, kUnitRows,
                         CU_TENSOR_MAP_SWIZZLE_NONE))
         return cudaErrorInvalidValue;
-    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, act_f16, unscale, s);
+    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, act_f16, unscale, dev.sm_count, s);
     if (e != cudaSuccess) return e;
     WideParams p{};
     p.residual = static_cast<const __nv_bfloat16*>(a.residual);

@@ -176,7 +176,7 @@ cudaError_t launch_decode_fp4_stream(const LinearArgs& a, nvfp4_device_info& dev
                                      int* launches, cudaStream_t s);
 
 // --- act_f16.cu: BF16 activations -> FP16 copy with an exact per-token power-of-two scale; unscale[m] = 1/scale.
-cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, cudaStream_t s);
+cudaError_t launch_act_to_f16(const void* A, int M, int K, void* out_f16, float* unscale, int sm_count, cudaStream_t s);
 
 // --- prefill_pair.cu: fused dequant + tcgen05 GEMM on pairs of SMs, weights expanded into tensor memory.
 bool prefill_umma_supported(const LinearArgs& a);

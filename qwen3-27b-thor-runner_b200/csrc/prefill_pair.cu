@@ -11,7 +11,7 @@
 //   warp 2      TMA: token blocks (T/2 x 64 k, FP16, 128-byte swizzle); both CTAs' blocks complete on the leader's barrier.
 //   warps 8-15  dequantise: thread = weight row = TMEM lane; 64 k of a 128-k unit each group, cvt.rn.f16x2.e2m1x2 + one f16x2 multiply by
 //               the block scale (exact), tcgen05.st into a ring of A units; arrive on the leader's barrier.
-//   warp 1      of the leader CTA issues the MMAs; commits free the A units and token stages.
+//   warps 1, 3  of the leader CTA issue the MMAs, one row tile or every other 128 k each; commits free the A units and token stages.
 //   warps 4-7, 16-19  epilogue: thread = weight row, registers = tokens: a warp stores 32 consecutive outputs of one token.
 //
 // What bounds it and why this form.  With both operands in shared memory (128 tokens x 256 rows per CTA, a dequantised block
@@ -20,15 +20,18 @@
 // shared-memory bandwidth, and a pair of SMs stages each token once: 60-80 B/clk.  T is any multiple of 32, so 149 tokens are one
 // tile of 160 instead of two of 128.  What bounds it now is the issue of the MMAs beside the dequantising warps for
 // T < 192 (see the issuers), the power cap for long runs of T = 192, and for a few hundred tokens the reduction of split tiles.
-// Measured before -> after, pre-pass included: 34816 x 5120 at 8192 / 1111 / 256 / 149 tokens 2810 -> 1940, 379-426 -> 300, 87 -> 77,
-// 83 -> 46 us; 5120 x 17408 1380 -> 1080, 226 -> 149, 67 -> 54, 63 -> 40 us; BF16 5120 x 5120 at 512 tokens 48 -> 32 us.
+// Measured, the kernel before this form -> now, pre-pass included, weights from memory, four calls back to back after a pause (median;
+// a run of seconds at the power cap is up to a sixth slower): 34816 x 5120 at 149 / 256 / 1111 / 2048 / 4096 tokens 92 -> 51, 95 -> 84,
+// 385 -> 278, 637 -> 505, 1280 -> 1015 us; 5120 x 17408 with a residual 69 -> 40, 72 -> 59, 244 -> 155, 343 -> 288, 675 -> 542 us; BF16
+// 7168 x 5120 at 256 / 512 tokens 46 -> 26, 64 -> 42 us.
+// ncu at 34816 x 5120, 2048 tokens: tensor pipe active 81 % of the time, DRAM 14 %, L2 25 %, issue slots 45 %.
 //
 // Operands are FP16 because the hardware E2M1 conversion produces FP16 and every e2m1 x ue4m3 product is exact in FP16
 // (kind::f16 takes both operands in ONE 16-bit format).  A pre-pass turns the BF16 activations into FP16 with an exact
 // per-token power-of-two scale in the handle workspace.
 //
-// Work items left over after whole waves are split along k over all pairs (stream-K): partial tiles in FP32 with a flag
-// per part, every participant then sums its own slice of the tile in a fixed order (deterministic).
+// Work items left over after whole waves may be split along k (pair_plan.h): partial tiles in FP32 with a flag per part, every
+// participant then sums its own slice of the tile in a fixed order (deterministic).
 //
 // DENSE: the weight is BF16 [N,K] and the activations are the caller's BF16 rows; the weight blocks (128 rows x 64 k)
 // come by TMA as the shared-memory A operand and nothing is dequantised.
@@ -670,7 +673,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
     if (all_reduce) {
-        // Every tile was split and nothing else is left to do: all 16 warps reduce.
+        // Every tile was split and nothing else is left to do: all 20 warps reduce.
         ptx::griddep_wait();
         const unsigned int epoch = *s_epoch;
         const int pairs = gridDim.x >> 1, id = blockIdx.x >> 1;
@@ -786,7 +789,7 @@ cudaError_t launch_prefill_umma(const LinearArgs& a, nvfp4_device_info& dev, voi
         !make_map_cached(dev.maps, &tms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.scale, (uint64_t)a.K / 16, (uint64_t)a.N, 16, TR,
                   CU_TENSOR_MAP_SWIZZLE_NONE))
         return cudaErrorInvalidValue;
-    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, ah, unscale, s);
+    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, ah, unscale, dev.sm_count, s);
     if (e != cudaSuccess) return e;
     p.residual = static_cast<const __nv_bfloat16*>(a.residual);
     p.C = static_cast<__nv_bfloat16*>(a.C);

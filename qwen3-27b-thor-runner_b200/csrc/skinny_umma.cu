@@ -121,7 +121,7 @@ __device__ __forceinline__ void store_output(const SkinnyParams& p, int m, int n
     p.C[o] = __float2bfloat16_rn(f);
 }
 
-// Reduction of one split row tile (see reduce_split_tile of the prefill kernel: same protocol).
+// Reduction of one split row tile (as reduce_split of the prefill kernel: a flag per part, then every participant sums its slice).
 // The P participants each take 1/P of the tokens; with fewer tokens than participants the
 // rows are split instead.  t = 0..nthreads-1, nthreads a multiple of 128.
 __device__ __forceinline__ void reduce_split_rows(const SkinnyParams& p, unsigned int epoch, int tile, int kstages, int t,
@@ -481,7 +481,7 @@ cudaError_t launch_skinny_umma(const LinearArgs& a, nvfp4_device_info& dev, void
         !make_map_cached(dev.maps, &tms, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.scale, (uint64_t)a.K / 16, (uint64_t)a.N, 16, TR,
                   CU_TENSOR_MAP_SWIZZLE_NONE))
         return cudaErrorInvalidValue;
-    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, base, unscale, s);
+    cudaError_t e = launch_act_to_f16(a.A, a.M, a.K, base, unscale, dev.sm_count, s);
     if (e != cudaSuccess) return e;
     pl.p.unscale = unscale;
     pl.p.residual = static_cast<const __nv_bfloat16*>(a.residual);

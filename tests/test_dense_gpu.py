@@ -67,9 +67,9 @@ def test_dense_lm_head_shape_sample(handle):
     (17, 256, 256, False),         # one tile, one stage
     (24, 256, 512, True),
     (128, 1000, 1024, True),       # N not a multiple of the 256-row tile
-    (300, 2048, 1280, False),      # three token tiles: a pair and a single
+    (300, 2048, 1280, False),      # several token tiles, the last one short
     (1000, 640, 5120, True),       # few tiles, deep K: split along k over the CTAs
-    (130, 40000, 256, True),       # more tiles than CTAs: whole waves of pairs + a split remainder
+    (130, 40000, 256, True),       # more items than pairs of CTAs, a stage each
 ])
 def test_dense_gemm_vs_oracle(handle, M, N, K, res):
     """More than 16 tokens: the tcgen05 GEMM with the BF16 weight blocks loaded straight into the

@@ -82,7 +82,8 @@ def _sample_rows(N, seed, count=96):
     (16, 1024, 2048),
     (40, 1000, 17408),    # few-token tcgen05 kernel, every tile split along k
     (64, 5120, 4352),
-    (300, 15360, 3840),   # prefill kernel: a whole wave of tiles + tiles split along k
+    (300, 15360, 3840),   # prefill kernel: whole items of two row tiles
+    (869, 3608, 3584),    # prefill kernel: whole items, then tiles split along k
     (130, 512, 5120),     # prefill kernel, every tile split
 ])
 def test_graph_replay_linear(handle, M, N, K):

@@ -429,7 +429,9 @@ def test_prefill_shapes_the_tensor_core_kernel_does_not_take(handle, M, N, K):
     assert ob.rel_frobenius(got, ob.linear(A, packed, scale, 1.0, residual=R, mode=ob.GEMM, threads=8)) <= TOL
 
 
-@pytest.mark.parametrize("M,N,K,res", [(300, 15360, 3840, True),    # 180 tiles: one whole wave + 32 tiles split by k
+@pytest.mark.parametrize("M,N,K,res", [(300, 15360, 3840, True),    # prefill kernel, whole items only
+                                         (869, 3608, 3584, True),      # prefill kernel: a whole wave, then tiles split by k
+                                         (200, 1056, 5888, False),     # prefill kernel: ten tiles of six parts
                                          (64, 5120, 4352, False),      # 20 tiles, each shared by ~7 CTAs
                                          (40, 1000, 17408, True)])     # ragged N, deep K
 def test_prefill_split_tiles(handle, M, N, K, res):
@@ -671,7 +673,7 @@ def test_linear_f32_matches_bf16_path(handle):
     got32 = dC.cpu().numpy()
     got16 = run_linear(handle, A, packed, scale, 2.0)
     assert np.array_equal(ob.f32_to_bf16(got32), got16)
-    # beyond the GEMV kernels: the tcgen05 GEMM's FP32 epilogue (whole tiles and tiles split along k)
+    # beyond the GEMV kernels: the tcgen05 GEMM's FP32 epilogue (whole tiles; split ones: test_prefill_pair_gpu.py)
     handle.set_option("skinny_min_m", 129)           # the BF16 comparison through the same kernel
     try:
         for M2 in (17, 200):
