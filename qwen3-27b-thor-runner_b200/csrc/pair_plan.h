@@ -1,7 +1,6 @@
 // Tile plan and work list of the prefill kernel on pairs of SMs (prefill_pair.cu): plain arithmetic, no CUDA types, so that a
 // test can walk every plan on the CPU.
 #pragma once
-#include <algorithm>
 #include <cmath>
 
 #ifdef __CUDACC__
