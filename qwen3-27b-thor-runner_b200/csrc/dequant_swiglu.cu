@@ -2,6 +2,7 @@
 // the linear layer.
 #include "nvfp4_format.cuh"
 #include "nvfp4_internal.h"
+#include "ptx.cuh"
 
 namespace nvfp4 {
 namespace {
@@ -38,20 +39,47 @@ dequant_bf16_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restric
 // row_stride_in elements apart (I for separate tensors, 2I for the merged layout).  interleaved:
 // the input row holds slabs of 16 columns, 8 gate values followed by their 8 up values (the
 // output of a linear on row-interleaved gate/up weights); gate points at column 0, up at column 8.
+// Few tokens: bound by the launch, so it starts while the kernel before it finishes and lets the one behind it start its
+// prologue (a few-token linear: its weight stream).  With the norm below: an MLP of 5120 x 17408 on 40 tokens 69.8 -> 64.9 us,
+// two decode layers of 4 tokens 132.8 -> 131.0 (replayed from a graph, where plain launches follow each other faster).
+constexpr int kSwigluHeld = 2;         // vectors of eight outputs a thread has in flight
 
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
               __nv_bfloat16* __restrict__ out, long long row_stride_in, long long row_stride_out, int M, int I,
               int interleaved) {
+    ptx::griddep_launch_dependents();
+    ptx::griddep_wait();                       // gate and up are the output of the kernel before this one
     const int vec_per_row = I >> 3;
     const long long total = (long long)M * vec_per_row;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += stride) {
-        const int m = (int)(v / vec_per_row), c = (int)(v % vec_per_row) * 8;
-        const int cin = interleaved ? 2 * c : c;
-        const uint4 g4 = *reinterpret_cast<const uint4*>(gate + (size_t)m * row_stride_in + cin);
-        const uint4 u4 = *reinterpret_cast<const uint4*>(up + (size_t)m * row_stride_in + cin);
-        *reinterpret_cast<uint4*>(out + (size_t)m * row_stride_out + c) = swiglu_bf16x8(g4, u4);
+    long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < total) {
+        // row and column of vector v, carried along instead of divided out each time
+        const int dm = (int)(stride / vec_per_row), dc = (int)(stride % vec_per_row);
+        int m = (int)(v / vec_per_row), c = (int)(v % vec_per_row);
+        while (v < total) {
+            uint4 g4[kSwigluHeld], u4[kSwigluHeld];
+            size_t to[kSwigluHeld];
+            bool live[kSwigluHeld];
+#pragma unroll
+            for (int j = 0; j < kSwigluHeld; ++j) {
+                live[j] = v < total;
+                to[j] = (size_t)m * row_stride_out + c * 8;
+                if (live[j]) {
+                    const size_t from = (size_t)m * row_stride_in + (interleaved ? 16 : 8) * c;
+                    g4[j] = *reinterpret_cast<const uint4*>(gate + from);
+                    u4[j] = *reinterpret_cast<const uint4*>(up + from);
+                }
+                v += stride;
+                m += dm;
+                c += dc;
+                if (c >= vec_per_row) { c -= vec_per_row; ++m; }
+            }
+#pragma unroll
+            for (int j = 0; j < kSwigluHeld; ++j)
+                if (live[j]) *reinterpret_cast<uint4*>(out + to[j]) = swiglu_bf16x8(g4[j], u4[j]);
+        }
     }
     // I % 8 tail columns, scalar.
     const int tail0 = vec_per_row * 8;
@@ -64,6 +92,21 @@ swiglu_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __res
             out[(size_t)m * row_stride_out + c] = __float2bfloat16_rn(silu(g) * u);
         }
     }
+}
+
+// Launch with programmatic stream serialization: the kernel's prologue may run while the kernel before it finishes.
+template <class... P, class... A>
+cudaError_t launch_behind(void (*kernel)(P...), int grid, int threads, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 int grid_for(long long work_items, int block) {
@@ -115,53 +158,65 @@ namespace {
 
 // RMSNorm with the centred weight, one CTA per token:
 //   out = bf16( (x * rsqrt(mean(x^2) + eps)) * (1 + w) ), FP32 throughout
-// (rmsnorm_kernel, src/engine/light_ops.cu:65-106).  With `bias` the row is x + bias first, kept
+// (rmsnorm_kernel, src/engine/light_ops.cu:65-106).  BIAS: the row is x + bias first, kept
 // unrounded for the norm, and bf16(x + bias) goes back to x (fused_add_rmsnorm_kernel, :270-318).
-// 16-byte chunks; a thread keeps up to kNormCache chunks in registers between the two passes and
-// reads the row again beyond that.  1/sqrtf and a true division, not the fast-math forms.
+// 16-byte chunks; a thread keeps up to kNormCache chunks in registers between the two passes, as the BF16 they
+// came as, and reads the row again beyond that.  1/sqrtf and a true division, not the fast-math forms.
+// Bound by latency: a launch, one trip to memory, two barriers.  So all loads (without a bias the weight's too) go out before the
+// first use, the kernel starts while the one before it finishes and lets the one behind it do the same; for that a CTA has to
+// fit beside a persistent GEMV's (123 registers x 384 threads), hence at most 64 registers.
 constexpr int kNormThreads = 256;
-constexpr int kNormCache = 6;                 // x 256 threads x 8 elements = 12288 columns from registers
+constexpr int kNormCache = 4, kNormBiasCache = 3;   // x 256 threads x 8 elements: 8192 (6144 with a bias) columns from registers
 
-__global__ void __launch_bounds__(kNormThreads)
+template <bool BIAS>
+__global__ void __launch_bounds__(kNormThreads, 4)
 rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __restrict__ bias,
                const __nv_bfloat16* __restrict__ weight, float eps, int K) {
     __shared__ float s_part[kNormThreads / 32];
-    __shared__ float s_inv;
+    constexpr int kHeld = BIAS ? kNormBiasCache : kNormCache;
     const int tid = threadIdx.x;
     const size_t row = (size_t)blockIdx.x * K;
     const int chunks = K >> 3;
-    auto load = [&](int c, float (&v)[8]) {
-        const uint4 a = *reinterpret_cast<const uint4*>(x + row + (size_t)c * 8);
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+    ptx::griddep_launch_dependents();
+    ptx::griddep_wait();                      // x (and bias) are the output of the kernel before this one
+    auto load_x = [&](int c) { return *reinterpret_cast<const uint4*>(x + row + (size_t)c * 8); };
+    auto load_b = [&](int c) { return __ldg(reinterpret_cast<const uint4*>(bias + row + (size_t)c * 8)); };
+    auto load_w = [&](int c) { return __ldg(reinterpret_cast<const uint4*>(weight + (size_t)c * 8)); };
+    auto values = [&](const uint4& a, const uint4& b, float (&v)[8]) {
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             v[2 * i] = __uint_as_float(aw[i] << 16);
             v[2 * i + 1] = __uint_as_float(aw[i] & 0xFFFF0000u);
-        }
-        if (bias) {
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias + row + (size_t)c * 8));
-            const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            if (BIAS) {
                 v[2 * i] += __uint_as_float(bw[i] << 16);
                 v[2 * i + 1] += __uint_as_float(bw[i] & 0xFFFF0000u);
             }
         }
     };
-    float cache[kNormCache][8];
+    uint4 xs[kHeld], bs[BIAS ? kHeld : 1], ws[BIAS ? 1 : kHeld];
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) {
+        const int c = tid + j * kNormThreads;
+        xs[j] = c < chunks ? load_x(c) : make_uint4(0u, 0u, 0u, 0u);
+        if (BIAS) bs[j] = c < chunks ? load_b(c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (!BIAS) {
+#pragma unroll
+        for (int j = 0; j < kHeld; ++j)
+            if (tid + j * kNormThreads < chunks) ws[j] = load_w(tid + j * kNormThreads);
+    }
     float ss = 0.0f;
 #pragma unroll
-    for (int j = 0; j < kNormCache; ++j) {
-        const int c = tid + j * kNormThreads;
-        if (c < chunks) {
-            load(c, cache[j]);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) ss = fmaf(cache[j][i], cache[j][i], ss);
-        }
-    }
-    for (int c = tid + kNormCache * kNormThreads; c < chunks; c += kNormThreads) {
+    for (int j = 0; j < kHeld; ++j) {            // chunks beyond the row are zeros
         float v[8];
-        load(c, v);
+        values(xs[j], bs[BIAS ? j : 0], v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
+    }
+    for (int c = tid + kHeld * kNormThreads; c < chunks; c += kNormThreads) {
+        float v[8];
+        values(load_x(c), BIAS ? load_b(c) : make_uint4(0u, 0u, 0u, 0u), v);
 #pragma unroll
         for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
     }
@@ -169,16 +224,11 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((tid & 31) == 0) s_part[tid >> 5] = ss;
     __syncthreads();
-    if (tid == 0) {
-        float t = 0.0f;
+    float t = 0.0f;
 #pragma unroll
-        for (int i = 0; i < kNormThreads / 32; ++i) t += s_part[i];
-        s_inv = 1.0f / sqrtf(t / (float)K + eps);
-    }
-    __syncthreads();
-    const float inv = s_inv;
-    auto store = [&](int c, const float (&v)[8]) {
-        const uint4 w4 = __ldg(reinterpret_cast<const uint4*>(weight + (size_t)c * 8));
+    for (int i = 0; i < kNormThreads / 32; ++i) t += s_part[i];      // the same sum in every thread
+    const float inv = 1.0f / sqrtf(t / (float)K + eps);
+    auto store = [&](int c, const float (&v)[8], const uint4& w4) {
         const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
         uint32_t o[4], r[4];
 #pragma unroll
@@ -189,19 +239,21 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
             const __nv_bfloat162 q = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
             r[i] = *reinterpret_cast<const uint32_t*>(&q);
         }
-        if (bias) *reinterpret_cast<uint4*>(x + row + (size_t)c * 8) = make_uint4(r[0], r[1], r[2], r[3]);
+        if (BIAS) *reinterpret_cast<uint4*>(x + row + (size_t)c * 8) = make_uint4(r[0], r[1], r[2], r[3]);
         *reinterpret_cast<uint4*>(out + row + (size_t)c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
     };
     // the uncached tail first: with a bias its x is still the old value only until it is stored
-    for (int c = tid + kNormCache * kNormThreads; c < chunks; c += kNormThreads) {
+    for (int c = tid + kHeld * kNormThreads; c < chunks; c += kNormThreads) {
         float v[8];
-        load(c, v);
-        store(c, v);
+        values(load_x(c), BIAS ? load_b(c) : make_uint4(0u, 0u, 0u, 0u), v);
+        store(c, v, load_w(c));
     }
 #pragma unroll
-    for (int j = 0; j < kNormCache; ++j) {
+    for (int j = 0; j < kHeld; ++j) {
         const int c = tid + j * kNormThreads;
-        if (c < chunks) store(c, cache[j]);
+        float v[8];
+        values(xs[j], bs[BIAS ? j : 0], v);
+        if (c < chunks) store(c, v, BIAS ? load_w(c) : ws[BIAS ? 0 : j]);
     }
 }
 
@@ -209,20 +261,18 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
 
 cudaError_t launch_rmsnorm(void* out, void* x, const void* bias, const void* weight, float eps, int M, int K,
                            cudaStream_t s) {
-    rmsnorm_kernel<<<M, kNormThreads, 0, s>>>(static_cast<__nv_bfloat16*>(out), static_cast<__nv_bfloat16*>(x),
-                                              static_cast<const __nv_bfloat16*>(bias),
-                                              static_cast<const __nv_bfloat16*>(weight), eps, K);
-    return cudaGetLastError();
+    __nv_bfloat16 *o = static_cast<__nv_bfloat16*>(out), *xb = static_cast<__nv_bfloat16*>(x);
+    const __nv_bfloat16 *b = static_cast<const __nv_bfloat16*>(bias), *w = static_cast<const __nv_bfloat16*>(weight);
+    return b ? launch_behind(rmsnorm_kernel<true>, M, kNormThreads, s, o, xb, b, w, eps, K)
+             : launch_behind(rmsnorm_kernel<false>, M, kNormThreads, s, o, xb, b, w, eps, K);
 }
 
 cudaError_t launch_swiglu(const void* gate, const void* up, long long row_stride_in, int M, int I,
                           void* out, long long row_stride_out, cudaStream_t s, bool interleaved) {
     const long long vecs = (long long)M * ((I + 7) >> 3);
-    swiglu_kernel<<<grid_for(vecs, 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(gate),
-                                                    static_cast<const __nv_bfloat16*>(up),
-                                                    static_cast<__nv_bfloat16*>(out), row_stride_in, row_stride_out, M, I,
-                                                    interleaved ? 1 : 0);
-    return cudaGetLastError();
+    return launch_behind(swiglu_kernel, grid_for(vecs, 256), 256, s, static_cast<const __nv_bfloat16*>(gate),
+                         static_cast<const __nv_bfloat16*>(up), static_cast<__nv_bfloat16*>(out), row_stride_in, row_stride_out, M,
+                         I, interleaved ? 1 : 0);
 }
 
 }  // namespace nvfp4
