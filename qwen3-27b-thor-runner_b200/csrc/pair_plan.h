@@ -19,7 +19,7 @@ constexpr int kBlocks = WK / BK;
 constexpr int kWPackedBytes = TR * WK / 2;     // 16 KB
 constexpr int kWScaleBytes = TR * WK / 16;     // 2 KB
 constexpr int kWStageBytes = kWPackedBytes + kWScaleBytes;
-constexpr int XK = 128;                        // k per token stage and A unit (two operand blocks)
+constexpr int XK = 128;                        // k per token stage and planned A unit (two operand blocks)
 constexpr int kDenseBlockBytes = TR * BK * 2;  // 16 KB
 constexpr int kDenseUnitBytes = 2 * kDenseBlockBytes;
 constexpr int kUnitCols = XK / 2;              // 64 TMEM columns of FP16 pairs per A unit (128 rows x 128 k)
@@ -122,7 +122,7 @@ constexpr Prices kPricesBf16 = {73.5, 68.0, 16384.0, 6.2, 18.8, 1060.0, 7900.0, 
 inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem) {
     const int kst = p.K / WK;
     p.row_tiles = (p.N + 2 * TR - 1) / (2 * TR);
-    // T up to 192: two accumulators and two 64-column A units fill tensor memory.  BF16 weights: up to 224, four 32 KB A units
+    // T up to 192: two accumulators and two 64-column A units (four of 64 k in the kernel) fill tensor memory.  BF16 weights: up to 224, four 32 KB A units
     // and three token stages; from 192 on only with two row tiles an item (one row tile takes two token stages a turn: 512 x 5120
     // x 8192 at T = 192 64 us, at T = 128 40) and never split all over.
     const int t_max = dense ? 224 : 192;

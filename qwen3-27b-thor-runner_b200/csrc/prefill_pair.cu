@@ -9,22 +9,25 @@
 // (512 x T: one accumulator each, every staged token block used twice).
 //   warp 0      TMA: raw weight stages (128 rows x 256 k: 16 KB codes, 2 KB scales) of this CTA, barriers of this CTA.
 //   warp 2      TMA: token blocks (T/2 x 64 k, FP16, 128-byte swizzle); both CTAs' blocks complete on the leader's barrier.
-//   warps 8-15  dequantise: thread = weight row = TMEM lane; 64 k of a 128-k unit each group, cvt.rn.f16x2.e2m1x2 + one f16x2 multiply by
+//   warps 8-15  dequantise: thread = weight row = TMEM lane; every other unit each group, cvt.rn.f16x2.e2m1x2 + one f16x2 multiply by
 //               the block scale (exact), tcgen05.st into a ring of A units; arrive on the leader's barrier.
-//   warps 1, 3  of the leader CTA issue the MMAs, one row tile or every other 128 k each; commits free the A units and token stages.
+//   warps 1, 3  of the leader CTA issue the MMAs, one row tile or every other unit each; commits free the A units and token stages, in
+//               both CTAs.
 //   warps 4-7, 16-19  epilogue: thread = weight row, registers = tokens: a warp stores 32 consecutive outputs of one token.
 //
 // What bounds it and why this form.  With both operands in shared memory (128 tokens x 256 rows per CTA, a dequantised block
 // for one or two token tiles) the shared memory was the bound: per 128 x 256 x 64 block the MMA reads 96 B/clk, the
 // dequantised block's stores 32-64, TMA and raw weights 50-70, of 128 B/clk.  From tensor memory the weights cost no
 // shared-memory bandwidth, and a pair of SMs stages each token once: 60-80 B/clk.  T is any multiple of 32, so 149 tokens are one
-// tile of 160 instead of two of 128.  What bounds it now is the issue of the MMAs beside the dequantising warps for
-// T < 192 (see the issuers), the power cap for long runs of T = 192, and for a few hundred tokens the reduction of split tiles.
-// Measured, the kernel before this form -> now, pre-pass included, weights from memory, four calls back to back after a pause (median;
-// a run of seconds at the power cap is up to a sixth slower): 34816 x 5120 at 149 / 256 / 1111 / 2048 / 4096 tokens 92 -> 51, 95 -> 84,
-// 385 -> 278, 637 -> 505, 1280 -> 1015 us; 5120 x 17408 with a residual 69 -> 40, 72 -> 59, 244 -> 155, 343 -> 288, 675 -> 542 us; BF16
-// 7168 x 5120 at 256 / 512 tokens 46 -> 26, 64 -> 42 us.
-// ncu at 34816 x 5120, 2048 tokens: tensor pipe active 81 % of the time, DRAM 14 %, L2 25 %, issue slots 45 %.
+// tile of 160 instead of two of 128.  Then the hand-overs were the bound: a wait that finds its phase complete costs a warp 60-130
+// clocks, a commit 75, and a group of dequantising warps spent 800 clocks on 64 k of every unit, 250 of them on arithmetic.  Now a
+// group takes whole units in turn (128 k: one wait, one arrival), where tensor memory leaves only two of those (T = 160, 192; FINE)
+// units of 64 k, and commits reach both CTAs' barriers themselves (a warp that passed them on came 200 clocks later).  Issuers at
+// T = 128 / 160 / 192: 100 / 100 / 120 clocks an MMA -> 75 / 81 / 110.  What bounds it now is the issue of the MMAs for T <= 128, the way
+// around the A ring at T = 192, draining the accumulators (5-8 thousand clocks an item), and the power cap for long runs.
+// Measured, before -> now, pre-pass included, weights from memory, calls back to back in short bursts: 34816 x 5120 at 100 / 149 / 256 /
+// 512 / 1111 / 2048 tokens 43.7 -> 38.8, 46.5 -> 43.8, 78.1 -> 70.5, 136 -> 133, 274 -> 266, 497 -> 483 us; 5120 x 17408 with a residual at
+// 100 / 256 / 1111 34.7 -> 32.4, 54.9 -> 51.2, 149 -> 143; BF16 5120 x 5120 at 512 34.7 -> 30.3 (two warps stream its blocks).
 //
 // Operands are FP16 because the hardware E2M1 conversion produces FP16 and every e2m1 x ue4m3 product is exact in FP16
 // (kind::f16 takes both operands in ONE 16-bit format).  A pre-pass turns the BF16 activations into FP16 with an exact
@@ -58,6 +61,8 @@ using namespace umma;
 constexpr int kThreads = 640;
 constexpr int kGroupWarps = 4, kEpiWarps = 4;  // two dequantising groups of four warps (one per TMEM lane quarter)
 constexpr int kMaxT = 256;                     // columns a partial slot has room for
+constexpr int kCoarseT = 128;                  // up to this many tokens a tile, an A unit of NVFP4 weights is 128 k
+constexpr int kRingMax = 2 * kMaxUnits;
 constexpr int kSlotFloats = TR * kMaxT;        // one FP32 partial: [token][row]
 
 struct PairParams : Plan {
@@ -89,18 +94,16 @@ struct Ring {
 };
 
 // ---------------------------------------------------------------- tcgen05, CTA pairs
-// The eight MMAs of 128 k on one accumulator (first clears it when `accumulate` is 0), from one elected lane of a converged
-// warp: A from tensor memory (8 columns per MMA) or from two shared-memory blocks, B from two blocks `step` (16-byte units)
-// apart.  Election and address arithmetic sit inside one asm block: the issuing warp shares its scheduler and instruction
-// cache with the dequantising warps, and every instruction of its loop counts.
+// The MMAs of a unit on one accumulator, which the first clears when `accumulate` is 0, from one elected lane of a converged
+// warp: eight (128 k, B in two blocks `step` 16-byte units apart) or, without `step`, the four of one block (64 k).  A from tensor
+// memory (8 columns per MMA) or from a shared-memory block.  Election and address arithmetic sit inside one asm block: the issuing warp shares its scheduler
+// and instruction cache with the dequantising warps, and every instruction of its loop counts.
 __device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t step, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a1, a2, a3, a4, a5, a6, a7;\n\t.reg .b64 s, b1, b2, b3, b4, b5, b6, b7;\n\t"
         "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tcvt.u64.u32 s, %5;\n\t"
-        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\tadd.u32 a4, %1, 32;\n\t"
-        "add.u32 a5, %1, 40;\n\tadd.u32 a6, %1, 48;\n\tadd.u32 a7, %1, 56;\n\t"
-        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\tadd.u64 b4, %2, s;\n\t"
-        "add.u64 b5, b4, 2;\n\tadd.u64 b6, b4, 4;\n\tadd.u64 b7, b4, 6;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\tadd.u32 a4, %1, 32;\n\tadd.u32 a5, %1, 40;\n\tadd.u32 a6, %1, 48;\n\tadd.u32 a7, %1, 56;\n\t"
+        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\tadd.u64 b4, %2, s;\n\tadd.u64 b5, b4, 2;\n\tadd.u64 b6, b4, 4;\n\tadd.u64 b7, b4, 6;\n\t"
         "elect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, t;\n\t"
@@ -113,34 +116,50 @@ __device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint
         ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(step)
         : "memory");
 }
-__device__ __forceinline__ void mma8_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t step, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 s, a1, a2, a3, a4, a5, a6, a7, b1, b2, b3, b4, b5, b6, b7;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tcvt.u64.u32 s, %5;\n\t"
-        "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\tadd.u64 a4, %1, 1024;\n\t"
-        "add.u64 a5, a4, 2;\n\tadd.u64 a6, a4, 4;\n\tadd.u64 a7, a4, 6;\n\t"
-        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\tadd.u64 b4, %2, s;\n\t"
-        "add.u64 b5, b4, 2;\n\tadd.u64 b6, b4, 4;\n\tadd.u64 b7, b4, 6;\n\t"
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], b2, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], b3, %3, t;\n\t}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma8_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
+        "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"
+        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
         "elect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, t;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, t;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, t;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a4, b4, %3, t;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a5, b5, %3, t;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a6, b6, %3, t;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a7, b7, %3, t;\n\t}"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(step)
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, t;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // Arrives on the leader's barrier at this shared-memory address once all MMAs issued so far have completed, in both CTAs
-// (converged warp).  Whichever warp of the leader waits there passes the news on to the other CTA.
+// (converged warp).
 __device__ __forceinline__ void commit_leader(uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
-// The leader's barrier has completed a phase: complete the same one of the other CTA.
+// ... and on the same barrier of the other CTA, `other` bytes on in the cluster's shared memory.
+__device__ __forceinline__ void commit_pair(uint32_t bar, uint32_t other) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b32 r;\n\tadd.u32 r, %0, %1;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [r];\n\t}" ::"r"(bar), "r"(other) : "memory");
+}
+// The leader's barrier has completed a phase: complete the same one of the other CTA.  For the token stages, whose ring is deep; a
+// commit of the issuers' own costs them 70 clocks more.
 __device__ __forceinline__ void relay(uint64_t* bar) {
     tc_fence_after();
     tc_fence_before();
@@ -263,7 +282,7 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
     }
 }
 
-template <int MODE>
+template <int MODE, bool FINE>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_scale, const PairParams p) {
@@ -273,13 +292,13 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     unsigned char* s_x = smem;
     unsigned char* s_w = s_x + p.x_stages * xbytes;                  // raw weight stages, or (DENSE) the ring of A blocks
     uint64_t* bars = reinterpret_cast<uint64_t*>(s_w + (MODE == kDense ? p.units * kDenseUnitBytes : p.w_stages * kWStageBytes));
-    uint64_t* afull = bars;                        // [kMaxUnits]   leader's, both CTAs' dequantisers (or TMA) arrive
-    uint64_t* aempty = afull + kMaxUnits;          // [kMaxUnits]   the leader's by commit, the other's by relay
-    uint64_t* xfull = aempty + kMaxUnits;          // [kMaxX]       leader's
-    uint64_t* xempty = xfull + kMaxX;              // [kMaxX]       the same
+    uint64_t* afull = bars;                        // [kRingMax]    leader's, both CTAs' dequantisers (or TMA) arrive
+    uint64_t* aempty = afull + kRingMax;          // [kRingMax]    each CTA its own, by commit
+    uint64_t* xfull = aempty + kRingMax;          // [kMaxX]       leader's
+    uint64_t* xempty = xfull + kMaxX;              // [kMaxX]       each CTA its own, by commit (!FINE: the other's by relay)
     uint64_t* wfull = xempty + kMaxX;              // [kMaxW]       each CTA its own
     uint64_t* wempty = wfull + kMaxW;              // [kMaxW]       each CTA its own
-    uint64_t* tfull = wempty + kMaxW;              // [kMaxAccs]    the same
+    uint64_t* tfull = wempty + kMaxW;              // [kMaxAccs]    each CTA its own, by commit
     uint64_t* tempty = tfull + kMaxAccs;           // [kMaxAccs]    leader's
     float* s_factor = reinterpret_cast<float*>(tempty + kMaxAccs);   // [kMaxT]
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_factor + kMaxT);
@@ -290,10 +309,14 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const int rank = (int)ptx::cluster_ctarank();
     const int kstages = p.K / WK;
     const bool all_reduce = p.dp_items == 0 && p.sk_tiles > 0;
+    // The ring of A: FINE two units of 64 k for each planned one, and in tensor memory two more in an odd 64 columns.
+    const int spare = FINE && MODE != kDense ? (p.a_col0 - p.accs * p.T) / kUnitCols * 2 : 0;
+    const int ring = FINE ? 2 * p.units + spare : p.units;
+    constexpr uint32_t kRingCols = FINE ? kUnitCols / 2 : kUnitCols;
 
     if (tid == 0) {
-        for (int i = 0; i < kMaxUnits; ++i) { ptx::mbar_init(&afull[i], MODE == kDense ? 1 : 4 * kGroupWarps); ptx::mbar_init(&aempty[i], 1); }
-        for (int i = 0; i < kMaxX; ++i) { ptx::mbar_init(&xfull[i], 1); ptx::mbar_init(&xempty[i], rank == 0 ? 2 : 1); }
+        for (int i = 0; i < kRingMax; ++i) { ptx::mbar_init(&afull[i], MODE == kDense ? 1 : 2 * kGroupWarps); ptx::mbar_init(&aempty[i], 1); }
+        for (int i = 0; i < kMaxX; ++i) { ptx::mbar_init(&xfull[i], 1); ptx::mbar_init(&xempty[i], FINE || rank == 0 ? 2 : 1); }
         for (int i = 0; i < kMaxW; ++i) { ptx::mbar_init(&wfull[i], 1); ptx::mbar_init(&wempty[i], 2 * kGroupWarps); }
         for (int i = 0; i < kMaxAccs; ++i) { ptx::mbar_init(&tfull[i], 1); ptx::mbar_init(&tempty[i], 4 * kEpiWarps); }
         *s_abort = 0;
@@ -307,42 +330,39 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     __syncthreads();
     ptx::cluster_sync();                   // both CTAs' barriers exist before anyone arrives on the other's
     tc_fence_after();
-    const uint32_t tmem_base = *s_tmem;
+    const uint32_t tmem_base = *s_tmem, a_col0 = tmem_base + (uint32_t)(p.a_col0 - spare * (kUnitCols / 2));
     ptx::griddep_launch_dependents();      // the next kernel in the stream may start its own prologue
 
     Work work(p, kstages, gridDim.x >> 1, blockIdx.x >> 1);
     Item it;
-    if (warp == 0) {
+    if (warp == 0 || (MODE == kDense && warp == 8)) {
         // ------------------------------------------------------------------ weight stream
         ptx::prefetch_tensormap(&tm_w);
         const uint64_t pol = ptx::policy_evict_first();
         int s = 0;
         uint32_t ph = 0;
         if (MODE == kDense) {
-            int turn = 0;                  // the first round of waits finds fresh barriers: nothing to relay
+            // Two warps, every other unit each, as the issuers: one warp's turn (wait, expectation, copy) takes as long as the MMAs.
+            const int me = warp >> 3;
+            const uint32_t full0 = ptx::mapa_shared(ptx::smem_u32(afull), 0);
+            s = me;
             ptx::griddep_wait();           // a BF16 weight may come from the kernel right before; there is no pre-pass to stream behind
             while (work.next(p, it)) {
-                for (int k = it.ks0 * WK; k < it.ks1 * WK; k += XK) {
-                    for (int r = 0; r < it.rows; ++r) {
-                        const bool ok = ptx::mbar_wait(&aempty[s], ph ^ 1u, s_abort, p.status, 0x410u + s);
-                        const bool pass = rank == 0 && turn++ >= p.units;
-                        if (ptx::elect_one() && ok) {
-                            if (pass) relay(&aempty[s]);
-                            if (rank == 0) ptx::mbar_arrive_expect_tx(&afull[s], 2 * kDenseUnitBytes);
-                            const uint32_t bar = ptx::mapa_shared(ptx::smem_u32(&afull[s]), 0);
-                            const int row = ((it.rt + r) * 2 + rank) * TR;
-                            ptx::tma_load_2d_pair(s_w + s * kDenseUnitBytes, &tm_w, bar, k, row, pol);
-                            ptx::tma_load_2d_pair(s_w + s * kDenseUnitBytes + kDenseBlockBytes, &tm_w, bar, k + BK, row, pol);
-                        }
-                        if (++s == p.units) { s = 0; ph ^= 1u; }
+                const int row = ((it.rt + (it.rows == 2 ? me : 0)) * 2 + rank) * TR, step = it.rows == 2 ? BK : 2 * BK;
+                for (int k = it.ks0 * WK + (it.rows == 2 ? 0 : me * BK); k < it.ks1 * WK; k += step) {
+                    const bool ok = ptx::mbar_wait(&aempty[s], ph ^ 1u, s_abort, p.status, 0x410u + s);
+                    if (ptx::elect_one() && ok) {
+                        if (rank == 0) ptx::mbar_arrive_expect_tx(&afull[s], 2 * kDenseBlockBytes);
+                        ptx::tma_load_2d_pair(s_w + s * kDenseBlockBytes, &tm_w, full0 + s * 8, k, row, pol);
                     }
+                    s += 2;
+                    if (s >= ring) { s = me; ph ^= 1u; }
                 }
             }
-            for (int i = 0; i < p.units; ++i) {      // nothing of the leader's may still be on its way to this CTA's barriers at the end
-                const bool ok = ptx::mbar_wait(&aempty[s], ph ^ 1u, s_abort, p.status, 0x418u);
-                const bool pass = rank == 0 && turn++ >= p.units;
-                if (ptx::elect_one() && ok && pass) relay(&aempty[s]);
-                if (++s == p.units) { s = 0; ph ^= 1u; }
+            for (int i = 0; i < ring; i += 2) {      // nothing of the leader's may still be on its way to this CTA's barriers at the end
+                ptx::mbar_wait(&aempty[s], ph ^ 1u, s_abort, p.status, 0x41Fu);
+                s += 2;
+                if (s >= ring) { s = me; ph ^= 1u; }
             }
         } else {
             ptx::prefetch_tensormap(&tm_scale);
@@ -375,7 +395,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         while (work.next(p, it)) {
             for (int k = it.ks0 * WK; k < it.ks1 * WK; k += XK) {
                 const bool ok = ptx::mbar_wait(&xempty[s], ph ^ 1u, s_abort, p.status, 0x400u + s);
-                const bool pass = rank == 0 && turn++ >= p.x_stages;      // the first round finds fresh barriers
+                const bool pass = !FINE && rank == 0 && turn++ >= p.x_stages;      // the first round finds fresh barriers
                 if (ptx::elect_one() && ok) {
                     if (pass) relay(&xempty[s]);
                     if (rank == 0) ptx::mbar_arrive_expect_tx(&xfull[s], 2u * (uint32_t)xbytes);
@@ -389,7 +409,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         }
         for (int i = 0; i < p.x_stages; ++i) {       // as above
             const bool ok = ptx::mbar_wait(&xempty[s], ph ^ 1u, s_abort, p.status, 0x40Eu);
-            const bool pass = rank == 0 && turn++ >= p.x_stages;
+            const bool pass = !FINE && rank == 0 && turn++ >= p.x_stages;
             if (ptx::elect_one() && ok && pass) relay(&xempty[s]);
             if (++s == p.x_stages) { s = 0; ph ^= 1u; }
         }
@@ -397,82 +417,105 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         // ------------------------------------------------------------------ MMA issuers (leader only): one warp per row tile
         if (rank == 0) {
             const int me = warp >> 1;
-            // The issue rate is the bound to watch: a loop that handled 64 k at a time (four MMAs, two waits, up to three commits)
-            // took 900 clocks a turn for 384 clocks of MMAs, waits that find their barrier completed costing ~100 each.  Hence
-            // 128 k a turn, and the next unit's (and token stage's) barrier is looked at before this unit's MMAs are issued
-            // and only waited for when that look came too early; and hence two warps, one per row tile and accumulator of an item.
-            // Two row tiles: each warp its own, on the same token stage.  One: the warps take its 128-k steps in turn, each on an
-            // accumulator of its own, which the epilogue adds.  Either way an item takes two units and two accumulators a turn.
+            // The issue rate is the bound to watch for T <= 128.  Measured alone, a warp takes 60 clocks an MMA whatever T is, ~75 a
+            // commit and up to ~130 for a wait that finds its phase complete; hence two warps, 128 k (eight MMAs) a turn, one look
+            // at all barriers of a turn, and waits only where that look came too early.
+            // Two row tiles: each warp its own, on the same token stage.  One: the warps take its units in turn, each on an
+            // accumulator of its own, which the epilogue adds.  Either way the warps take every other unit, and an item takes two
+            // accumulators.
+            // With accumulators of 160 and 192 columns tensor memory is left for two units of 128 k, and a unit's way around -- commit,
+            // dequantisers, stores, arrival -- takes longer than the other's eight MMAs: 1111 tokens ran at 120 clocks an MMA of 96.
+            // There a unit and a turn are 64 k: 81 clocks at T = 160 (of 80).
             // A parity wait cannot tell a phase from the one two before it, so whoever waits on a barrier must have seen
             // each of its phases: every warp waits for every token stage, and a stage is free when both have said so; the
             // numbers of units and accumulators are even, so a warp always meets the same ones.
-            Ring x(p.x_stages), u(p.units), t(p.accs);
+            Ring x(p.x_stages), u(ring), t(p.accs);
             u.advance(me);
             t.advance(me);
-            bool xready = false, aready = false, ok = true;
-            const uint32_t x0 = ptx::smem_u32(s_x), xstep = (uint32_t)(xbytes / 2) >> 4;
+            bool ok = true;
+            const uint32_t x0 = ptx::smem_u32(s_x), xhalf = (uint32_t)xbytes / 2;
             const uint32_t aempty0 = ptx::smem_u32(aempty), xempty0 = ptx::smem_u32(xempty), tfull0 = ptx::smem_u32(tfull);
+            const uint32_t other = ptx::mapa_shared(aempty0, 1) - aempty0;
             while (ok && work.next(p, it)) {
                 const bool one = it.rows == 1;
-                const int turns = (it.ks1 - it.ks0) * (WK / XK) / (one ? 2 : 1);
+                const bool pairwise = one && !FINE;            // two token stages a turn, one of them this warp's
+                const int turns = (it.ks1 - it.ks0) * (FINE ? 4 : 2) / (one ? 2 : 1);
                 const uint32_t d = tmem_base + (uint32_t)(t.i * p.T);
                 ok = ptx::mbar_wait(&tempty[t.i], t.phase ^ 1u, s_abort, p.status, 0x440u + t.i);
                 for (int turn = 0; turn < turns; ++turn) {
-                    if (!xready) ok = ok && ptx::mbar_wait(&xfull[x.i], x.phase, s_abort, p.status, 0x420u + x.i);
-                    const uint32_t xa = (uint32_t)x.i;
-                    x.advance(1);
-                    uint32_t xb = xa;
-                    if (one) {
-                        ok = ok && ptx::mbar_wait(&xfull[x.i], x.phase, s_abort, p.status, 0x420u + x.i);
-                        xb = (uint32_t)x.i;
-                        x.advance(1);
+                    const bool second = FINE && !one && (turn & 1);       // the other block of the last turn's token stage
+                    Ring y = x;                                           // pairwise: the stage behind x
+                    if (!FINE) y.advance(1);
+                    bool ready = ptx::mbar_test_wait(&afull[u.i], u.phase);
+                    if (!second) ready &= ptx::mbar_test_wait(&xfull[x.i], x.phase);
+                    if (pairwise) ready &= ptx::mbar_test_wait(&xfull[y.i], y.phase);
+                    if (!ready) {
+                        if (!second) ok = ok && ptx::mbar_wait(&xfull[x.i], x.phase, s_abort, p.status, 0x420u + x.i);
+                        if (pairwise) ok = ok && ptx::mbar_wait(&xfull[y.i], y.phase, s_abort, p.status, 0x420u + y.i);
+                        ok = ok && ptx::mbar_wait(&afull[u.i], u.phase, s_abort, p.status, 0x430u + u.i);
                     }
-                    if (!aready) ok = ok && ptx::mbar_wait(&afull[u.i], u.phase, s_abort, p.status, 0x430u + u.i);
                     // One decision for the warp: where a wait runs out in some lanes only, those would leave and the others
                     // stay for ever in the elections of the MMAs and commits below.
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t ui = (uint32_t)u.i;
+                    const uint64_t xdesc = umma_desc_sw128(x0 + (uint32_t)(pairwise && me ? y.i : x.i) * xbytes + (second || (FINE && one && me) ? xhalf : 0u));
+                    if (MODE == kDense) mma8_ss(d, umma_desc_sw128(ptx::smem_u32(s_w) + (uint32_t)u.i * kDenseBlockBytes), xdesc, p.idesc, (uint32_t)turn);
+                    else if (FINE) mma8_ts(d, a_col0 + (uint32_t)u.i * kRingCols, xdesc, p.idesc, (uint32_t)turn);
+                    else mma8_ts(d, a_col0 + (uint32_t)u.i * kRingCols, xdesc, xhalf >> 4, p.idesc, (uint32_t)turn);
+                    commit_pair(aempty0 + (uint32_t)u.i * 8, other);
                     u.advance(2);
-                    aready = ptx::mbar_test_wait(&afull[u.i], u.phase);
-                    xready = ptx::mbar_test_wait(&xfull[x.i], x.phase);
-                    const uint64_t xdesc = umma_desc_sw128(x0 + (me ? xb : xa) * xbytes);
-                    if (MODE == kDense) mma8_ss(d, umma_desc_sw128(ptx::smem_u32(s_w) + ui * kDenseUnitBytes), xdesc, xstep, p.idesc, (uint32_t)turn);
-                    else mma8_ts(d, tmem_base + (uint32_t)p.a_col0 + ui * kUnitCols, xdesc, xstep, p.idesc, (uint32_t)turn);
-                    commit_leader(aempty0 + ui * 8);
-                    commit_leader(xempty0 + xa * 8);
-                    if (one) commit_leader(xempty0 + xb * 8);
+                    if (FINE) {
+                        if (one || second) {
+                            commit_pair(xempty0 + (uint32_t)x.i * 8, other);
+                            x.advance(1);
+                        }
+                    } else {
+                        commit_leader(xempty0 + (uint32_t)x.i * 8);
+                        if (pairwise) commit_leader(xempty0 + (uint32_t)y.i * 8);
+                        x.advance(pairwise ? 2 : 1);
+                    }
                 }
-                if (ok) commit_leader(tfull0 + (uint32_t)t.i * 8);
+                if (ok) commit_pair(tfull0 + (uint32_t)t.i * 8, other);
                 t.advance(2);
             }
         }
     } else if (warp >= 8 && warp < 16) {
         if (MODE != kDense) {
         // ------------------------------------------------------------------ dequantise into TMEM
+        // Two groups of four warps fill the units in turn, the order the MMAs take them in: two row tiles, one each; one, every other
+        // unit.
         const int quarter = warp & 3;                     // TMEM lanes 32*quarter .. +31 (= warp id % 4)
-        const int group = (warp - 8) >> 2;                // the 64-k half of every unit this warp fills
+        const int group = (warp - 8) >> 2;
         const int row = quarter * 32 + lane;
         const int sw7 = row & 7;
-        int sw = 0, su = 0, turn = 0;
+        int sw = 0, su = group;
         uint32_t pw = 0, pu = 0;
-        const bool relays = rank == 0 && warp == 8 && lane == 0;
+        const uint32_t full0 = ptx::mapa_shared(ptx::smem_u32(afull), 0);
+        const uint32_t a_base = a_col0 + ((uint32_t)(quarter * 32) << 16);
         while (work.next(p, it)) {
+            const bool two = it.rows == 2;
             for (int ks = it.ks0; ks < it.ks1; ++ks) {
-                // the stages of the item's row tiles, their 128-k halves in turn: the order the MMAs take
-                for (int u = 0; u < 2 * it.rows; ++u) {
-                    const int r = it.rows == 2 ? u & 1 : 0, h = it.rows == 2 ? u >> 1 : u;
-                    int s = sw + r;
-                    uint32_t ph = pw;
-                    if (s >= p.w_stages) { s -= p.w_stages; ph ^= 1u; }
-                    if (h == 0) ptx::mbar_wait(&wfull[s], ph, s_abort, p.status, 0x450u + s);
-                    const unsigned char* wp = s_w + s * kWPackedBytes + row * 128;
-                    const unsigned char* ws = s_w + p.w_stages * kWPackedBytes + s * kWScaleBytes + row * 16;
-                    const int j = 2 * h + group;
+                // every warp waits for every stage, see the issuers
+                const int first = sw;
+                int st = sw;
+                ptx::mbar_wait(&wfull[sw], pw, s_abort, p.status, 0x450u + sw);
+                if (two) {
+                    if (++sw == p.w_stages) { sw = 0; pw ^= 1u; }
+                    ptx::mbar_wait(&wfull[sw], pw, s_abort, p.status, 0x450u + sw);
+                    if (group) st = sw;
+                }
+                const unsigned char* wp = s_w + st * kWPackedBytes + row * 128;
+                const unsigned char* ws = s_w + p.w_stages * kWPackedBytes + st * kWScaleBytes + row * 16;
+                // this group's 64-k blocks of the stage: two row tiles, all; one, every other unit's
+                const int j0 = two ? 0 : (FINE ? group : 2 * group), step = !two && FINE ? 2 : 1, count = two ? 4 : 2;
+                for (int i = 0; i < count; ++i) {
+                    const int j = j0 + i * step;
+                    const bool opens = FINE || !(i & 1), closes = FINE || (i & 1);
                     const uint4 q0 = *reinterpret_cast<const uint4*>(wp + (((2 * j) ^ sw7) << 4));
                     const uint4 q1 = *reinterpret_cast<const uint4*>(wp + (((2 * j + 1) ^ sw7) << 4));
                     const uint32_t scw = mask_scale_bytes(*reinterpret_cast<const uint32_t*>(ws + 4 * j));
+                    const bool ready = !opens || ptx::mbar_test_wait(&aempty[su], pu ^ 1u);
                     const uint32_t q[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
                     uint32_t o[2][16];
                     uint32_t one = 0u, more = 0u;          // kRounded: what a block's 1.0 comes to, and twice what 1.5 has over it
@@ -504,32 +547,31 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                             for (int i = 0; i < 4; ++i) o[c >> 2][(c & 3) * 4 + i] = ptx::mul_f16x2(e[i], S);
                         }
                     }
-                    const bool ok = ptx::mbar_wait(&aempty[su], pu ^ 1u, s_abort, p.status, 0x460u + su);
-                    tc_fence_after();
-                    if (relays && ok && turn >= p.units) relay(&aempty[su]);
-                    ++turn;
-                    __syncwarp();
-                    const uint32_t a_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(p.a_col0 + su * kUnitCols + group * (BK / 2));
+                    if (!ready) ptx::mbar_wait(&aempty[su], pu ^ 1u, s_abort, p.status, 0x460u + su);
+                    if (opens) tc_fence_after();
+                    const uint32_t a_addr = a_base + (uint32_t)su * kRingCols + (opens ? 0u : (uint32_t)(kUnitCols / 2));
                     tmem_st16(a_addr, o[0]);
                     tmem_st16(a_addr + 16, o[1]);
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&afull[su]), 0));
-                        if (h == 1) ptx::mbar_arrive(&wempty[s]);
+                    if (closes) {
+                        tmem_wait_st();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive_cluster(full0 + su * 8);
+                        su += 2;
+                        if (su >= ring) { su = group; pu ^= 1u; }
                     }
-                    if (++su == p.units) { su = 0; pu ^= 1u; }
                 }
-                sw += it.rows;
-                if (sw >= p.w_stages) { sw -= p.w_stages; pw ^= 1u; }
+                if (lane == 0) {
+                    ptx::mbar_arrive(&wempty[first]);
+                    if (two) ptx::mbar_arrive(&wempty[sw]);
+                }
+                if (++sw == p.w_stages) { sw = 0; pw ^= 1u; }
             }
         }
-        for (int i = 0; i < p.units; ++i) {          // as above
-            const bool ok = ptx::mbar_wait(&aempty[su], pu ^ 1u, s_abort, p.status, 0x46Eu);
-            if (relays && ok && turn >= p.units) relay(&aempty[su]);
-            ++turn;
-            if (++su == p.units) { su = 0; pu ^= 1u; }
+        for (int i = 0; i < ring; i += 2) {          // as above
+            ptx::mbar_wait(&aempty[su], pu ^ 1u, s_abort, p.status, 0x46Fu);
+            su += 2;
+            if (su >= ring) { su = group; pu ^= 1u; }
         }
         }
     } else {
@@ -566,8 +608,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 for (int i = 2 * begin + lane; i < 2 * end; i += 32)
                     ptx::prefetch_l2(src + (size_t)(i >> 1) * p.N + min(n - lane + 16 * (i & 1), p.N - 1));
             }
-            for (int i = t.i; i < t.i + 2; ++i)
-                if (ptx::mbar_wait(&tfull[i], t.phase, s_abort, p.status, 0x470u + i) && rank == 0 && tt == 0) relay(&tfull[i]);
+            for (int i = t.i; i < t.i + 2; ++i) ptx::mbar_wait(&tfull[i], t.phase, s_abort, p.status, 0x470u + i);
             __syncwarp();
             tc_fence_after();
             {
@@ -703,7 +744,7 @@ int plan_pair(PairParams& p, const nvfp4_device_info& dev, bool dense, int* smem
     return 2 * pairs;
 }
 
-template <int MODE>
+template <int MODE, bool FINE>
 cudaError_t launch(const PairParams& p, int grid, int smem, const CUtensorMap& tma, const CUtensorMap& tmw, const CUtensorMap& tms,
                    cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
@@ -720,7 +761,7 @@ cudaError_t launch(const PairParams& p, int grid, int smem, const CUtensorMap& t
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, prefill_pair_kernel<MODE>, tma, tmw, tms, p);
+    return cudaLaunchKernelEx(&cfg, prefill_pair_kernel<MODE, FINE>, tma, tmw, tms, p);
 }
 
 }  // namespace
@@ -743,9 +784,11 @@ size_t prefill_umma_scratch_bytes(int M, int /*N*/, int K) {
 }
 
 cudaError_t configure_prefill_umma(nvfp4_device_info& dev) {
-    cudaError_t e = configure_large_smem(prefill_pair_kernel<kExact>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kRounded>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kDense>, kSmemMax);
+    cudaError_t e = configure_large_smem(prefill_pair_kernel<kExact, false>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kExact, true>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kRounded, false>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kRounded, true>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kDense, true>, kSmemMax);
     if (e != cudaSuccess) return e;
     // The split tiles need every pair resident at once: no more pairs than the device can place.
     cudaLaunchConfig_t cfg{};
@@ -760,7 +803,7 @@ cudaError_t configure_prefill_umma(nvfp4_device_info& dev) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, prefill_pair_kernel<kExact>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&clusters, prefill_pair_kernel<kExact, true>, &cfg);
     if (e != cudaSuccess) return e;
     if (clusters < 1) return cudaErrorLaunchOutOfResources;
     dev.max_pairs = clusters;
@@ -807,9 +850,9 @@ cudaError_t launch_prefill_umma(const LinearArgs& a, nvfp4_device_info& dev, voi
         std::frexp(2688.0f * a.inv_gs, &ex);                 // 2688 / gs = f * 2^ex, f in [0.5, 1)
         p.wshift = std::ldexp(1.0f, 15 - ex);
         p.out_mul = std::ldexp(1.0f, ex - 15);
-        e = launch<kRounded>(p, grid, smem, tma, tmp, tms, s);
+        e = p.T > kCoarseT ? launch<kRounded, true>(p, grid, smem, tma, tmp, tms, s) : launch<kRounded, false>(p, grid, smem, tma, tmp, tms, s);
     } else {
-        e = launch<kExact>(p, grid, smem, tma, tmp, tms, s);
+        e = p.T > kCoarseT ? launch<kExact, true>(p, grid, smem, tma, tmp, tms, s) : launch<kExact, false>(p, grid, smem, tma, tmp, tms, s);
     }
     if (launches) *launches = 2;
     return e;
@@ -842,7 +885,7 @@ cudaError_t launch_dense_umma(const DenseArgs& a, nvfp4_device_info& dev, void* 
     p.status = static_cast<unsigned int*>(scratch);
     p.flags = reinterpret_cast<unsigned int*>(sk);
     p.partials = reinterpret_cast<float*>(sk + 4096);
-    const cudaError_t e = launch<kDense>(p, grid, smem, tma, tmw, tmw, s);
+    const cudaError_t e = launch<kDense, true>(p, grid, smem, tma, tmw, tmw, s);
     if (launches) *launches = 1;
     return e;
 }
