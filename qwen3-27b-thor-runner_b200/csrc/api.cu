@@ -23,7 +23,10 @@ struct nvfp4_handle {
     int prefill_impl = 0;
     int decode_max_m = 16;
     int wide_gemv = 1;                           // 9..16 tokens: one launch of the wide GEMV kernel
-    int skinny_min_m = 9, skinny_max_m = 64;     // token counts routed to the weights-in-TMEM kernel
+    // Token counts routed to the few-token kernel.  80: with the weights following the stream it is ahead of the prefill kernel on every
+    // shape measured at 65 and 80 tokens (34816 x 5120 38.4 -> 33.1 us, 5120 x 17408 31.6 -> 26.6, 7168 x 5120 20.8 -> 18.5, 2048 x 2048
+    // 10.9 -> 10.2), at 96 behind on some (5120 x 6144 20.0 -> 22.0).
+    int skinny_min_m = 9, skinny_max_m = 80;
     int fp4_native = 1;                          // the NVFP4 tensor-core GEMV (weights untouched, activations as NVFP4 terms) ...
     int fp4_min_m = 1;                           // ... from this token count on (up to 16)
     int fp4_stream_min_m = 10;                   // from this token count on its activations travel through the ring (decode_fp4_stream.cu)
@@ -171,7 +174,7 @@ int run_linear(nvfp4_handle* h, const LinearArgs& a, cudaStream_t s, size_t ws_b
         return cuda_status(e);
     }
     if (fast_path_wanted && a.M >= h->skinny_min_m && a.M <= h->skinny_max_m && skinny_umma_supported(a) &&
-        kDecodeScratchBytes + prefill_umma_reserved_bytes() <= ws_bytes) {
+        kDecodeScratchBytes + (a.M > 64 ? prefill_umma_scratch_bytes(a.M, a.N, a.K) : prefill_umma_reserved_bytes()) <= ws_bytes) {
         int nl = 0;
         cudaError_t e = launch_skinny_umma(a, h->dev, h->workspace, ws_bytes, kDecodeScratchBytes, &nl, s);
         h->launches += (unsigned long long)nl;

@@ -1,4 +1,4 @@
-// Linear layer for a few dozen tokens (1 <= M <= 128 supported, routed here for 17..64 by
+// Linear layer for a few dozen tokens (1 <= M <= 128 supported, routed here for 17..80 by
 // default): the dequantised weights are the A operand of tcgen05.mma and live in tensor memory,
 // the activations are the B operand.
 //
@@ -13,15 +13,15 @@
 //   warp 2      TMA producer of activation stages: tokens x 256 k of the FP16 activation copy (made
 //               by a small pre-pass kernel with an exact per-token power-of-two scale) as four
 //               128-byte-swizzled K-major blocks.  Starts once that pre-pass has finished
-//               (programmatic dependent launch); the weight stream above does not wait for it.
+//               (programmatic dependent launch); up to 64 tokens the weight stream above does not wait for it.
 //   warps 8-15  dequantise: thread = weight row = TMEM lane.  cvt.rn.f16x2.e2m1x2 + one f16x2
 //               multiply by the block scale (every product is exact in FP16), then tcgen05.st of
 //               the FP16 row segment into a ring of 64-column (128-k) A units in tensor memory;
 //               warps 8-11 fill the even units, warps 12-15 the odd ones, one lane quarter each.
-//   warp 1      one elected thread issues tcgen05.mma kind::f16 (A = FP16 in TMEM, B = FP16
-//               shared-memory descriptor, D = FP32 in TMEM, M = 128, N = tokens, K = 16) and
-//               commits completion to the mbarriers that recycle the buffers.
-//   warps 4-7   epilogue: tcgen05.ld of the FP32 accumulator (lane = weight row, column = token),
+//   warps 1, 3  issue tcgen05.mma kind::f16 (A = FP16 in TMEM, B = FP16 shared-memory descriptor, D =
+//               FP32 in TMEM, M = 128, N = tokens, K = 16) for one half of every stage each, on an
+//               accumulator of their own, and commit completion to the mbarriers that recycle the buffers.
+//   warps 4-7   epilogue: tcgen05.ld of the two FP32 accumulators (lane = weight row, column = token), their sum,
 //               per-token unscale, 1/global_scale and the residual in FP32, one rounding to BF16.
 // The (row tile, 256-k stage) units are spread evenly over one persistent CTA per SM (stream-K);
 // a row tile shared by several CTAs is summed from FP32 partial tiles in CTA order, each CTA
@@ -31,12 +31,15 @@
 // exact dequantised weights, BF16 activations, FP32 accumulation, one multiplication by
 // 1/global_scale, residual added in FP32 before the only rounding.
 //
-// Measured on B200 (an MLP of 5120 x 17408, 40 tokens, norm + gate_up + SwiGLU + down): 72.1 us, 94.8 us while the MMAs
-// were issued behind `lane == 0`.  The issue rate was the bound: one tcgen05.mma (128 x N x 16) per ~111-137 clocks
-// whatever N is; behind elect.sync (ptx::elect_one) it is one per 51 clocks up to N = 64 (2048 weights, 6.4 TB/s of
-// packed weights over the chip) and 68 at N = 128.  kind::f16 takes both operands in ONE 16-bit format:
-// an instruction descriptor with A = FP16 and B = BF16 raises an illegal-instruction fault,
-// hence the FP16 activation copy.
+// What bounds it.  The issue of the MMAs: a warp takes 60 clocks for one whatever N is (behind `lane == 0` instead of
+// elect.sync 111-137), ~75 for a commit and up to 130 for a wait that finds its phase complete.  One issuing warp took 1650 clocks a
+// stage, whose weights are 780 clocks of HBM; two take ~920, and the dequantising warps as long (arithmetic 480, the rest waits
+// and stores).  Then the epilogue (one load of the token's factor an element: 6800 clocks for 48 tokens; factors in shared memory
+// and sixteen elements at a time: 2500) and the reduction of split tiles (an element at a time; now four).
+// Measured, weights from memory, calls back to back, before -> now: 34816 x 5120 at 17 / 40 / 64 tokens 31.9 -> 24.7, 34.0 -> 26.0, 36.9 ->
+// 27.0 us; 5120 x 17408 with a residual 24.1 -> 20.9, 25.8 -> 22.0, 30.7 -> 22.5; 7168 x 5120 at 40 19.7 -> 14.3; 2048 x 2048 at 32 10.5 -> 7.5.
+// kind::f16 takes both operands in ONE 16-bit format: an instruction descriptor with A = FP16 and B = BF16 raises an
+// illegal-instruction fault, hence the FP16 activation copy.
 //
 // Every mbarrier wait is bounded; a wait that runs out records its code in the handle's status
 // word and the kernel winds down (TMEM is always freed).
@@ -60,7 +63,7 @@ constexpr int WK = 256;            // k per stage
 constexpr int kMaxTokens = 128;    // UMMA N <= 128 here: two accumulators + the A ring = 512 TMEM columns
 constexpr int kWPackedBytes = TR * WK / 2;     // 16 KB
 constexpr int kWScaleBytes = TR * WK / 16;     // 2 KB
-constexpr int kMaxWStages = 8, kMaxXStages = 4, kMaxAUnits = 6, kAccs = 2;
+constexpr int kMaxWStages = 8, kMaxXStages = 4, kMaxAUnits = 4, kMaxItems = 2;
 constexpr int kThreads = 512;
 constexpr int kDequantWarps = 8, kEpiWarps = 4;
 constexpr int kAUnitK = 128;       // k per A unit in tensor memory: half a stage, filled by four warps
@@ -78,7 +81,9 @@ struct SkinnyParams {
     int NT;                    // UMMA N: tokens rounded up to a multiple of 16
     int row_tiles, sk_tiles;   // tiles [0, sk_tiles) are split by k over all CTAs
     int w_stages, x_stages;
-    int acc_cols;              // TMEM columns per accumulator (two accumulators from column 0)
+    int follow;                // the weights wait for the stream (more than 64 tokens)
+    int acc_cols;              // TMEM columns per accumulator (from column 0: two an item, one of each issuer)
+    int items;                 // items whose accumulators fit: 2, one drained while the next is summed (more than 64 tokens: 1)
     int a_units, a_col0;       // ring of A units (64 columns each) behind the accumulators
     uint32_t idesc;
     float* partials;           // [grid][2][kMaxTokens][128] FP32
@@ -113,38 +118,45 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// One token of one weight row: scale, residual, round, store.
-__device__ __forceinline__ void store_output(const SkinnyParams& p, int m, int n, float v) {
-    const size_t o = (size_t)m * p.N + n;
-    float f = v * (p.unscale[m] * kBlockScaleUnfold * p.inv_gs);
-    if (p.residual) f += __bfloat162float(p.residual[o]);
-    p.C[o] = __float2bfloat16_rn(f);
-}
-
 // Reduction of one split row tile (as reduce_split of the prefill kernel: a flag per part, then every participant sums its slice).
 // The P participants each take 1/P of the tokens; with fewer tokens than participants the
 // rows are split instead.  t = 0..nthreads-1, nthreads a multiple of 128.
 __device__ __forceinline__ void reduce_split_rows(const SkinnyParams& p, unsigned int epoch, int tile, int kstages, int t,
-                                                  int nthreads, volatile int* s_abort) {
+                                                  int nthreads, const float* s_factor, volatile int* s_abort) {
     int first, last;
     split_tile_participants(p.sk_tiles, kstages, tile, first, last);
     if (!wait_split_tile_flags(p.flags, epoch, first, last, t, s_abort, p.status)) return;
     const int P = last - first + 1, me = blockIdx.x - first;
-    const int total = p.M * TR;                      // elements [token][row] of the tile that matter
+    const int total = p.M * (TR / 4);                // chunks of four rows [token][chunk] of the tile that matter
     const int e0 = (int)((long long)me * total / P), e1 = (int)((long long)(me + 1) * total / P);
-    const float* head = p.partials + ((size_t)first * 2 + 1) * kSlotFloats;
+    const float4* parts = reinterpret_cast<const float4*>(p.partials);
+    const float4* head = parts + ((size_t)first * 2 + 1) * (kSlotFloats / 4);
     for (int e = e0 + t; e < e1; e += nthreads) {
-        float s = __ldcg(head + e);
-        for (int c = first + 1; c <= last; c += 8) {
-            float x[8];
+        float4 s = __ldcg(head + e);
+        for (int c = first + 1; c <= last; c += 4) {
+            float4 x[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)          // eight loads in flight; absent participants add zero
-                x[i] = c + i <= last ? __ldcg(p.partials + (size_t)(c + i) * 2 * kSlotFloats + e) : 0.0f;
+            for (int i = 0; i < 4; ++i)          // four loads in flight; absent participants add zero
+                x[i] = c + i <= last ? __ldcg(parts + (size_t)(c + i) * 2 * (kSlotFloats / 4) + e) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s += x[i];
+            for (int i = 0; i < 4; ++i) { s.x += x[i].x; s.y += x[i].y; s.z += x[i].z; s.w += x[i].w; }
         }
-        const int m = e / TR, n = tile * TR + (e % TR);
-        if (n < p.N) store_output(p, m, n, s);
+        const int m = e / (TR / 4), n = tile * TR + (e % (TR / 4)) * 4;
+        const float k = s_factor[m];
+        const float v[4] = {s.x * k, s.y * k, s.z * k, s.w * k};
+        const size_t o = (size_t)m * p.N + n;
+        if ((p.N & 3) == 0) {                    // chunks inside or outside as a whole, eight bytes aligned
+            if (n >= p.N) continue;
+            uint2 r = make_uint2(0u, 0u);
+            if (p.residual) r = *reinterpret_cast<const uint2*>(p.residual + o);
+            const __nv_bfloat162 a = __floats2bfloat162_rn(v[0] + __uint_as_float(r.x << 16), v[1] + __uint_as_float(r.x & 0xFFFF0000u));
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2] + __uint_as_float(r.y << 16), v[3] + __uint_as_float(r.y & 0xFFFF0000u));
+            *reinterpret_cast<uint2*>(p.C + o) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (n + i < p.N) p.C[o + i] = __float2bfloat16_rn(v[i] + (p.residual ? __bfloat162float(p.residual[o + i]) : 0.0f));
     }
 }
 
@@ -167,9 +179,10 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
     uint64_t* xempty = xfull + kMaxXStages;        // [kMaxXStages]
     uint64_t* afull = xempty + kMaxXStages;        // [kMaxAUnits]
     uint64_t* aempty = afull + kMaxAUnits;         // [kMaxAUnits]
-    uint64_t* tfull = aempty + kMaxAUnits;         // [kAccs]
-    uint64_t* tempty = tfull + kAccs;              // [kAccs]
-    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(tempty + kAccs);
+    uint64_t* tfull = aempty + kMaxAUnits;         // [kMaxItems]
+    uint64_t* tempty = tfull + kMaxItems;              // [kMaxItems]
+    float* s_factor = reinterpret_cast<float*>(tempty + kMaxItems);      // [kMaxTokens] what a token's sums are multiplied by
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_factor + kMaxTokens);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     volatile unsigned int* s_epoch = reinterpret_cast<volatile unsigned int*>(s_tmem + 2);
 
@@ -179,9 +192,9 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
 
     if (tid == 0) {
         for (int i = 0; i < kMaxWStages; ++i) { ptx::mbar_init(&wfull[i], 1); ptx::mbar_init(&wempty[i], kDequantWarps); }
-        for (int i = 0; i < kMaxXStages; ++i) { ptx::mbar_init(&xfull[i], 1); ptx::mbar_init(&xempty[i], 1); }
+        for (int i = 0; i < kMaxXStages; ++i) { ptx::mbar_init(&xfull[i], 1); ptx::mbar_init(&xempty[i], 2); }
         for (int i = 0; i < kMaxAUnits; ++i) { ptx::mbar_init(&afull[i], kDequantWarps / 2); ptx::mbar_init(&aempty[i], 1); }
-        for (int i = 0; i < kAccs; ++i) { ptx::mbar_init(&tfull[i], 1); ptx::mbar_init(&tempty[i], kEpiWarps); }
+        for (int i = 0; i < kMaxItems; ++i) { ptx::mbar_init(&tfull[i], 2); ptx::mbar_init(&tempty[i], kEpiWarps); }
         *s_abort = 0;
         ptx::fence_mbar_init();
     }
@@ -197,6 +210,7 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
         {
             ptx::prefetch_tensormap(&tm_packed);
             ptx::prefetch_tensormap(&tm_scale);
+            if (p.follow) ptx::griddep_wait();
             const uint64_t pol = ptx::policy_evict_first();
             int sw = 0;
             uint32_t pw = 0;
@@ -237,42 +251,43 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
                 }
             }
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
+    } else if (warp == 1 || warp == 3) {
+        // ------------------------------------------------------------------ MMA issuers
+        // One half of every stage each (its A units are every other one), on an accumulator of its own; the epilogue adds the two.
         {
-            int sx = 0, au = 0, acc = 0;
+            const int me = warp >> 1;
+            int sx = 0, au = me, slot = 0;
             uint32_t px = 0, pa = 0, pt = 0;
             Schedule sched(p.sk_tiles, p.row_tiles, kstages);
             Segment sg;
             while (sched.next(sg)) {
-                ptx::mbar_wait(&tempty[acc], pt ^ 1u, s_abort, p.status, 0x540u + acc);
+                ptx::mbar_wait(&tempty[slot], pt ^ 1u, s_abort, p.status, 0x540u + slot);
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.acc_cols);
+                const uint32_t d_tmem = tmem_base + (uint32_t)((2 * slot + me) * p.acc_cols);
                 for (int ks = sg.ks0; ks < sg.ks1; ++ks) {
-                    ptx::mbar_wait(&xfull[sx], px, s_abort, p.status, 0x520u + sx);
-                    const uint64_t xdesc = umma_desc_sw128(ptx::smem_u32(s_x + sx * xbytes));
-#pragma unroll
-                    for (int h = 0; h < WK / kAUnitK; ++h) {
+                    const bool ready = (int)ptx::mbar_test_wait(&xfull[sx], px) & (int)ptx::mbar_test_wait(&afull[au], pa);
+                    if (!ready) {
+                        ptx::mbar_wait(&xfull[sx], px, s_abort, p.status, 0x520u + sx);
                         ptx::mbar_wait(&afull[au], pa, s_abort, p.status, 0x530u + au);
-                        tc_fence_after();
-                        const uint32_t a_tmem = tmem_base + (uint32_t)(p.a_col0 + au * kAUnitCols);
-                        if (ptx::elect_one()) {
-#pragma unroll
-                            for (int k = 0; k < kAUnitK / 16; ++k) {
-                                const int kk = h * (kAUnitK / 16) + k;      // 16-k step inside the stage
-                                // 64-k block kk/4 of the stage (NT x 128 B each), 32 bytes per step inside it
-                                const uint64_t bdesc = xdesc + (uint64_t)(((kk >> 2) * (p.NT * 128) + (kk & 3) * 32) >> 4);
-                                umma_f16_ts(d_tmem, a_tmem + k * 8, bdesc, p.idesc, (ks > sg.ks0 || kk > 0) ? 1u : 0u);
-                            }
-                            umma_commit(&aempty[au]);  // the A unit is free once these MMAs have read it
-                        }
-                        if (++au == p.a_units) { au = 0; pa ^= 1u; }
                     }
-                    if (ptx::elect_one()) umma_commit(&xempty[sx]);
+                    tc_fence_after();
+                    const uint64_t xdesc = umma_desc_sw128(ptx::smem_u32(s_x + sx * xbytes + me * (p.NT * 256)));      // 64-k blocks of NT x 128 B
+                    const uint32_t a_tmem = tmem_base + (uint32_t)(p.a_col0 + au * kAUnitCols);
+                    if (ptx::elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < kAUnitK / 16; ++k) {
+                            const uint64_t bdesc = xdesc + (uint64_t)(((k >> 2) * (p.NT * 128) + (k & 3) * 32) >> 4);
+                            umma_f16_ts(d_tmem, a_tmem + k * 8, bdesc, p.idesc, (ks > sg.ks0 || k > 0) ? 1u : 0u);
+                        }
+                        umma_commit(&aempty[au]);          // the A unit is free once these MMAs have read it
+                        umma_commit(&xempty[sx]);
+                    }
+                    au += 2;
+                    if (au >= p.a_units) { au = me; pa ^= 1u; }
                     if (++sx == p.x_stages) { sx = 0; px ^= 1u; }
                 }
-                if (ptx::elect_one()) umma_commit(&tfull[acc]);
-                if (++acc == kAccs) { acc = 0; pt ^= 1u; }
+                if (ptx::elect_one()) umma_commit(&tfull[slot]);
+                if (++slot == p.items) { slot = 0; pt ^= 1u; }
             }
         }
     } else if (warp >= 8) {
@@ -294,26 +309,28 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
 #pragma unroll
                 for (int c = 0; c < 4; ++c) q[c] = *reinterpret_cast<const uint4*>(wp + (((4 * half + c) ^ sw7) << 4));
                 const uint2 sc = *reinterpret_cast<const uint2*>(s_ws + sw * kWScaleBytes + row * 16 + 8 * half);
-                ptx::mbar_wait(&aempty[au], pa ^ 1u, s_abort, p.status, 0x560u + au);
-                tc_fence_after();
-                const uint32_t a_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(p.a_col0 + au * kAUnitCols);
+                const bool ready = ptx::mbar_test_wait(&aempty[au], pa ^ 1u);
+                uint32_t r[4][16];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {              // chunk c: 32 k = two block scales = 16 columns
                     const uint32_t w[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
                     const uint32_t scw = mask_scale_bytes(c < 2 ? sc.x : sc.y);
                     const uint32_t S0 = scale_byte_to_f16x2(scw, 2 * (c & 1));          // scale / 2^8, undone in the epilogue
                     const uint32_t S1 = scale_byte_to_f16x2(scw, 2 * (c & 1) + 1);
-                    uint32_t r[16];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         uint32_t e[4];
                         ptx::cvt_e2m1x8_to_f16x2(w[i], e);
                         const uint32_t S = i < 2 ? S0 : S1;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) r[4 * i + j] = ptx::mul_f16x2(e[j], S);
+                        for (int j = 0; j < 4; ++j) r[c][4 * i + j] = ptx::mul_f16x2(e[j], S);
                     }
-                    tmem_st16(a_addr + c * 16, r);
                 }
+                if (!ready) ptx::mbar_wait(&aempty[au], pa ^ 1u, s_abort, p.status, 0x560u + au);
+                tc_fence_after();
+                const uint32_t a_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(p.a_col0 + au * kAUnitCols);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_st16(a_addr + c * 16, r[c]);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
@@ -330,12 +347,13 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
         // ------------------------------------------------------------------ epilogue: thread = weight row
         const int ew = warp - 4;                          // TMEM lanes 32*ew .. +31 (= warp id % 4)
         const int te = ew * 32 + lane;
-        int acc = 0;
+        int acc = 0;                                      // item slot
         uint32_t pt = 0;
         int pend[2] = {-1, -1};
         ptx::griddep_wait();                              // C, the residual and the scratch belong to earlier kernels until now
         // the tag of this launch's split-tile flags, from the counter in the scratch; the four epilogue warps share it
         if (te == 0) *s_epoch = ptx::take_launch_epoch(p.status);
+        if (te < p.NT) s_factor[te] = te < p.M ? p.unscale[te] * kBlockScaleUnfold * p.inv_gs : 0.0f;
         ptx::named_barrier_sync(1, kEpiWarps * 32);
         const unsigned int epoch = *s_epoch;
         Schedule sched(p.sk_tiles, p.row_tiles, kstages);
@@ -344,25 +362,54 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
         while (more) {
             const int n = sg.tile * TR + te;
             const bool complete = sg.ks0 == 0 && sg.ks1 == kstages;
+            // Sixteen tokens of the residual, all in flight together (it may be C itself): asked for a chunk ahead, the first before the
+            // wait.
+            unsigned short res[16];
+            const size_t o0 = (size_t)n;
+            auto ask = [&](int c0) {
+                const unsigned short* src = reinterpret_cast<const unsigned short*>(p.residual) + o0 + (size_t)c0 * p.N;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) res[i] = c0 + i < p.M ? src[(size_t)i * p.N] : (unsigned short)0;
+            };
+            const bool adds = p.residual && complete && n < p.N;
+            if (adds) ask(0);
             ptx::mbar_wait(&tfull[acc], pt, s_abort, p.status, 0x570u + acc);
             tc_fence_after();
-            const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * p.acc_cols);
+            const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(2 * acc * p.acc_cols);
             const int which = sg.ks0 == 0 ? 1 : 0;        // head of a tile (span end) or tail (span start)
             float* slot = p.partials + ((size_t)blockIdx.x * 2 + which) * kSlotFloats;
             for (int c0 = 0; c0 < p.NT; c0 += 16) {
-                uint32_t r[16];
+                uint32_t r[16], r2[16];
                 tmem_ld16(t_addr + c0, r);
-                if (complete) {
-                    if (n < p.N) {
+                tmem_ld16(t_addr + p.acc_cols + c0, r2);
+                float f[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (c0 + i < p.M) store_output(p, c0 + i, n, __uint_as_float(r[i]));
-                    }
-                } else {
+                for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(r[i]) + __uint_as_float(r2[i]);
+                const int cnt = min(16, p.M - c0);
+                if (!complete) {
+                    float* dst = slot + c0 * TR + te;
 #pragma unroll
                     for (int i = 0; i < 16; ++i)           // [token][row]: a warp stores 128 contiguous bytes
-                        if (c0 + i < p.M) __stcg(slot + (c0 + i) * TR + te, __uint_as_float(r[i]));
+                        if (i < cnt) __stcg(dst + i * TR, f[i]);
+                    continue;
                 }
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(s_factor + c0 + i);
+                    f[i] *= k4.x;
+                    f[i + 1] *= k4.y;
+                    f[i + 2] *= k4.z;
+                    f[i + 3] *= k4.w;
+                }
+                if (n >= p.N) continue;
+                if (adds) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) f[i] += bf16_bits_to_float(res[i]);
+                    if (c0 + 16 < p.M) ask(c0 + 16);
+                }
+                __nv_bfloat16* dst = p.C + o0 + (size_t)c0 * p.N;
+#pragma unroll
+                for (int i = 0; i < 16; ++i, dst += p.N) if (i < cnt) *dst = __float2bfloat16_rn(f[i]);
             }
             if (!complete) {
                 __threadfence();
@@ -373,14 +420,14 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&tempty[acc]);
-            if (++acc == kAccs) { acc = 0; pt ^= 1u; }
+            if (++acc == p.items) { acc = 0; pt ^= 1u; }
             more = sched.next(sg);
             // Whole tiles follow the stream-K region: these four warps reduce the split tiles now,
             // behind the MMAs of the next tiles.  (With no whole tiles all warps do it at the end.)
             if (!all_reduce && (pend[0] >= 0 || pend[1] >= 0) && (!more || sg.tile >= p.sk_tiles)) {
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
-                    if (pend[w] >= 0) reduce_split_rows(p, epoch, pend[w], kstages, te, kEpiWarps * 32, s_abort);
+                    if (pend[w] >= 0) reduce_split_rows(p, epoch, pend[w], kstages, te, kEpiWarps * 32, s_factor, s_abort);
                     pend[w] = -1;
                 }
             }
@@ -400,7 +447,7 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
         split_tiles_of_cta(p.sk_tiles, kstages, split);
 #pragma unroll
         for (int w = 0; w < 2; ++w)
-            if (split[w] >= 0) reduce_split_rows(p, epoch, split[w], kstages, tid, kThreads, s_abort);
+            if (split[w] >= 0) reduce_split_rows(p, epoch, split[w], kstages, tid, kThreads, s_factor, s_abort);
     }
 }
 
@@ -416,6 +463,7 @@ bool plan_skinny(const LinearArgs& a, const nvfp4_device_info& dev, SkinnyPlan* 
     p.M = a.M; p.N = a.N; p.K = a.K;
     p.NT = (a.M + 15) / 16 * 16;
     p.row_tiles = (a.N + TR - 1) / TR;
+    p.follow = a.M > 64 ? 1 : 0;
     const int kstages = a.K / WK;
     const int xbytes = p.NT * WK * 2;
     p.x_stages = p.NT <= 32 ? 4 : (p.NT <= 64 ? 3 : 2);
@@ -423,10 +471,11 @@ bool plan_skinny(const LinearArgs& a, const nvfp4_device_info& dev, SkinnyPlan* 
     if (ws > kMaxWStages) ws = kMaxWStages;
     if (ws < 2) return false;
     p.w_stages = ws;
-    out->smem = 1024 + p.x_stages * xbytes + ws * (kWPackedBytes + kWScaleBytes) + 512;
-    // Tensor memory (512 columns): two accumulators, then as many 64-column A units as fit (even count).
+    out->smem = 1024 + p.x_stages * xbytes + ws * (kWPackedBytes + kWScaleBytes) + 1024;      // barriers, token factors, a few words
+    // Tensor memory (512 columns): two accumulators an item, then four 64-column A units.
     p.acc_cols = p.NT <= 64 ? 64 : 128;
-    p.a_units = p.NT <= 64 ? 6 : 4;
+    p.items = p.NT <= 64 ? 2 : 1;
+    p.a_units = kMaxAUnits;
     p.a_col0 = 512 - p.a_units * kAUnitCols;
     // kind::f16: D = FP32, A = B = FP16, both K-major, M = 128, N = NT
     p.idesc = (1u << 4) | ((uint32_t)(p.NT >> 3) << 17) | ((uint32_t)(TR >> 4) << 24);

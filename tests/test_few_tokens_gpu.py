@@ -1,0 +1,87 @@
+"""The few-token kernel where its two issuing warps, its reduction in chunks of four rows and its token range can go wrong."""
+import numpy as np
+import pytest
+
+import oracle_binding as ob
+import util
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-3      # BF16 rounding of sums in another order: last bits flip in a few elements
+
+
+@pytest.fixture(scope="module")
+def handle():
+    import nvfp4
+    h = nvfp4.Handle(0, 128 << 20)
+    yield h
+    h.close()
+
+
+@pytest.mark.parametrize("M,N,K,res", [
+    (17, 128, 256, False),        # one stage: a unit for each issuer
+    (33, 130, 512, True),         # two rows in the second tile, N % 4 != 0
+    (64, 1001, 5120, True),       # split tiles, odd N: scalar stores in the reduction
+    (48, 1004, 5120, True),       # split tiles, N % 4 == 0: eight-byte ones, the last tile cut
+    (64, 19200, 1024, True),      # 150 tiles: two items a CTA on the first slots, accumulators in turn
+    (65, 512, 5120, True),        # beyond 64 tokens: one item at a time in tensor memory
+    (80, 19208, 768, False),      # the same with more tiles than CTAs, the last one cut
+    (80, 640, 17408, True),       # deep split
+])
+def test_against_the_oracle(handle, M, N, K, res):
+    import torch
+    packed, scale = util.make_weight(N, K, seed=M + N, sigma=0.14)
+    A, R = util.make_bf16((M, K), seed=M), util.make_bf16((M, N), seed=N)
+    dA, dP, dS = util.to_dev(A), util.to_dev(packed), util.to_dev(scale)
+    outs = []
+    for _ in range(2):
+        C = util.to_dev(R) if res else torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        handle.linear(dA, M, dP, dS, 1.5, N, K, C, residual=C if res else None)
+        torch.cuda.synchronize()
+        outs.append(util.to_host_u16(C))
+    assert handle.device_status() == 0
+    assert np.array_equal(outs[0], outs[1])               # a fixed order of summation
+    # the kernel's arithmetic: exact weights, 1 / gs once in FP32 (the oracle's GEMM form rounds the scaled weights to BF16)
+    assert ob.rel_frobenius(outs[0], ob.linear(A, packed, scale, 1.5, residual=R if res else None, mode=ob.GEMV, threads=8)) <= TOL
+
+
+@pytest.mark.parametrize("M", [65, 80])
+def test_weights_follow_the_stream_beyond_64_tokens(handle, M):
+    """A weight copied into place right before the call, on the same stream, is the one that is used."""
+    import torch
+    N, K = 4096, 2048
+    sets = [tuple(util.to_dev(a) for a in util.make_weight(N, K, seed=s)) for s in (1, 2)]
+    A = util.to_dev(util.make_bf16((M, K), seed=3))
+    packed, scale = torch.empty_like(sets[0][0]), torch.empty_like(sets[0][1])
+    want = []
+    for p, s in sets:
+        C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        torch.cuda.synchronize()
+        handle.linear(A, M, p, s, 1.0, N, K, C)
+        torch.cuda.synchronize()
+        want.append(util.to_host_u16(C))
+    for i in range(12):
+        C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        packed.copy_(sets[i % 2][0])
+        scale.copy_(sets[i % 2][1])
+        handle.linear(A, M, packed, scale, 1.0, N, K, C)
+        torch.cuda.synchronize()
+        assert np.array_equal(util.to_host_u16(C), want[i % 2]), i
+
+
+def test_a_workspace_too_small_is_refused_as_before(handle):
+    """65 to 80 tokens on a handle sized for fewer: the same refusal as above, before any launch."""
+    import ctypes
+    import torch
+    import nvfp4
+    M, N, K = 80, 128, 17408
+    size = ctypes.c_size_t(0)
+    nvfp4.load().nvfp4_workspace_bytes(17, N, 256, ctypes.byref(size))
+    h = nvfp4.Handle(0, size.value)
+    try:
+        p, s = (util.to_dev(a) for a in util.make_weight(N, K, seed=1))
+        C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        with pytest.raises(nvfp4.Nvfp4Error, match="workspace"):
+            h.linear(util.to_dev(util.make_bf16((M, K), seed=2)), M, p, s, 1.0, N, K, C)
+        assert h.launch_count() == 0 and not C.any()
+    finally:
+        h.close()
