@@ -282,7 +282,12 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
     }
 }
 
-template <int MODE, bool FINE>
+// SPLIT: what the plan left to split by k.  An instantiation each, because the registers run out (96 a thread): with the code of
+// parts and reduction in one kernel every call paid for its spills, 0.5-1 us (149 x 5120 x 17408 35.7 -> 34.4 us, BF16 100 x 5120 x 5120
+// 19.1 -> 17.9), and whole items had none left to ask for the residual a chunk ahead (2048 x 5120 x 5120 with a residual 92 -> 83.4).
+enum Split { kWhole = 0, kAllSplit = 1, kTailSplit = 2 };
+
+template <int MODE, bool FINE, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_scale, const PairParams p) {
@@ -308,7 +313,6 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)ptx::cluster_ctarank();
     const int kstages = p.K / WK;
-    const bool all_reduce = p.dp_items == 0 && p.sk_tiles > 0;
     // The ring of A: FINE two units of 64 k for each planned one, and in tensor memory two more in an odd 64 columns.
     const int spare = FINE && MODE != kDense ? (p.a_col0 - p.accs * p.T) / kUnitCols * 2 : 0;
     const int ring = FINE ? 2 * p.units + spare : p.units;
@@ -597,7 +601,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 ptx::named_barrier_sync(1, 2 * kEpiWarps * 32);
             }
             const float* factor = s_factor;
-            const bool complete = it.ks0 == 0 && it.ks1 == kstages;
+            const bool complete = SPLIT == kWhole || (SPLIT == kTailSplit && it.ks0 == 0 && it.ks1 == kstages);      // all split: no part is a whole tile
             const int which = it.ks0 == 0 ? 1 : 0;        // head of a tile (span end) or tail (span start)
             const bool two = it.rows == 2;
             // Both groups wait for and free both accumulators (accs is even: a pair never wraps).
@@ -608,6 +612,14 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 for (int i = 2 * begin + lane; i < 2 * end; i += 32)
                     ptx::prefetch_l2(src + (size_t)(i >> 1) * p.N + min(n - lane + 16 * (i & 1), p.N - 1));
             }
+            // the residual of sixteen tokens, all in flight together (it may be C itself): asked for a chunk ahead, the first before the wait
+            unsigned short res[16];
+            auto ask = [&](int c0) {
+                const unsigned short* src = reinterpret_cast<const unsigned short*>(p.residual) + (size_t)(m0 + c0) * p.N + n;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) res[i] = c0 + i < end ? src[(size_t)i * p.N] : (unsigned short)0;
+            };
+            if (SPLIT == kWhole && p.residual && n < p.N) ask(begin);
             for (int i = t.i; i < t.i + 2; ++i) ptx::mbar_wait(&tfull[i], t.phase, s_abort, p.status, 0x470u + i);
             __syncwarp();
             tc_fence_after();
@@ -661,11 +673,10 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                         continue;
                     }
                     if (p.residual) {
-                        __nv_bfloat16 res[16];                 // all in flight together; the residual may be C itself
+                        if (SPLIT != kWhole) ask(c0);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) res[i] = i < cnt ? p.residual[o + (size_t)i * p.N] : __nv_bfloat16(0.0f);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) f[i] += __bfloat162float(res[i]);
+                        for (int i = 0; i < 16; ++i) f[i] += bf16_bits_to_float(res[i]);
+                        if (SPLIT == kWhole && c0 + 16 < end) ask(c0 + 16);
                     }
                     __nv_bfloat16* dst = p.C + o;
                     if (cnt == 16) {
@@ -693,7 +704,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
             more = work.next(p, it);
             // Whole items follow the split ones: these warps reduce the split tiles they stored now, behind the MMAs
             // of the next items.  (With no whole items all warps do it at the end.)
-            if (!all_reduce && (pend[0] >= 0 || pend[1] >= 0) && (!more || it.sk < 0)) {
+            if (SPLIT == kTailSplit && (pend[0] >= 0 || pend[1] >= 0) && (!more || it.sk < 0)) {
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
                     if (pend[w] >= 0) reduce_split(p, epoch, pend[w], kstages, tt, 2 * kEpiWarps * 32, s_abort);
@@ -713,7 +724,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
-    if (all_reduce) {
+    if (SPLIT == kAllSplit) {
         // Every tile was split and nothing else is left to do: all 20 warps reduce.
         ptx::griddep_wait();
         const unsigned int epoch = *s_epoch;
@@ -744,8 +755,8 @@ int plan_pair(PairParams& p, const nvfp4_device_info& dev, bool dense, int* smem
     return 2 * pairs;
 }
 
-template <int MODE, bool FINE>
-cudaError_t launch(const PairParams& p, int grid, int smem, const CUtensorMap& tma, const CUtensorMap& tmw, const CUtensorMap& tms,
+template <int MODE, bool FINE, int SPLIT>
+cudaError_t launch_as(const PairParams& p, int grid, int smem, const CUtensorMap& tma, const CUtensorMap& tmw, const CUtensorMap& tms,
                    cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
@@ -761,7 +772,28 @@ cudaError_t launch(const PairParams& p, int grid, int smem, const CUtensorMap& t
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, prefill_pair_kernel<MODE, FINE>, tma, tmw, tms, p);
+    return cudaLaunchKernelEx(&cfg, prefill_pair_kernel<MODE, FINE, SPLIT>, tma, tmw, tms, p);
+}
+
+template <int MODE>
+cudaError_t launch(const PairParams& p, int grid, int smem, const CUtensorMap& tma, const CUtensorMap& tmw, const CUtensorMap& tms,
+                   cudaStream_t s) {
+    const int split = p.sk_tiles == 0 ? kWhole : (p.dp_items == 0 ? kAllSplit : kTailSplit);
+    if (MODE == kDense || p.T > kCoarseT)
+        return split == kWhole ? launch_as<MODE, true, kWhole>(p, grid, smem, tma, tmw, tms, s)
+               : split == kAllSplit ? launch_as<MODE, true, kAllSplit>(p, grid, smem, tma, tmw, tms, s)
+                                    : launch_as<MODE, true, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
+    return split == kWhole ? launch_as<MODE, MODE == kDense, kWhole>(p, grid, smem, tma, tmw, tms, s)
+           : split == kAllSplit ? launch_as<MODE, MODE == kDense, kAllSplit>(p, grid, smem, tma, tmw, tms, s)
+                                : launch_as<MODE, MODE == kDense, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
+}
+
+template <int MODE, bool FINE>
+cudaError_t configure() {
+    cudaError_t e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kWhole>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kAllSplit>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kTailSplit>, kSmemMax);
+    return e;
 }
 
 }  // namespace
@@ -784,11 +816,11 @@ size_t prefill_umma_scratch_bytes(int M, int /*N*/, int K) {
 }
 
 cudaError_t configure_prefill_umma(nvfp4_device_info& dev) {
-    cudaError_t e = configure_large_smem(prefill_pair_kernel<kExact, false>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kExact, true>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kRounded, false>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kRounded, true>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<kDense, true>, kSmemMax);
+    cudaError_t e = configure<kExact, false>();
+    if (e == cudaSuccess) e = configure<kExact, true>();
+    if (e == cudaSuccess) e = configure<kRounded, false>();
+    if (e == cudaSuccess) e = configure<kRounded, true>();
+    if (e == cudaSuccess) e = configure<kDense, true>();
     if (e != cudaSuccess) return e;
     // The split tiles need every pair resident at once: no more pairs than the device can place.
     cudaLaunchConfig_t cfg{};
@@ -803,7 +835,7 @@ cudaError_t configure_prefill_umma(nvfp4_device_info& dev) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, prefill_pair_kernel<kExact, true>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&clusters, prefill_pair_kernel<kExact, true, kAllSplit>, &cfg);
     if (e != cudaSuccess) return e;
     if (clusters < 1) return cudaErrorLaunchOutOfResources;
     dev.max_pairs = clusters;
@@ -850,9 +882,9 @@ cudaError_t launch_prefill_umma(const LinearArgs& a, nvfp4_device_info& dev, voi
         std::frexp(2688.0f * a.inv_gs, &ex);                 // 2688 / gs = f * 2^ex, f in [0.5, 1)
         p.wshift = std::ldexp(1.0f, 15 - ex);
         p.out_mul = std::ldexp(1.0f, ex - 15);
-        e = p.T > kCoarseT ? launch<kRounded, true>(p, grid, smem, tma, tmp, tms, s) : launch<kRounded, false>(p, grid, smem, tma, tmp, tms, s);
+        e = launch<kRounded>(p, grid, smem, tma, tmp, tms, s);
     } else {
-        e = p.T > kCoarseT ? launch<kExact, true>(p, grid, smem, tma, tmp, tms, s) : launch<kExact, false>(p, grid, smem, tma, tmp, tms, s);
+        e = launch<kExact>(p, grid, smem, tma, tmp, tms, s);
     }
     if (launches) *launches = 2;
     return e;
@@ -885,7 +917,7 @@ cudaError_t launch_dense_umma(const DenseArgs& a, nvfp4_device_info& dev, void* 
     p.status = static_cast<unsigned int*>(scratch);
     p.flags = reinterpret_cast<unsigned int*>(sk);
     p.partials = reinterpret_cast<float*>(sk + 4096);
-    const cudaError_t e = launch<kDense, true>(p, grid, smem, tma, tmw, tmw, s);
+    const cudaError_t e = launch<kDense>(p, grid, smem, tma, tmw, tmw, s);
     if (launches) *launches = 1;
     return e;
 }
