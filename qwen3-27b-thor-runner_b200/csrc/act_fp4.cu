@@ -38,7 +38,6 @@ using namespace fp4q;
 
 constexpr int kSliceBlocks = 64;        // 16-element blocks (1024 k) per CTA
 constexpr int kPreThreads = 4 * kSliceBlocks;
-constexpr int kMaxRowLoads = 4;         // 16-byte loads of the row per thread held in registers at once
 
 // Where the activations come from (the fusions of nvfp4_linear_ex that act on them):
 //   kPlain   A itself;
@@ -76,9 +75,13 @@ __device__ __forceinline__ uint32_t absmax_bf16x8(uint4 x) {
 // use, so the kernel pays one trip to L2.
 // Columns beyond tokens x terms are never written: whatever an earlier call left there only reaches
 // accumulator columns the GEMV's epilogue does not read (stale codes and scales are finite).
+//
+// Row loads a thread has in flight: 9 take 18432 columns in one trip (with 4 a row of 17408 took three), as many as leave the
+// CTA room beside a GEMV's.  SwiGLU and RMSNorm load a second vector with each.
 template <int TERMS, int MODE>
 __global__ void __launch_bounds__(kPreThreads)
 act_to_fp4_kernel(const ActParams p) {
+    constexpr int kMaxRowLoads = MODE == kPlain ? 9 : 4;
     __shared__ unsigned int s_max;
     __shared__ float s_part[kPreThreads / 32];
     const int m = blockIdx.y;
@@ -86,8 +89,8 @@ act_to_fp4_kernel(const ActParams p) {
     const int blocks = K / 16;
     if (threadIdx.x == 0) s_max = 0u;
     ptx::griddep_launch_dependents();      // the GEMV behind this kernel may set itself up and start streaming weights
-    ptx::griddep_wait();                   // A is the output of the kernel before this one
     __syncthreads();
+    ptx::griddep_wait();                   // A is the output of the kernel before this one
     const uint4* src = reinterpret_cast<const uint4*>(p.A + (size_t)m * p.a_stride);
     const uint4* src_up = MODE == kSwiglu ? reinterpret_cast<const uint4*>(p.up + (size_t)m * p.a_stride) : nullptr;
     const int b = blockIdx.x * kSliceBlocks + (threadIdx.x >> 2), part = threadIdx.x & 3;     // block, quarter of it

@@ -21,8 +21,8 @@
 //     accumulating FP32 in tensor memory; tcgen05.commit recycles the ring stage;
 //   * the activations are the B operand: a pre-pass (act_fp4.cu) expands every BF16 token into six
 //     (five for 3, 6 and 9 tokens) NVFP4 term rows whose sum reproduces it to 1e-5 (8e-5) of each block's largest element; the CTA's k
-//     range of the codes is loaded once by warp 2 and stays resident in shared memory, next to their
-//     block scales (copied in by warps 8-11 before their first accumulator arrives).  For one or two
+//     range of the codes is loaded once by warps 2 and 3 and stays resident in shared memory, next to their
+//     block scales (one or two bulk copies by warp 3).  For one or two
 //     tokens without SwiGLU or RMSNorm in front, where a CTA's k range is short (up to 8 chunks), there
 //     is no pre-pass at all: warps 4-11 expand the CTA's k range of the activations themselves,
 //     straight into the operand layout in shared memory (CTAs repeat each other's work, but a
@@ -33,6 +33,13 @@
 //     publish FP32 partials as {value, launch tag} pairs (8-byte single transactions, the tag
 //     from a counter in the scratch), the owner adds them in CTA order (deterministic).
 // Every wait is bounded and reports through the status word; tensor memory is always freed.
+//
+// What bounds it: HBM while it streams (6.2-6.6 TB/s), and ~5 us a call in which nothing streams that was not asked for before: the
+// kernel boundaries, the pre-pass and the trips to L2 between the activations' arrival and the first MMA, and between the last MMA
+// and the outputs.  So everything behind those is asked for early: block scales by bulk copy (a loop of loads and stores: five
+// trips), the row and its own slice in one go, the residual before the sums, token factors once.  Two decode layers (hidden 5120,
+// MLP 17408) with one token 118.4 -> 109.6 us, four 135.4 -> 121.7, sixteen (the streamed form) 174.8 -> 161.0; 34816 x 5120 alone at one
+// token 21.0 -> 20.2, 5120 x 17408 15.0 -> 14.1, 7168 x 5120 9.1 -> 8.4.
 //
 // Arithmetic: the weight side is exact (the tensor core multiplies e2m1 x ue4m3 exactly and
 // accumulates in FP32); the activation side carries the pre-pass's remainder.  Against the
@@ -94,6 +101,7 @@ struct Fp4Params {
 constexpr int kOwnTokens = 2;       // most tokens the kernel expands itself
 constexpr int kOwnThreads = 8 * 32; // warps 4-11
 constexpr int kOwnMaxChunks = 8;    // ... and most resident 256-k chunks x tokens it does so for
+constexpr int kOwnTasks = kOwnMaxChunks * 64 / kOwnThreads;
 
 template <int TERMS, bool OWN, bool DUAL = false>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -118,7 +126,7 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     volatile unsigned int* s_epoch = reinterpret_cast<volatile unsigned int*>(s_tmem + 2);
     unsigned int* s_amax = s_tmem + 3;                                      // [2] largest magnitude of a token (BF16 bits)
-    float* s_unscale = reinterpret_cast<float*>(s_tmem + 5);                // [2] 1 / c of a token
+    float* s_unscale = reinterpret_cast<float*>(s_tmem + 5);                // [kTokens] 1 / c of a token
 
     unsigned int* status = reinterpret_cast<unsigned int*>(p.scratch);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -133,8 +141,8 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             ptx::mbar_init(&empty_bar[s], 1);
             ptx::mbar_init(&sfa_bar[s], 4);
         }
-        ptx::mbar_init(&b_bar[0], 1);
-        ptx::mbar_init(&b_bar[1], OWN ? 1 : 4);
+        ptx::mbar_init(&b_bar[0], OWN ? 1 : 2);
+        ptx::mbar_init(&b_bar[1], 1);
         s_amax[0] = s_amax[1] = 0u;
         for (int i = 0; i < 2; ++i) { ptx::mbar_init(&tfull[i], 1); ptx::mbar_init(&tempty[i], 4); }
         *s_abort = 0;
@@ -153,6 +161,25 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
         using namespace fp4q;
         const int tq = tid - 4 * 32;
         ptx::griddep_wait();                                  // A is the output of the kernel before this one
+        // One task = a quarter (4 elements) of a 16-element block of one token in one resident chunk; a quad of
+        // lanes holds the block.  64 tasks per token and chunk, so whole warps are in or out of range together.  A thread's
+        // (kOwnTasks, kOwnMaxChunks has no more) are asked for with the row, before its largest magnitude is known.
+        const int total = p.M * p.slots * 64;
+        const int kc0 = p.act_all ? 0 : kc_begin;
+        uint2 x[kOwnTasks];
+#pragma unroll
+        for (int u = 0; u < kOwnTasks; ++u) {
+            const int id = tq + u * kOwnThreads;
+            x[u] = make_uint2(0u, 0u);
+            if (id < total) {
+                const int part = id & 3, bl = (id >> 2) & 15, rest = id >> 6;
+                const int m = rest / p.slots, j = rest - m * p.slots;
+                int kcj = kc0 + j;
+                if (kcj >= p.kchunks) kcj -= p.kchunks;
+                const int k = kcj * kKC + bl * 16 + part * 4;
+                if (k < p.k_valid) x[u] = __ldcg(reinterpret_cast<const uint2*>(p.A + (size_t)m * p.a_stride + k));
+            }
+        }
         const int chunks = p.k_valid / 8;
 #pragma unroll
         for (int m = 0; m < kOwnTokens; ++m) {
@@ -160,15 +187,15 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             const uint4* src = reinterpret_cast<const uint4*>(p.A + (size_t)m * p.a_stride);
             unsigned int amax = 0;
             for (int i0 = tq; i0 < chunks; i0 += kOwnThreads * 4) {
-                uint4 x[4];
+                uint4 y[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int i = i0 + j * kOwnThreads;
-                    x[j] = i < chunks ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+                    y[j] = i < chunks ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const uint32_t v[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
+                    const uint32_t v[4] = {y[j].x, y[j].y, y[j].z, y[j].w};
 #pragma unroll
                     for (int q = 0; q < 4; ++q) amax = max(amax, max(v[q] & 0x7FFFu, (v[q] >> 16) & 0x7FFFu));
                 }
@@ -184,52 +211,32 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             c[m] = __uint_as_float((uint32_t)se << 23);
             if (tq == m) s_unscale[m] = token_unscale(s_amax[m], se);
         }
-        // One task = a quarter (4 elements) of a 16-element block of one token in one resident chunk; a quad of
-        // lanes holds the block.  64 tasks per token and chunk, so whole warps are in or out of range together.
-        const int total = p.M * p.slots * 64;
-        const int kc0 = p.act_all ? 0 : kc_begin;
-        for (int id0 = tq; id0 < total; id0 += kOwnThreads * 4) {
-            uint2 x[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int id = id0 + u * kOwnThreads;
-                x[u] = make_uint2(0u, 0u);
-                if (id < total) {
-                    const int part = id & 3, bl = (id >> 2) & 15, rest = id >> 6;
-                    const int m = rest / p.slots, j = rest - m * p.slots;
-                    int kcj = kc0 + j;
-                    if (kcj >= p.kchunks) kcj -= p.kchunks;
-                    const int k = kcj * kKC + bl * 16 + part * 4;
-                    if (k < p.k_valid) x[u] = __ldcg(reinterpret_cast<const uint2*>(p.A + (size_t)m * p.a_stride + k));
-                }
+        for (int u = 0; u < kOwnTasks; ++u) {
+            const int id = tq + u * kOwnThreads;
+            if (id >= total) continue;                        // uniform across the warp
+            const int part = id & 3, bl = (id >> 2) & 15, rest = id >> 6;
+            const int m = rest / p.slots, j = rest - m * p.slots;
+            const float cm = m == 0 ? c[0] : c[1];
+            float r[4] = {__uint_as_float(x[u].x << 16) * cm, __uint_as_float(x[u].x & 0xFFFF0000u) * cm,
+                          __uint_as_float(x[u].y << 16) * cm, __uint_as_float(x[u].y & 0xFFFF0000u) * cm};
+            float bmax = fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3])));
+            bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
+            bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
+            const int p0 = first_term_exponent(bmax);
+            // Operand layout (K-major, 128-byte swizzle, as TMA would have written it): row = MMA column, a row
+            // holds the chunk's 256 codes in eight 16-byte pieces, piece i of row r at position i ^ (r % 8).
+            unsigned char* row0 = s_b + j * b_bytes;
+            unsigned char* sf0 = s_sfb + j * p.groups * 512 + (bl >> 2) * 4 + (bl & 3);
+#pragma unroll
+            for (int t = 0; t < TERMS; ++t) {
+                const int pw = term_exponent(p0, t);
+                const uint32_t w = take_term(r, pw);
+                const int col = m * TERMS + t;
+                *reinterpret_cast<uint16_t*>(row0 + col * 128 + (((bl >> 1) ^ (col & 7)) << 4) + (bl & 1) * 8 + part * 2) = (uint16_t)w;
+                if (part == 0) sf0[(col & 31) * 16] = (uint8_t)ue4m3_pow2(pw);
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int id = id0 + u * kOwnThreads;
-                if (id >= total) continue;                        // uniform across the warp
-                const int part = id & 3, bl = (id >> 2) & 15, rest = id >> 6;
-                const int m = rest / p.slots, j = rest - m * p.slots;
-                const float cm = m == 0 ? c[0] : c[1];
-                float r[4] = {__uint_as_float(x[u].x << 16) * cm, __uint_as_float(x[u].x & 0xFFFF0000u) * cm,
-                              __uint_as_float(x[u].y << 16) * cm, __uint_as_float(x[u].y & 0xFFFF0000u) * cm};
-                float bmax = fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3])));
-                bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
-                bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
-                const int p0 = first_term_exponent(bmax);
-                // Operand layout (K-major, 128-byte swizzle, as TMA would have written it): row = MMA column, a row
-                // holds the chunk's 256 codes in eight 16-byte pieces, piece i of row r at position i ^ (r % 8).
-                unsigned char* row0 = s_b + j * b_bytes;
-                unsigned char* sf0 = s_sfb + j * p.groups * 512 + (bl >> 2) * 4 + (bl & 3);
-#pragma unroll
-                for (int t = 0; t < TERMS; ++t) {
-                    const int pw = term_exponent(p0, t);
-                    const uint32_t w = take_term(r, pw);
-                    const int col = m * TERMS + t;
-                    *reinterpret_cast<uint16_t*>(row0 + col * 128 + (((bl >> 1) ^ (col & 7)) << 4) + (bl & 1) * 8 + part * 2) = (uint16_t)w;
-                    if (part == 0) sf0[(col & 31) * 16] = (uint8_t)ue4m3_pow2(pw);
-                }
             }
-        }
         ptx::fence_proxy_async_smem();                        // the tensor core reads the codes through the asynchronous proxy
         ptx::named_barrier_sync(2, kOwnThreads);
         if (tq == 0) {
@@ -276,16 +283,25 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
                 if (kc >= p.kchunks) { kc = 0; ++tile; }
             }
         }
-    } else if (warp == 2) {
+    } else if (warp == 2 || warp == 3) {
         // ------------------------------------------------------------------ resident activations (the pre-pass's output)
+        // Two warps, every other chunk each (a copy takes a warp ~50 clocks to issue); one of them first asks for the block scales,
+        // which lie as shared memory wants them: one bulk copy, two where the CTA's k range wraps.
         if (!OWN) {
-            ptx::prefetch_tensormap(&tm_act);
+            const int me = warp - 2, kc0 = p.act_all ? 0 : kc_begin;
+            if (me == 0) ptx::prefetch_tensormap(&tm_act);
             ptx::griddep_wait();
             const uint64_t pol = ptx::policy_evict_last();
             if (ptx::elect_one()) {
-                ptx::mbar_arrive_expect_tx(&b_bar[0], (uint32_t)(p.slots * b_bytes));
-                const int kc0 = p.act_all ? 0 : kc_begin;
-                for (int j = 0; j < p.slots; ++j) {
+                if (me == 1) {
+                    const uint32_t chunk = (uint32_t)p.groups * 512;
+                    const int run = min(p.slots, p.kchunks - kc0);
+                    ptx::mbar_arrive_expect_tx(&b_bar[1], (uint32_t)p.slots * chunk);
+                    ptx::bulk_load(s_sfb, p.sfb + (size_t)kc0 * chunk, (uint32_t)run * chunk, &b_bar[1]);
+                    if (run < p.slots) ptx::bulk_load(s_sfb + (size_t)run * chunk, p.sfb, (uint32_t)(p.slots - run) * chunk, &b_bar[1]);
+                }
+                ptx::mbar_arrive_expect_tx(&b_bar[0], (uint32_t)((p.slots + 1 - me) / 2 * b_bytes));
+                for (int j = me; j < p.slots; j += 2) {
                     int kc = kc0 + j;
                     if (kc >= p.kchunks) kc -= p.kchunks;
                     ptx::tma_load_2d(s_b + j * b_bytes, &tm_act, &b_bar[0], kc * (kKC / 2), 0, pol);
@@ -391,26 +407,10 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
         const int ew = warp - 8;                              // tensor-memory lanes 32 ew .. +31 (= warp id % 4)
         const int te = ew * 32 + lane;
         ptx::griddep_wait();                                  // C, the residual and the scratch belong to earlier kernels until now
-        // this launch's tag for the split-tile pairs: one atomic per CTA on one address, about a microsecond
-        // under contention, so it is left in flight while the scales are copied
-        unsigned int epoch_taken = 0;
-        if (te == 0) epoch_taken = ptx::take_launch_epoch(p.scratch);
+        // this launch's tag for the split-tile pairs: one atomic per CTA on one address, about a microsecond under contention
+        if (te == 0) *s_epoch = ptx::take_launch_epoch(p.scratch);
+        if (!OWN && te >= 32 && te - 32 < p.M) s_unscale[te - 32] = p.unscale[te - 32];
         unsigned char* pairs = p.pairs;
-        if (!OWN) {
-            // The activations' block scales of the CTA's k range into shared memory (512 bytes per resident chunk
-            // and column group, as the pre-pass left them); the warps of the scale path wait for this.
-            const int kc0 = p.act_all ? 0 : kc_begin;
-            const int words = p.slots * p.groups * 32;              // 16-byte words
-            for (int i = te; i < words; i += kEpiThreads) {
-                const int j = i / (p.groups * 32), rest = i - j * (p.groups * 32);
-                int kcj = kc0 + j;
-                if (kcj >= p.kchunks) kcj -= p.kchunks;
-                reinterpret_cast<uint4*>(s_sfb)[i] = __ldcg(reinterpret_cast<const uint4*>(p.sfb + (size_t)kcj * p.groups * 512) + rest);
-            }
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&b_bar[1]);
-        }
-        if (te == 0) *s_epoch = epoch_taken;
         ptx::named_barrier_sync(1, kEpiThreads);
         const unsigned int epoch = *s_epoch;
         int acc = 0;
@@ -425,21 +425,24 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             int last = cta;                                   // contributors are CTAs cta+1 .. last
             if (owner && !complete)
                 while (last + 1 < G && (long long)(last + 1) * p.units / G < tile_end) ++last;
+            constexpr int KT = OWN ? kOwnTokens : kTokens;
+            unsigned short res[KT];
+            if (!DUAL && owner && p.out.residual) fp4_ask_residual(res, p.out, tile, te);      // a dual call has none
             ptx::mbar_wait(&tfull[acc], (pt >> acc) & 1u, s_abort, status, 0xA50u + (unsigned)acc);
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * kAccStride);
-            float v[kTokens];
+            float v[KT];
 #pragma unroll
-            for (int m = 0; m < kTokens; ++m) v[m] = 0.0f;
+            for (int m = 0; m < KT; ++m) v[m] = 0.0f;
 #pragma unroll
-            for (int c0 = 0; c0 < 48; c0 += 16) {
+            for (int c0 = 0; c0 < (KT * TERMS + 15) / 16 * 16; c0 += 16) {
                 if (c0 < p.NCp) {
                     uint32_t r[16];
                     tmem_ld16(t_addr + c0, r);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const int c = c0 + i;                 // column c = token * TERMS + term (compile-time after unrolling)
-                        if (c / TERMS < kTokens) v[c / TERMS] += __uint_as_float(r[i]);
+                        if (c / TERMS < KT) v[c / TERMS] += __uint_as_float(r[i]);
                     }
                 }
             }
@@ -452,17 +455,17 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             kc = kc_first + (seg_end - (tile_end - p.kchunks + kc_first));
 
 #pragma unroll
-            for (int m = 0; m < kTokens; ++m)
-                if (m < p.M) v[m] *= OWN ? s_unscale[m < kOwnTokens ? m : 0] : p.unscale[m];
+            for (int m = 0; m < KT; ++m)
+                if (m < p.M) v[m] *= s_unscale[m];
             if (!owner) {
                 unsigned char* slot = pairs + (size_t)cta * (kPairTokens * kRT) * 8;
 #pragma unroll
-                for (int m = 0; m < kTokens; ++m)
+                for (int m = 0; m < KT; ++m)
                     if (m < p.M) ptx::st_volatile_v2(slot + (m * kRT + te) * 8, __float_as_uint(v[m]), epoch);
             } else {
                 fp4_gather_pairs(v, pairs, (size_t)(kPairTokens * kRT) * 8, cta + 1, last, p.M, te, epoch, s_abort, status, 0xA60u);
-                if (!DUAL || tile < p.tiles0) fp4_store_rows(v, p.out, tile, te);
-                else fp4_store_rows(v, p.out2, tile - p.tiles0, te);
+                if (!DUAL || tile < p.tiles0) fp4_store_rows(v, res, p.out, tile, te);
+                else fp4_store_rows(v, res, p.out2, tile - p.tiles0, te);
             }
             if (kc >= p.kchunks) { kc = 0; ++tile; }
         }
@@ -480,7 +483,7 @@ struct Fp4Plan {
     int grid, smem;
 };
 
-constexpr int kFixedSmem = 1024 + (3 * kMaxStages + 6) * 8 + 64;
+constexpr int kFixedSmem = 1024 + (3 * kMaxStages + 6) * 8 + 64;      // alignment, barriers, words (5 + kTokens)
 
 bool plan_fp4(const LinearArgs& a, const nvfp4_device_info& dev, Fp4Plan* out) {
     Fp4Params& p = out->p;

@@ -110,6 +110,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(tempty + 2);
     volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
     volatile unsigned int* s_epoch = reinterpret_cast<volatile unsigned int*>(s_tmem + 2);
+    float* s_unscale = reinterpret_cast<float*>(s_tmem + 3);        // [kMaxTokens] 1 / c of a token
 
     unsigned int* status = reinterpret_cast<unsigned int*>(p.scratch);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -305,6 +306,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
         const int te = ew * 32 + lane;
         ptx::griddep_wait();                                  // C, the residual and the scratch belong to earlier kernels until now
         if (te == 0) *s_epoch = ptx::take_launch_epoch(p.scratch);      // this launch's tag for the split-tile pairs
+        if (te >= 32 && te - 32 < p.M) s_unscale[te - 32] = p.unscale[te - 32];
         unsigned char* pairs = p.pairs;
         ptx::named_barrier_sync(1, kEpiThreads);
         const unsigned int epoch = *s_epoch;
@@ -320,6 +322,8 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
             int last = cta;                                   // contributors are CTAs cta+1 .. last
             if (owner && !complete)
                 while (last + 1 < G && (long long)(last + 1) * p.units / G < tile_end) ++last;
+            unsigned short res[fp4::kMaxTokens];
+            if (owner && p.out.residual) fp4_ask_residual(res, p.out, tile, te);
             ptx::mbar_wait(&tfull[acc], (pt >> acc) & 1u, s_abort, status, 0xB50u + (unsigned)acc);
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * p.acc_stride);
@@ -348,7 +352,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
 
 #pragma unroll
             for (int m = 0; m < fp4::kMaxTokens; ++m)
-                if (m < p.M) v[m] *= p.unscale[m];
+                if (m < p.M) v[m] *= s_unscale[m];
             if (!owner) {
                 unsigned char* slot = pairs + (size_t)cta * (kPairTokens * kRT) * 8;
 #pragma unroll
@@ -356,7 +360,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
                     if (m < p.M) ptx::st_volatile_v2(slot + (m * kRT + te) * 8, __float_as_uint(v[m]), epoch);
             } else {
                 fp4_gather_pairs(v, pairs, (size_t)(kPairTokens * kRT) * 8, cta + 1, last, p.M, te, epoch, s_abort, status, 0xB60u);
-                fp4_store_rows(v, p.out, tile, te);
+                fp4_store_rows(v, res, p.out, tile, te);
             }
             if (kc >= p.kchunks) { kc = 0; ++tile; }
         }
@@ -374,7 +378,7 @@ struct Fp4Plan {
     int grid, smem;
 };
 
-constexpr int kFixedSmem = 1024 + (4 * kMaxStages + 4) * 8 + 64;
+constexpr int kFixedSmem = 1024 + (4 * kMaxStages + 4) * 8 + 96;      // alignment, barriers, words (3 + kMaxTokens)
 
 bool plan_fp4(const LinearArgs& a, const nvfp4_device_info& dev, Fp4Plan* out) {
     Fp4Params& p = out->p;
