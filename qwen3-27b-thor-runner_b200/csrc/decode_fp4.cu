@@ -30,7 +30,7 @@
 //   * warps 8-11 read the accumulator (thread = weight row), add the term columns of each token,
 //     undo the token scale, apply 1/global_scale and the residual in FP32 and round once.  A row
 //     tile split over several CTAs is finished by the CTA holding its first half-unit: the others
-//     publish FP32 partials as {value, launch tag} pairs (8-byte single transactions, the tag
+//     publish FP32 partials, three and the launch's tag in sixteen bytes (single accesses, the tag
 //     from a counter in the scratch), the owner adds them in CTA order (deterministic).
 // Every wait is bounded and reports through the status word; tensor memory is always freed.
 //
@@ -38,7 +38,7 @@
 // kernel boundaries, the pre-pass and the trips to L2 between the activations' arrival and the first MMA, and between the last MMA
 // and the outputs.  So everything behind those is asked for early: block scales by bulk copy (a loop of loads and stores: five
 // trips), the row and its own slice in one go, the residual before the sums, token factors once.  Two decode layers (hidden 5120,
-// MLP 17408) with one token 118.4 -> 109.6 us, four 135.4 -> 121.7, sixteen (the streamed form) 174.8 -> 161.0; 34816 x 5120 alone at one
+// MLP 17408) with one token 118.4 -> 107.3 us, four 135.4 -> 118.3, sixteen (the streamed form) 174.8 -> 140.4; 34816 x 5120 alone at one
 // token 21.0 -> 20.2, 5120 x 17408 15.0 -> 14.1, 7168 x 5120 9.1 -> 8.4.
 //
 // Arithmetic: the weight side is exact (the tensor core multiplies e2m1 x ue4m3 exactly and
@@ -76,8 +76,8 @@ constexpr int kSfCol = 2 * kAccStride;             // per half-unit of the ring 
 constexpr int kMaxRingHalfUnits = (512 - kSfCol) / 32;   // 12
 constexpr int kTokens = 9;                         // most tokens of this kernel: 9 x 5 = 45 of its 48 MMA columns
 constexpr int kMaxGrid = 160;                      // CTAs whose pair slots fit the kernel's share of the scratch
-constexpr int kPairTokens = kTokens;               // token rows of a CTA's pair slot (9 KB per CTA)
-static_assert((size_t)kMaxGrid * kPairTokens * kRT * 8 <= fp4::kPairBytes, "pair slots");
+constexpr size_t kSlotBytes = (size_t)quads_of(kTokens) * kRT * 16;      // of a CTA's partial sums: 6 KB
+static_assert(kMaxGrid * kSlotBytes <= fp4::kPairBytes, "slots");
 
 struct Fp4Params {
     Fp4Out out;                     // residual, C, 1 / global_scale, M, N and the output options
@@ -89,7 +89,7 @@ struct Fp4Params {
     int k_valid;
     const unsigned char* sfb;       // the pre-pass's block scales: [K/256][column groups of 32][32 lanes][16 bytes]
     unsigned char* scratch;         // status word at 0, launch counter at 64
-    unsigned char* pairs;           // [CTA][kPairTokens][128 rows] x {FP32 value, tag}
+    unsigned char* pairs;           // the CTAs' slots for partial sums (fp4_store.cuh)
     int M, N, K;
     int NCp, groups;                // MMA columns (tokens x terms padded to 16), groups of 32 of them
     int units, kchunks;
@@ -458,12 +458,9 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             for (int m = 0; m < KT; ++m)
                 if (m < p.M) v[m] *= s_unscale[m];
             if (!owner) {
-                unsigned char* slot = pairs + (size_t)cta * (kPairTokens * kRT) * 8;
-#pragma unroll
-                for (int m = 0; m < KT; ++m)
-                    if (m < p.M) ptx::st_volatile_v2(slot + (m * kRT + te) * 8, __float_as_uint(v[m]), epoch);
+                fp4_publish(v, pairs + (size_t)cta * kSlotBytes, p.M, te, epoch);
             } else {
-                fp4_gather_pairs(v, pairs, (size_t)(kPairTokens * kRT) * 8, cta + 1, last, p.M, te, epoch, s_abort, status, 0xA60u);
+                fp4_gather(v, pairs, kSlotBytes, cta + 1, last, p.M, te, epoch, s_abort, status, 0xA60u);
                 if (!DUAL || tile < p.tiles0) fp4_store_rows(v, res, p.out, tile, te);
                 else fp4_store_rows(v, res, p.out2, tile - p.tiles0, te);
             }

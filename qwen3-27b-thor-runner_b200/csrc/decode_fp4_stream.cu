@@ -31,7 +31,7 @@
 //   * warps 8-11 read the accumulator (thread = weight row), add the term columns of each token,
 //     undo the token scale, apply 1/global_scale and the residual in FP32 and round once.  A row
 //     tile split over several CTAs is finished by the CTA holding its first half-unit: the others
-//     publish FP32 partials as {value, launch tag} pairs (8-byte single transactions, the tag
+//     publish FP32 partials, three and the launch's tag in sixteen bytes (single accesses, the tag
 //     from a counter in the scratch), the owner adds them in CTA order (deterministic).
 // Every wait is bounded and reports through the status word; tensor memory is always freed.
 //
@@ -68,14 +68,14 @@ constexpr int kSmemBudget = 225 * 1024;
 // of the ring 32 columns: 16 of the weights' scales, 16 of the activations' (4 per MMA: up to 128 MMA columns).
 constexpr int kMaxCols = fp4::kMaxCols;            // MMA columns (tokens x terms, padded to 16)
 constexpr int kMaxGrid = 160;                      // CTAs whose pair slots fit the kernel's 2.5 MB of scratch
-constexpr int kPairTokens = fp4::kMaxTokens;       // token rows of a CTA's pair slot (16 KB per CTA)
-static_assert((size_t)kMaxGrid * kPairTokens * kRT * 8 <= fp4::kPairBytes, "pair slots");
+constexpr size_t kSlotBytes = (size_t)quads_of(fp4::kMaxTokens) * kRT * 16;      // of a CTA's partial sums: 12 KB
+static_assert(kMaxGrid * kSlotBytes <= fp4::kPairBytes, "slots");
 
 struct Fp4Params {
     Fp4Out out;                     // residual, C, 1 / global_scale, M, N and the output options
     const float* unscale;           // per token: 1 / c of the pre-pass
     unsigned char* scratch;         // status word at 0, launch counter at 64
-    unsigned char* pairs;           // [CTA][kPairTokens][128 rows] x {FP32 value, tag}
+    unsigned char* pairs;           // the CTAs' slots for partial sums (fp4_store.cuh)
     int M, N, K;
     int NCp, groups;                // MMA columns (tokens x terms padded to 16), groups of 32 of them
     int acc_stride;                 // tensor-memory columns per accumulator
@@ -354,12 +354,9 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
             for (int m = 0; m < fp4::kMaxTokens; ++m)
                 if (m < p.M) v[m] *= s_unscale[m];
             if (!owner) {
-                unsigned char* slot = pairs + (size_t)cta * (kPairTokens * kRT) * 8;
-#pragma unroll
-                for (int m = 0; m < fp4::kMaxTokens; ++m)
-                    if (m < p.M) ptx::st_volatile_v2(slot + (m * kRT + te) * 8, __float_as_uint(v[m]), epoch);
+                fp4_publish(v, pairs + (size_t)cta * kSlotBytes, p.M, te, epoch);
             } else {
-                fp4_gather_pairs(v, pairs, (size_t)(kPairTokens * kRT) * 8, cta + 1, last, p.M, te, epoch, s_abort, status, 0xB60u);
+                fp4_gather(v, pairs, kSlotBytes, cta + 1, last, p.M, te, epoch, s_abort, status, 0xB60u);
                 fp4_store_rows(v, res, p.out, tile, te);
             }
             if (kc >= p.kchunks) { kc = 0; ++tile; }

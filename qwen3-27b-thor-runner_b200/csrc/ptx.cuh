@@ -263,6 +263,20 @@ __device__ __forceinline__ uint2 ld_volatile_v2(const void* p) {
     return v;
 }
 
+// Sixteen bytes as one access (relaxed, GPU scope): the words arrive together.
+__device__ __forceinline__ void st_relaxed_b128(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile(
+        "{\n\t.reg .b128 q;\n\t.reg .b64 lo, hi;\n\tmov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 q, {lo, hi};\n\t"
+        "st.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint4 ld_relaxed_b128(const void* p) {
+    uint4 v;
+    asm volatile(
+        "{\n\t.reg .b128 q;\n\t.reg .b64 lo, hi;\n\tld.relaxed.gpu.global.b128 q, [%4];\n\tmov.b128 {lo, hi}, q;\n\t"
+        "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -39,3 +39,27 @@ def test_in_place_residual(handle, M, N, K):
     got = util.to_host_u16(C)
     for m in range(M):
         assert ob.rel_frobenius(got[m:m + 1], want[m:m + 1]) <= TOL, m
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 7, 9, 10, 13, 16])
+def test_a_launch_takes_its_own_partial_sums_only(handle, M):
+    """Launches with other activations follow each other on the same slots; every tile is split over several CTAs.  An old value beside
+    a new tag would show: what a launch gives is compared bit by bit with what the same inputs gave when nothing else ran."""
+    import torch
+    N, K = 4352, 5120
+    p, s = (util.to_dev(a) for a in util.make_weight(N, K, seed=7))
+    sets = []
+    for i in range(3):
+        A = util.to_dev(util.make_bf16((M, K), seed=10 * M + i))
+        C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        handle.linear(A, M, p, s, 1.0, N, K, C)
+        handle.linear(A, M, p, s, 1.0, N, K, C)      # the slots hold this very launch's values: right whatever is torn
+        torch.cuda.synchronize()
+        sets.append((A, C.clone()))
+    wrong = torch.zeros(1, dtype=torch.int64, device="cuda")
+    for it in range(200):
+        A, want = sets[it % 3]
+        C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        handle.linear(A, M, p, s, 1.0, N, K, C)
+        wrong += (C != want).sum()
+    assert int(wrong) == 0 and handle.device_status() == 0
