@@ -133,13 +133,13 @@ __device__ __forceinline__ void reduce_split_rows(const SkinnyParams& p, unsigne
     const float4* head = parts + ((size_t)first * 2 + 1) * (kSlotFloats / 4);
     for (int e = e0 + t; e < e1; e += nthreads) {
         float4 s = __ldcg(head + e);
-        for (int c = first + 1; c <= last; c += 4) {
-            float4 x[4];
+        for (int c = first + 1; c <= last; c += 8) {
+            float4 x[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)          // four loads in flight; absent participants add zero
+            for (int i = 0; i < 8; ++i)          // eight loads in flight (four: 33 x 1048 x 4864, 17 parts a tile, 20.1 instead of 16.3 us)
                 x[i] = c + i <= last ? __ldcg(parts + (size_t)(c + i) * 2 * (kSlotFloats / 4) + e) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { s.x += x[i].x; s.y += x[i].y; s.z += x[i].z; s.w += x[i].w; }
+            for (int i = 0; i < 8; ++i) { s.x += x[i].x; s.y += x[i].y; s.z += x[i].z; s.w += x[i].w; }
         }
         const int m = e / (TR / 4), n = tile * TR + (e % (TR / 4)) * 4;
         const float k = s_factor[m];
