@@ -369,6 +369,7 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             while (hu < seg_end) {
                 const int cnt = (seg_end - hu) >= hps ? hps : 1;
                 ptx::mbar_wait(&full_bar[stage], ph, s_abort, status, 0xA40u + (unsigned)stage);
+                __syncwarp();                                  // the stores to tensor memory want one warp
                 for (int h = 0; h < cnt; ++h) {
                     const int slot = p.act_all ? kc + h : (hu - u_begin) + h;
                     const unsigned char* raw = s_raw + (stage * hps + h) * kScaleBytes + lane * 16;
@@ -429,6 +430,7 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
             unsigned short res[KT];
             if (!DUAL && owner && p.out.residual) fp4_ask_residual(res, p.out, tile, te);      // a dual call has none
             ptx::mbar_wait(&tfull[acc], (pt >> acc) & 1u, s_abort, status, 0xA50u + (unsigned)acc);
+            __syncwarp();
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * kAccStride);
             float v[KT];

@@ -265,6 +265,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
                 const int cnt = (seg_end - hu) >= hps ? hps : 1;
                 ptx::mbar_wait(&full_bar[stage], ph, s_abort, status, 0xB40u + (unsigned)stage);
                 ptx::mbar_wait(&fullb_bar[stage], ph, s_abort, status, 0xB40u + (unsigned)stage);
+                __syncwarp();                                  // the stores to tensor memory want one warp
                 for (int h = 0; h < cnt; ++h) {
                     const int bslot = stage * hps + h;
                     const unsigned char* raw = s_raw + (stage * hps + h) * kScaleBytes + lane * 16;
@@ -325,6 +326,7 @@ decode_fp4_stream_kernel(const __grid_constant__ CUtensorMap tm_packed, const __
             unsigned short res[fp4::kMaxTokens];
             if (owner && p.out.residual) fp4_ask_residual(res, p.out, tile, te);
             ptx::mbar_wait(&tfull[acc], (pt >> acc) & 1u, s_abort, status, 0xB50u + (unsigned)acc);
+            __syncwarp();
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * p.acc_stride);
             float v[fp4::kMaxTokens];

@@ -25,6 +25,8 @@ __device__ __forceinline__ void umma_fp4(uint32_t tmem_d, uint64_t adesc, uint64
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
 }
+// For whole, converged warps (.sync.aligned): lanes that come from a wait, or from rows beyond the weight, one by one are brought together by
+// a __syncwarp() or a vote first.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "

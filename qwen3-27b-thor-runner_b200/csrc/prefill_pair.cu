@@ -174,6 +174,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// For whole, converged warps (.sync.aligned): lanes that come from a wait, or from rows beyond the weight, one by one are brought together by
+// a __syncwarp() or a vote first.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -551,7 +553,10 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                             for (int i = 0; i < 4; ++i) o[c >> 2][(c & 3) * 4 + i] = ptx::mul_f16x2(e[i], S);
                         }
                     }
+                    // The stores want one warp: lanes that saw the unit free and lanes that waited for it meet here.  (A vote in front of the
+                    // wait instead: 149 tokens of an MLP 5120 x 17408 101.8 us, so 100.5; in the few-token kernel the vote is ahead.)
                     if (!ready) ptx::mbar_wait(&aempty[su], pu ^ 1u, s_abort, p.status, 0x460u + su);
+                    __syncwarp();
                     if (opens) tc_fence_after();
                     const uint32_t a_addr = a_base + (uint32_t)su * kRingCols + (opens ? 0u : (uint32_t)(kUnitCols / 2));
                     tmem_st16(a_addr, o[0]);
@@ -628,6 +633,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 float* slot = p.partials + ((size_t)blockIdx.x * 2 + which) * kSlotFloats + te;
                 for (int c0 = begin; c0 < end; c0 += 16) {
                     uint32_t v[16];
+                    __syncwarp();                  // lanes beyond the weight left the last chunk early
                     tmem_ld16(t_addr + c0, v);
                     if (!two) {
                         uint32_t w[16];

@@ -107,6 +107,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// For whole, converged warps (.sync.aligned): lanes that come from a wait, or from rows beyond the weight, one by one are brought together by
+// a __syncwarp() or a vote first.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -326,7 +328,10 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
                         for (int j = 0; j < 4; ++j) r[c][4 * i + j] = ptx::mul_f16x2(e[j], S);
                     }
                 }
-                if (!ready) ptx::mbar_wait(&aempty[au], pa ^ 1u, s_abort, p.status, 0x560u + au);
+                if (!__all_sync(0xffffffffu, ready)) {     // one decision for the warp: the stores want it whole
+                    ptx::mbar_wait(&aempty[au], pa ^ 1u, s_abort, p.status, 0x560u + au);
+                    __syncwarp();
+                }
                 tc_fence_after();
                 const uint32_t a_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(p.a_col0 + au * kAUnitCols);
 #pragma unroll
@@ -380,6 +385,7 @@ skinny_umma_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_cons
             float* slot = p.partials + ((size_t)blockIdx.x * 2 + which) * kSlotFloats;
             for (int c0 = 0; c0 < p.NT; c0 += 16) {
                 uint32_t r[16], r2[16];
+                __syncwarp();                              // the lanes come from the wait, or left the last chunk early
                 tmem_ld16(t_addr + c0, r);
                 tmem_ld16(t_addr + p.acc_cols + c0, r2);
                 float f[16];
