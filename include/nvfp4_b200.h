@@ -291,7 +291,7 @@ int nvfp4_swiglu(nvfp4_handle* h, const void* gate_bf16, const void* up_bf16_or_
  * (TMA ring + mma.sync BF16, FP32 accumulation, residual added before the only rounding); more tokens
  * (K % 256 == 0, N % 8 == 0) run the tcgen05 GEMM of the quantised path with the weight blocks loaded
  * straight into the operand buffers; other shapes fall back to a plain CUDA-core GEMM: correct,
- * not fast.  residual may alias C. */
+ * not fast.  residual may alias C.  Order: W follows the stream like A, residual and C, whatever M is. */
 int nvfp4_linear_bf16(nvfp4_handle* h, const void* A_bf16, int M, const void* W_bf16, int N, int K,
                       const void* residual_bf16_or_null, void* C_bf16, nvfp4_stream_t stream);
 

@@ -91,6 +91,10 @@ dense_gemv_kernel(const __grid_constant__ CUtensorMap tm_w, const DenseParams p)
         ptx::named_barrier_arrive(2, kDenseThreads);
         if (lane == 0) {
             ptx::prefetch_tensormap(&tm_w);
+            // W follows the stream.  A kernel before this one may trigger its dependents at its first instruction (RMSNorm and SwiGLU do),
+            // so without this wait the loads could run beside whatever writes W, two kernels back or more.  Calls back to back pay for
+            // it: 2048 x 2048 at one token 6.7 -> 7.6 us, 16384 x 5120 26.0 -> 27.5, a head of 248320 x 5120 none of 355.
+            ptx::griddep_wait();
             const uint64_t pol = ptx::policy_evict_first();
             int stage = 0;
             uint32_t ph = 0;

@@ -140,3 +140,38 @@ def test_dense_gemv_side_by_side_with_reference_kernels(handle):
         ref_bits = util.to_host_u16(o_ref)
         assert np.array_equal(ref_bits, ob.dense_gemv_ref(A, W, residual=R)), (N, K)      # the restatement, once more
         assert ob.rel_frobenius(run(handle, A, W, residual=R), ref_bits) <= TOL, (N, K)
+
+
+@pytest.mark.parametrize("between", ["nothing", "rmsnorm", "swiglu"])
+@pytest.mark.parametrize("M", [1, 16])
+def test_bf16_weights_follow_the_stream(handle, M, between):
+    """W is the output of a library call that leaves most SMs idle and lets its successor start early, right before the GEMV or with a
+    norm or a SwiGLU (which trigger at once) in between.  The bits are those of the same calls with a synchronisation after each."""
+    import torch
+    N, K, K1 = 2048, 256, 2560                           # the first call: N tokens, K weight rows
+    A1 = util.to_dev(util.make_bf16((N, K1), seed=M))
+    w1 = [tuple(util.to_dev(a) for a in util.make_weight(K, K1, seed=M + 2 + i, sigma=0.14)) for i in range(3)]
+    x, gate_up, weight = (util.to_dev(util.make_bf16(shape, seed=i)) for i, shape in enumerate([(M, K), (M, 2 * K), (K,)]))
+    W, act = torch.empty((N, K), dtype=torch.int16, device="cuda"), torch.empty((M, K), dtype=torch.int16, device="cuda")
+
+    def step(i, out, wait):
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        handle.linear(A1, N, w1[i][0], w1[i][1], 1.0, K, K1, W)
+        sync()
+        if between == "rmsnorm":
+            handle.rmsnorm(x, weight, 1e-6, M, K, act)
+        elif between == "swiglu":
+            handle.swiglu(gate_up, None, M, K, act)
+        sync()
+        handle.linear_bf16(x if between == "nothing" else act, M, W, N, K, out)
+        sync()
+
+    want = [torch.empty((M, N), dtype=torch.int16, device="cuda") for _ in range(3)]
+    for i in range(3):
+        step(i, want[i], True)
+    assert not torch.equal(want[0], want[1])
+    for r in range(30):
+        got = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        step(r % 3, got, False)
+        assert torch.equal(got, want[r % 3]), r
+    assert handle.device_status() == 0

@@ -29,3 +29,12 @@ def test_warps_are_whole_at_tensor_memory_accesses(name):
         # a loop whose lanes may leave a turn early meets a __syncwarp() before the next turn's load
         turn = re.search(r"for \(int c0 = (?:begin|0); c0 < (?:end|p\.NT); c0 \+= 16\) \{[^}]*$", before)
         assert not turn or "__syncwarp();" in turn.group(0)
+
+
+def test_bf16_weight_loader_waits_for_the_stream():
+    """The header lets W come from the kernel right before, and the kernels of this library let their successors start early: the
+    loading warp waits for them before its first load."""
+    src = source("dense_gemv.cu")
+    loader = src[src.index("if (warp == 2 * kGroupWarps)"):]
+    loader = loader[:loader.index("return;")]
+    assert "griddep_wait()" in loader and loader.index("griddep_wait()") < loader.index("tma_load_2d(")
