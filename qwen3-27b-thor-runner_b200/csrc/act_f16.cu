@@ -16,14 +16,14 @@ constexpr int kHeld = 4;       // 16-byte vectors a thread keeps between the two
 // One CTA per token.  Latency-bound: the row is read once (all loads of a thread in flight together) and stays in registers
 // between the row maximum and the conversion; rows beyond kHeld x blockDim vectors are read again for the rest.
 __global__ void __launch_bounds__(1024)
-act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out, float* __restrict__ unscale, int K) {
+act_to_f16_kernel(const __nv_bfloat16* A, __half* out, float* unscale, int K) {
     __shared__ unsigned int s_max;
     const int m = blockIdx.x, nv = K / 8;
     const uint4* src = reinterpret_cast<const uint4*>(A + (size_t)m * K);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)m * K);
     if (threadIdx.x == 0) s_max = 0u;
     ptx::griddep_launch_dependents();      // the GEMM behind this kernel may set itself up (few tokens: start streaming weights)
-    ptx::griddep_wait();                   // A is the output of the kernel before this one
+    ptx::griddep_wait();                   // A is the output of the kernel before this one: plain loads, see ptx::griddep_wait
     __syncthreads();
     unsigned int amax = 0;
     auto largest = [&](const uint4& x) {
@@ -35,11 +35,11 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
 #pragma unroll
     for (int j = 0; j < kHeld; ++j) {
         const int i = threadIdx.x + j * blockDim.x;
-        held[j] = i < nv ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+        held[j] = i < nv ? src[i] : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int j = 0; j < kHeld; ++j) largest(held[j]);
-    for (int i = threadIdx.x + kHeld * blockDim.x; i < nv; i += blockDim.x) largest(__ldg(src + i));
+    for (int i = threadIdx.x + kHeld * blockDim.x; i < nv; i += blockDim.x) largest(src[i]);
     amax = __reduce_max_sync(0xffffffffu, amax);
     if ((threadIdx.x & 31) == 0 && amax) atomicMax(&s_max, amax);
     __syncthreads();
@@ -60,7 +60,7 @@ act_to_f16_kernel(const __nv_bfloat16* __restrict__ A, __half* __restrict__ out,
         const int i = threadIdx.x + j * blockDim.x;
         if (i < nv) convert(held[j], i);
     }
-    for (int i = threadIdx.x + kHeld * blockDim.x; i < nv; i += blockDim.x) convert(__ldg(src + i), i);
+    for (int i = threadIdx.x + kHeld * blockDim.x; i < nv; i += blockDim.x) convert(src[i], i);
 }
 
 }  // namespace

@@ -98,9 +98,9 @@ act_to_fp4_kernel(const ActParams p) {
     const bool own_valid = live && b * 16 + part * 4 < p.k_valid;      // k_valid is a multiple of 8: a quarter is valid or not
     uint2 own = make_uint2(0u, 0u), own2 = make_uint2(0u, 0u);
     if (own_valid) {
-        own = __ldg(reinterpret_cast<const uint2*>(src + 2 * b) + part);
-        if (MODE == kSwiglu) own2 = __ldg(reinterpret_cast<const uint2*>(src_up + 2 * b) + part);
-        if (MODE == kNorm) own2 = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint4*>(p.norm_w) + 2 * b) + part);
+        own = reinterpret_cast<const uint2*>(src + 2 * b)[part];
+        if (MODE == kSwiglu) own2 = reinterpret_cast<const uint2*>(src_up + 2 * b)[part];
+        if (MODE == kNorm) own2 = reinterpret_cast<const uint2*>(reinterpret_cast<const uint4*>(p.norm_w) + 2 * b)[part];
     }
     unsigned int amax = 0;
     float ss = 0.0f, mt = 0.0f;
@@ -112,9 +112,9 @@ act_to_fp4_kernel(const ActParams p) {
             const int i = i0 + j * kPreThreads;
             x[j] = y[j] = make_uint4(0u, 0u, 0u, 0u);
             if (i < chunks) {
-                x[j] = __ldg(src + i);
-                if (MODE == kSwiglu) y[j] = __ldg(src_up + i);
-                if (MODE == kNorm) y[j] = __ldg(reinterpret_cast<const uint4*>(p.norm_w) + i);
+                x[j] = src[i];
+                if (MODE == kSwiglu) y[j] = src_up[i];
+                if (MODE == kNorm) y[j] = reinterpret_cast<const uint4*>(p.norm_w)[i];
             }
         }
 #pragma unroll

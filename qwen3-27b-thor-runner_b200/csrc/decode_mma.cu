@@ -104,9 +104,9 @@ struct ChainArgs {
 
 // Inside a chain a linear reads what an earlier linear of the same launch wrote from another SM: those
 // loads go to L2 (this SM's L1 may still hold the buffer's lines from an earlier read); a single linear
-// keeps the read-only path.
+// reads what the kernel before it wrote, which griddep_wait() has made visible to plain loads.
 template <bool CHAIN>
-__device__ __forceinline__ uint4 ld_act(const uint4* p) { return CHAIN ? __ldcg(p) : __ldg(p); }
+__device__ __forceinline__ uint4 ld_act(const uint4* p) { return CHAIN ? __ldcg(p) : *p; }
 template <bool CHAIN>
 __device__ __forceinline__ float ld_res(const __nv_bfloat16* p) {
     if (CHAIN) return __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(p)) << 16);
@@ -334,7 +334,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tm_packed0, const __grid_c
                     tk[u] = id / row_chunks;
                     const int c = id - tk[u] * row_chunks;
                     x[u] = ld_act<CHAIN>(reinterpret_cast<const uint4*>(p.A + (size_t)tk[u] * p.a_stride) + c);
-                    w[u] = __ldg(reinterpret_cast<const uint4*>(p.norm_w) + c);
+                    w[u] = reinterpret_cast<const uint4*>(p.norm_w)[c];
                 }
             }
 #pragma unroll
@@ -464,7 +464,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tm_packed0, const __grid_c
                 const int tkn = row % p.M;
                 int kc = kc0 + row / p.M;
                 if (kc >= p.kchunks) kc -= p.kchunks;
-                const uint4 w4 = __ldg(reinterpret_cast<const uint4*>(p.norm_w + kc * kKC) + (i & 31));
+                const uint4 w4 = reinterpret_cast<const uint4*>(p.norm_w + kc * kKC)[i & 31];
                 const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w};
                 const float inv = __uint_as_float(s_amax[8 + tkn]);
 #pragma unroll

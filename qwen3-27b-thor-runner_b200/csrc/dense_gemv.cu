@@ -141,7 +141,7 @@ dense_gemv_kernel(const __grid_constant__ CUtensorMap tm_w, const DenseParams p)
                     const int tk = r >> 4, c = r & 15;
                     int kc = kc0 + j;
                     if (kc >= p.kchunks) kc -= p.kchunks;
-                    x[u] = __ldg(reinterpret_cast<const uint4*>(p.A + (size_t)tk * p.K + kc * kUK) + c);
+                    x[u] = reinterpret_cast<const uint4*>(p.A + (size_t)tk * p.K + kc * kUK)[c];
                     dst[u] = (j * p.M + tk) * kTokRowBytes + c * 16;
                 }
             }

@@ -45,8 +45,8 @@ dequant_bf16_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restric
 constexpr int kSwigluHeld = 2;         // vectors of eight outputs a thread has in flight
 
 __global__ void __launch_bounds__(256)
-swiglu_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
-              __nv_bfloat16* __restrict__ out, long long row_stride_in, long long row_stride_out, int M, int I,
+swiglu_kernel(const __nv_bfloat16* gate, const __nv_bfloat16* up,
+              __nv_bfloat16* out, long long row_stride_in, long long row_stride_out, int M, int I,
               int interleaved) {
     ptx::griddep_launch_dependents();
     ptx::griddep_wait();                       // gate and up are the output of the kernel before this one
@@ -170,8 +170,7 @@ constexpr int kNormCache = 4, kNormBiasCache = 3;   // x 256 threads x 8 element
 
 template <bool BIAS>
 __global__ void __launch_bounds__(kNormThreads, 4)
-rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __restrict__ bias,
-               const __nv_bfloat16* __restrict__ weight, float eps, int K) {
+rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* bias, const __nv_bfloat16* weight, float eps, int K) {
     __shared__ float s_part[kNormThreads / 32];
     constexpr int kHeld = BIAS ? kNormBiasCache : kNormCache;
     const int tid = threadIdx.x;
@@ -180,8 +179,8 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
     ptx::griddep_launch_dependents();
     ptx::griddep_wait();                      // x (and bias) are the output of the kernel before this one
     auto load_x = [&](int c) { return *reinterpret_cast<const uint4*>(x + row + (size_t)c * 8); };
-    auto load_b = [&](int c) { return __ldg(reinterpret_cast<const uint4*>(bias + row + (size_t)c * 8)); };
-    auto load_w = [&](int c) { return __ldg(reinterpret_cast<const uint4*>(weight + (size_t)c * 8)); };
+    auto load_b = [&](int c) { return *reinterpret_cast<const uint4*>(bias + row + (size_t)c * 8); };
+    auto load_w = [&](int c) { return *reinterpret_cast<const uint4*>(weight + (size_t)c * 8); };
     auto values = [&](const uint4& a, const uint4& b, float (&v)[8]) {
         const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -194,7 +193,7 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
             }
         }
     };
-    uint4 xs[kHeld], bs[BIAS ? kHeld : 1], ws[BIAS ? 1 : kHeld];
+    uint4 xs[kHeld], bs[BIAS ? kHeld : 1], ws[kHeld];
 #pragma unroll
     for (int j = 0; j < kHeld; ++j) {
         const int c = tid + j * kNormThreads;
@@ -223,6 +222,11 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((tid & 31) == 0) s_part[tid >> 5] = ss;
+    if (BIAS) {                                  // here the registers have room; behind the first store a load would wait for the one before
+#pragma unroll
+        for (int j = 0; j < kHeld; ++j)
+            if (tid + j * kNormThreads < chunks) ws[j] = load_w(tid + j * kNormThreads);
+    }
     __syncthreads();
     float t = 0.0f;
 #pragma unroll
@@ -253,7 +257,7 @@ rmsnorm_kernel(__nv_bfloat16* out, __nv_bfloat16* x, const __nv_bfloat16* __rest
         const int c = tid + j * kNormThreads;
         float v[8];
         values(xs[j], bs[BIAS ? j : 0], v);
-        if (c < chunks) store(c, v, BIAS ? load_w(c) : ws[BIAS ? 0 : j]);
+        if (c < chunks) store(c, v, ws[j]);
     }
 }
 

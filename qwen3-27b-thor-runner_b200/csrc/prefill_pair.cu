@@ -188,7 +188,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 
 // ---------------------------------------------------------------- outputs
-__device__ __forceinline__ float token_factor(const PairParams& p, int m) { return p.unscale ? __ldg(p.unscale + m) * p.out_mul : 1.0f; }
+__device__ __forceinline__ float token_factor(const PairParams& p, int m) { return p.unscale ? p.unscale[m] * p.out_mul : 1.0f; }
 __device__ __forceinline__ float silu_pair(float gate, float up) {     // both already scaled; rounded as separate kernels would store them
     return silu(__bfloat162float(__float2bfloat16_rn(gate))) * __bfloat162float(__float2bfloat16_rn(up));
 }
@@ -252,12 +252,15 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
                 for (int i = 0; i < U; ++i) { s[i].x += x[i].x; s[i].y += x[i].y; s[i].z += x[i].z; s[i].w += x[i].w; }
             }
         }
+        float factor[U];                         // before the stores, behind which the loads would wait for one another
+#pragma unroll
+        for (int i = 0; i < U; ++i) factor[i] = b + i * nthreads < e1 ? token_factor(p, m0 + (b + i * nthreads) / (TR / 4)) : 0.0f;
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             const int e = b + i * nthreads;
             const int m = m0 + e / (TR / 4), n = n0 + e % (TR / 4) * 4;
             if (e >= e1 || n >= p.N) continue;   // N % 8 == 0: a chunk is inside or outside
-            const float mul = token_factor(p, m);
+            const float mul = factor[i];
             const float v[4] = {s[i].x * mul, s[i].y * mul, s[i].z * mul, s[i].w * mul};
             if (shift) {
                 if (e & 2) continue;

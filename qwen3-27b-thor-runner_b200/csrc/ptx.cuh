@@ -251,6 +251,8 @@ __device__ __forceinline__ void named_barrier_arrive(int id, int threads) {
 
 // Programmatic dependent launch (no-ops when the kernel was launched without the attribute).
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Behind the wait everything the kernels in front have written is there, for plain loads: not for __ldg() and const __restrict__
+// parameters, whose read-only path wants memory that nobody writes while this kernel runs, and it runs since before the wait.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // 8-byte volatile accesses (single transactions): {value, epoch} pairs exchanged between GPUs.

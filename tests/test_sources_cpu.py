@@ -38,3 +38,18 @@ def test_bf16_weight_loader_waits_for_the_stream():
     loader = src[src.index("if (warp == 2 * kGroupWarps)"):]
     loader = loader[:loader.index("return;")]
     assert "griddep_wait()" in loader and loader.index("griddep_wait()") < loader.index("tma_load_2d(")
+
+
+def test_what_the_kernel_before_writes_is_not_read_as_read_only():
+    """__ldg() and const __restrict__ parameters promise that nobody writes the memory while the kernel runs.  A kernel that starts
+    behind its predecessor runs while that one still writes; what it waits for then needs plain loads.  (A chain's parameter block
+    is written once, by the host.)"""
+    for name in sorted(os.listdir(CSRC)):
+        src = source(name) if name.endswith((".cu", ".cuh")) else ""
+        early = "ProgrammaticStreamSerialization" in src
+        for part in re.split(r"(?=__global__ )", src) if early else []:
+            head = part[:part.index("{")] if part.startswith("__global__") else ""
+            reads = [c for c in re.findall(r"__ldg\([^;]*", part) if "ch.params" not in c]
+            if head and "griddep_wait()" not in part:      # an ordinary launch in the same file
+                continue
+            assert "__restrict__" not in head and not reads, (name, head, reads)
