@@ -98,7 +98,7 @@ const char* nvfp4_status_string(int status);
  *                   expands the activations itself and no pre-pass kernel is launched; 0 = always
  *                   the pre-pass
  *   "prefill_impl": 0 = auto, 1 = dequant-to-workspace + CUDA-core GEMM (debug),
- *                   2 = fused dequant + tcgen05 GEMM
+ *                   2 = fused dequant + tcgen05 GEMM (where 0 takes the few-token kernel below: from 65 tokens on)
  *   "decode_max_m": largest M routed to the GEMV path (default 16)
  *   "wide_gemv": 1 (default) = 9..16 tokens take one launch of the wide GEMV kernel (two
  *                   8-token MMA tiles, activations streamed with the weights); 0 = off
@@ -107,7 +107,8 @@ const char* nvfp4_status_string(int status);
  *                   max 0 turns it off.  "skinny_split_cost": stage-times charged to
  *                   splitting row tiles along K when that kernel plans its work.
  *   "prefill_stream_k": 1 (default) = output tiles left over after whole waves of tiles are
- *                   split along K over all SMs; 0 = whole tiles only                */
+ *                   split along K over all SMs; 0 = whole tiles only, and from 65 tokens on
+ *                   that kernel whatever skinny_max_m says                          */
 int nvfp4_set_option(nvfp4_handle* h, const char* name, int value);
 int nvfp4_get_option(nvfp4_handle* h, const char* name, int* value);
 

@@ -173,7 +173,9 @@ int run_linear(nvfp4_handle* h, const LinearArgs& a, cudaStream_t s, size_t ws_b
         h->launches += (unsigned long long)nl;
         return cuda_status(e);
     }
-    if (fast_path_wanted && a.M >= h->skinny_min_m && a.M <= h->skinny_max_m && skinny_umma_supported(a) &&
+    // Above 64 tokens only by default: a caller who names the tcgen05 GEMM, or whole tiles, gets that kernel and what it refuses.
+    const bool prefill_named = a.M > 64 && (h->prefill_impl == 2 || !h->dev.prefill_stream_k);
+    if (fast_path_wanted && !prefill_named && a.M >= h->skinny_min_m && a.M <= h->skinny_max_m && skinny_umma_supported(a) &&
         kDecodeScratchBytes + (a.M > 64 ? prefill_umma_scratch_bytes(a.M, a.N, a.K) : prefill_umma_reserved_bytes()) <= ws_bytes) {
         int nl = 0;
         cudaError_t e = launch_skinny_umma(a, h->dev, h->workspace, ws_bytes, kDecodeScratchBytes, &nl, s);

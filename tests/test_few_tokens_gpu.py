@@ -85,3 +85,38 @@ def test_a_workspace_too_small_is_refused_as_before(handle):
         assert h.launch_count() == 0 and not C.any()
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("M", [65, 80])
+@pytest.mark.parametrize("option,value", [("prefill_impl", 2), ("prefill_stream_k", 0)])
+def test_options_that_name_the_prefill_kernel_reach_it(handle, M, option, value):
+    """Above 64 tokens the few-token kernel is the default, not what a caller gets who names another: the bits are the prefill kernel's,
+    and a number of rows that it refuses is refused."""
+    import torch
+    import nvfp4
+    N, K = 640, 5120
+    p, s = (util.to_dev(a) for a in util.make_weight(N, K, seed=M))
+    A = util.to_dev(util.make_bf16((M, K), seed=M + 1))
+
+    def call(settings):
+        old = {k: handle.get_option(k) for k in settings}
+        C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
+        try:
+            for k, v in settings.items():
+                handle.set_option(k, v)
+            handle.linear(A, M, p, s, 1.0, N, K, C)
+        finally:
+            for k, v in old.items():
+                handle.set_option(k, v)
+        return C
+
+    want = call({option: value, "skinny_max_m": 0})
+    assert not torch.equal(want, call({}))                # else the comparison below says nothing
+    assert torch.equal(want, call({option: value}))
+    if option == "prefill_impl":
+        handle.set_option(option, value)
+        try:
+            with pytest.raises(nvfp4.Nvfp4Error, match="shape"):
+                handle.linear(A, M, p, s, 1.0, N - 1, K, torch.zeros((M, N - 1), dtype=torch.int16, device="cuda"))
+        finally:
+            handle.set_option(option, 0)
