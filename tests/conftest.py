@@ -28,8 +28,14 @@ def handle():
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
     import nvfp4
     h = nvfp4.Handle(0, 512 << 20)
+    names = ("decode_impl", "prefill_impl", "decode_max_m", "prefill_stream_k", "wide_gemv", "fp4_native", "fp4_min_m", "fp4_own_quant",
+             "gemm_weight_rounding", "fp4_stream_min_m", "host_direct_out", "skinny_min_m", "skinny_max_m", "skinny_split_cost")
+    options = {name: h.get_option(name) for name in names}
     yield h
+    # a test that leaves an option changed has the ones behind it run through other kernels than users do
+    left = {name: h.get_option(name) for name in names}
     h.close()
+    assert left == options
 
 
 @pytest.fixture(scope="module")

@@ -43,11 +43,9 @@ def swiglu_of(plain, N):
 
 @pytest.fixture
 def pair_only(handle):
-    """17 to 64 tokens to the pair kernel too."""
-    handle.set_option("skinny_max_m", 0)
-    yield handle
-    handle.set_option("skinny_max_m", 64)
-    handle.set_option("gemm_weight_rounding", 0)
+    """17 to 80 tokens to the pair kernel too."""
+    with util.options(handle, skinny_max_m=0, gemm_weight_rounding=0):
+        yield handle
 
 
 @pytest.mark.parametrize("M,N,K,T,R,how", pair_forms.FP4)
@@ -172,7 +170,8 @@ def test_every_form_on_bf16_weights(handle, M, N, K, T, R, how):
     (2500, 2816, 256, False),     # many items of one stage: the rings run across items
     (1300, 5120, 768, True),      # items of two row tiles, three stages each
 ])
-def test_pair_kernel_vs_oracle(handle, M, N, K, res):
+def test_pair_kernel_vs_oracle(pair_only, M, N, K, res):
+    handle = pair_only
     packed, scale = util.make_weight(N, K, seed=M + N, sigma=0.14)
     A = util.make_bf16((M, K), seed=M + 5)
     R = util.make_bf16((M, N), seed=N + 6) if res else None
@@ -184,9 +183,10 @@ def test_pair_kernel_vs_oracle(handle, M, N, K, res):
 
 
 @pytest.mark.parametrize("M,N,K", [(70, 96, 256), (150, 5120, 2560), (333, 1024, 4352)])
-def test_swiglu_output_equals_linear_and_swiglu(handle, M, N, K):
+def test_swiglu_output_equals_linear_and_swiglu(pair_only, M, N, K):
     """Interleaved rows (8 gate, 8 up): the SwiGLU of the plain call's rounded outputs."""
     import torch
+    handle = pair_only
     packed, scale = util.make_weight(N, K, seed=M, sigma=0.14)
     A = util.make_bf16((M, K), seed=M + 1)
     dA, dp, ds = util.to_dev(A), util.to_dev(packed), util.to_dev(scale)
@@ -251,10 +251,11 @@ def test_few_tokens_need_the_kernels_whole_scratch(option, value, M):
 
 
 @pytest.mark.parametrize("M", [65, 300])
-def test_weights_follow_the_stream(handle, M):
+def test_weights_follow_the_stream(pair_only, M):
     """A weight written by the work right before the call, again and again into the same buffers: by a copy, and by a call of
     this library whose BF16 output serves as the codes (that kernel lets the next one start early)."""
     import torch
+    handle = pair_only
     N, K = 2048, 1024                                    # the second weight is the first call's [T, 256] output: N * K / 2 bytes
     T, K1 = 2048, 2560
     A = util.to_dev(util.make_bf16((M, K), seed=M))

@@ -14,13 +14,8 @@ TOL = 1e-3   # relative Frobenius error against the oracle
 
 @pytest.fixture()
 def skinny(handle):
-    handle.set_option("skinny_min_m", 1)
-    handle.set_option("skinny_max_m", 128)
-    handle.set_option("wide_gemv", 0)
-    yield handle
-    handle.set_option("wide_gemv", 1)
-    handle.set_option("skinny_min_m", 9)
-    handle.set_option("skinny_max_m", 64)
+    with util.options(handle, skinny_min_m=1, skinny_max_m=128, wide_gemv=0):
+        yield handle
 
 
 def run(h, A, packed, scale, gs, residual=None):

@@ -1,5 +1,7 @@
 """Seeded synthetic inputs in the reference's NVFP4 layout, shared by tests, golden
 generation and the benchmark's parity spot-checks.  numpy only."""
+import contextlib
+
 import numpy as np
 
 import oracle_binding as ob
@@ -47,3 +49,16 @@ def pad_cols(a, cols):
     out = np.zeros((a.shape[0], cols), a.dtype)
     out[:, :a.shape[1]] = a
     return out
+
+
+@contextlib.contextmanager
+def options(handle, **values):
+    """Sets options of a handle and puts back what was there."""
+    before = {name: handle.get_option(name) for name in values}
+    try:
+        for name, value in values.items():
+            handle.set_option(name, value)
+        yield handle
+    finally:
+        for name, value in before.items():
+            handle.set_option(name, value)
