@@ -44,6 +44,43 @@ def test_against_the_oracle(handle, M, N, K, res):
     assert ob.rel_frobenius(outs[0], ob.linear(A, packed, scale, 1.5, residual=R if res else None, mode=ob.GEMV, threads=8)) <= TOL
 
 
+@pytest.mark.parametrize("writer", ["linear", "swiglu"])
+@pytest.mark.parametrize("M", [65, 80])
+def test_weights_follow_a_kernel_that_lets_its_successor_start(handle, M, writer):
+    """The codes are the BF16 output of a library call right before, which leaves most SMs idle and lets its successor start early
+    (SwiGLU at its first instruction); a copy, as below, never does.  The bits of the synchronised sequence."""
+    import torch
+    N, K = 2048, 1024                                    # N * K / 2 bytes of codes: an output of [T, 256]
+    T, K1 = 2048, 2560
+    A, A1 = util.to_dev(util.make_bf16((M, K), seed=M)), util.to_dev(util.make_bf16((T, K1), seed=M + 1))
+    w1 = [tuple(util.to_dev(a) for a in util.make_weight(256, K1, seed=M + 2 + i, sigma=0.14)) for i in range(3)]
+    gate_up = [util.to_dev(util.make_bf16((T, 512), seed=M + 10 + i)) for i in range(3)]
+    scale = util.to_dev(util.make_weight(N, K, seed=M + 20, sigma=0.14)[1])
+    made = torch.empty((T, 256), dtype=torch.int16, device="cuda")
+    codes = made.view(torch.uint8).view(N, K // 2)
+
+    def step(i, out, wait):
+        if writer == "linear":
+            handle.linear(A1, T, w1[i][0], w1[i][1], 1.0, 256, K1, made)
+        else:
+            handle.swiglu(gate_up[i], None, T, 256, made)
+        if wait:
+            torch.cuda.synchronize()
+        handle.linear(A, M, codes, scale, 1.0, N, K, out)
+        if wait:
+            torch.cuda.synchronize()
+
+    want = [torch.empty((M, N), dtype=torch.int16, device="cuda") for _ in range(3)]
+    for i in range(3):
+        step(i, want[i], True)
+    assert not torch.equal(want[0], want[1])
+    for r in range(30):
+        got = torch.empty((M, N), dtype=torch.int16, device="cuda")
+        step(r % 3, got, False)
+        assert torch.equal(got, want[r % 3]), r
+    assert handle.device_status() == 0
+
+
 @pytest.mark.parametrize("M", [65, 80])
 def test_weights_follow_the_stream_beyond_64_tokens(handle, M):
     """A weight copied into place right before the call, on the same stream, is the one that is used."""
@@ -98,25 +135,15 @@ def test_options_that_name_the_prefill_kernel_reach_it(handle, M, option, value)
     p, s = (util.to_dev(a) for a in util.make_weight(N, K, seed=M))
     A = util.to_dev(util.make_bf16((M, K), seed=M + 1))
 
-    def call(settings):
-        old = {k: handle.get_option(k) for k in settings}
+    def call(**settings):
         C = torch.zeros((M, N), dtype=torch.int16, device="cuda")
-        try:
-            for k, v in settings.items():
-                handle.set_option(k, v)
+        with util.options(handle, **settings):
             handle.linear(A, M, p, s, 1.0, N, K, C)
-        finally:
-            for k, v in old.items():
-                handle.set_option(k, v)
         return C
 
-    want = call({option: value, "skinny_max_m": 0})
-    assert not torch.equal(want, call({}))                # else the comparison below says nothing
-    assert torch.equal(want, call({option: value}))
+    want = call(skinny_max_m=0, **{option: value})
+    assert not torch.equal(want, call())                  # else the comparison below says nothing
+    assert torch.equal(want, call(**{option: value}))
     if option == "prefill_impl":
-        handle.set_option(option, value)
-        try:
-            with pytest.raises(nvfp4.Nvfp4Error, match="shape"):
-                handle.linear(A, M, p, s, 1.0, N - 1, K, torch.zeros((M, N - 1), dtype=torch.int16, device="cuda"))
-        finally:
-            handle.set_option(option, 0)
+        with util.options(handle, prefill_impl=value), pytest.raises(nvfp4.Nvfp4Error, match="shape"):
+            handle.linear(A, M, p, s, 1.0, N - 1, K, torch.zeros((M, N - 1), dtype=torch.int16, device="cuda"))
