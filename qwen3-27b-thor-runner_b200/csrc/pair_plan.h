@@ -92,6 +92,13 @@ struct Work {          // of pair `id` of `pairs`
     }
 };
 
+// The kernel's ring of A units.  Above kCoarseT tokens a tile, and for BF16 weights, it has two units of 64 k for each planned one, and in
+// tensor memory (NVFP4) two more in an odd 64 columns: `spare` of them.  Two groups of warps take every other unit: an even number.
+constexpr int kCoarseT = 128;
+constexpr int kRingMax = 2 * kMaxUnits;
+NVFP4_HD int spare_units(const Plan& p, bool fine, bool dense) { return fine && !dense ? (p.a_col0 - p.accs * p.T) / kUnitCols * 2 : 0; }
+NVFP4_HD int ring_units(const Plan& p, bool fine, bool dense) { return fine ? 2 * p.units + spare_units(p, fine, dense) : p.units; }
+
 // Pairs first..last hold the parts of split tile `tile`, of which pair `id` holds one; the first one holds its head (slot 1),
 // the others a middle or tail (slot 0).
 NVFP4_HD void participants(const Plan& p, int kstages, int pairs, int id, int tile, int& first, int& last) {
@@ -118,8 +125,8 @@ constexpr Prices kPricesFp4 = {95.0, 37.0, 4608.0, 3.2, 5.4, 650.0, 7100.0, 27.0
 constexpr Prices kPricesBf16 = {73.5, 68.0, 16384.0, 6.2, 18.8, 1060.0, 7900.0, 35.5, 600.0, 11400.0, 670.0, 188.0, 46.0};
 
 // Fills the tile plan of a launch (p.M, p.N and p.K are set) for at most `pairs` CTA pairs; returns the pairs it runs on, and the
-// dynamic shared memory of a CTA in *smem.
-inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem) {
+// dynamic shared memory of a CTA in *smem.  `prices` choose among plans that are all valid.
+inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem, const Prices* prices = nullptr) {
     const int kst = p.K / WK;
     p.row_tiles = (p.N + 2 * TR - 1) / (2 * TR);
     // T up to 192: two accumulators and two 64-column A units (four of 64 k in the kernel) fill tensor memory.  BF16 weights: up to 224, four 32 KB A units
@@ -131,7 +138,7 @@ inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem) {
     // 17408, weights from memory): the plan chosen is 0.2 (BF16 1.0) % slower than the best one on average, 1.4 (5.6) at the 95th
     // percentile.  The list before it was fitted to large weights only, charged 23,500 clocks for any split and had none for
     // fewer stages than pairs: 65 x 512 x 5120 ran whole in 25 us, 14 split.
-    const Prices& c = dense ? kPricesBf16 : kPricesFp4;
+    const Prices& c = prices ? *prices : dense ? kPricesBf16 : kPricesFp4;
     double best = 1e30;
     int used = 1;
     for (int T = 32; T <= t_max; T += 32) {
@@ -178,7 +185,7 @@ inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem) {
                 }
             }
             const long long on = sk * kst < pairs ? sk * kst : pairs;
-            if (on >= sk)
+            if ((sk * kst + on - 1) / on < kst)                    // no part is a whole tile: the kernel for plans split all over has none
                 take((double)((sk * kst + on - 1) / on) * kBlocks * blk1 + c.split + 2.0 * c.split_token * tokens + c.part * on / sk + c.straddle + c.pair * on,
                      true, on);
         }

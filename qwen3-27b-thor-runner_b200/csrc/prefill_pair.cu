@@ -61,8 +61,6 @@ using namespace umma;
 constexpr int kThreads = 640;
 constexpr int kGroupWarps = 4, kEpiWarps = 4;  // two dequantising groups of four warps (one per TMEM lane quarter)
 constexpr int kMaxT = 256;                     // columns a partial slot has room for
-constexpr int kCoarseT = 128;                  // up to this many tokens a tile, an A unit of NVFP4 weights is 128 k
-constexpr int kRingMax = 2 * kMaxUnits;
 constexpr int kSlotFloats = TR * kMaxT;        // one FP32 partial: [token][row]
 
 struct PairParams : Plan {
@@ -318,9 +316,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)ptx::cluster_ctarank();
     const int kstages = p.K / WK;
-    // The ring of A: FINE two units of 64 k for each planned one, and in tensor memory two more in an odd 64 columns.
-    const int spare = FINE && MODE != kDense ? (p.a_col0 - p.accs * p.T) / kUnitCols * 2 : 0;
-    const int ring = FINE ? 2 * p.units + spare : p.units;
+    const int spare = spare_units(p, FINE, MODE == kDense), ring = ring_units(p, FINE, MODE == kDense);      // FINE: units of 64 k
     constexpr uint32_t kRingCols = FINE ? kUnitCols / 2 : kUnitCols;
 
     if (tid == 0) {

@@ -23,10 +23,10 @@ def lib(tmp_path_factory):
 
 
 def plan(lib, M, N, K, dense=False, pairs=PAIRS, stream_k=True):
-    out = (ctypes.c_int * 14)()
+    out = (ctypes.c_int * 15)()
     lib.pair_plan(M, N, K, pairs, int(stream_k), int(dense), out)
     p = dict(zip(("T", "R", "m_tiles", "row_tiles", "items", "dp_items", "sk_tiles", "w_stages", "x_stages", "units", "accs", "a_col0",
-                  "smem", "pairs"), out))
+                  "smem", "pairs", "ring"), out))
     p["how"] = ("whole" if not p["sk_tiles"] else "tail" if p["dp_items"] else
                 "parts" if p["pairs"] % p["sk_tiles"] == 0 else "straddle")
     return p
@@ -48,21 +48,24 @@ def _shapes(count):
 
 
 def test_every_output_is_summed_once(lib):
-    """All pairs' lists together: each stage of each tile once, no partial slot twice, all holders of a tile agree on the others."""
+    """All pairs' lists together: each stage of each tile once, no partial slot twice, all holders of a tile agree on the others, no whole
+    tile among the parts of a plan that is split all over.  Whatever the prices are: they choose among valid plans."""
     for M, N, K, dense, pairs in _shapes(2500):
-        for stream_k in (0, 1):
-            assert lib.pair_walk(M, N, K, pairs, stream_k, int(dense)) == 0, (M, N, K, dense, pairs, stream_k)
+        for stream_k, prices in ((0, 0), (1, 0), (1, 1)):
+            assert lib.pair_walk(M, N, K, pairs, stream_k, int(dense), prices) == 0, (M, N, K, dense, pairs, stream_k, prices)
 
 
 def test_plans_stay_within_the_chip(lib):
     """Shared memory, tensor memory (512 columns) and what the issuers rely on: an even number of units and accumulators, two token
-    stages a turn and one more."""
+    stages a turn and one more; a ring of an even number of units that has barriers (16) and, in tensor memory, columns."""
     for M, N, K, dense, pairs in _shapes(4000):
         p = plan(lib, M, N, K, dense, pairs)
         assert p["smem"] <= 225 * 1024 and 3 <= p["x_stages"] <= 8 and p["w_stages"] <= 8
         assert p["units"] in (2, 4, 6, 8) and p["accs"] in (2, 4)
         assert p["T"] % 32 == 0 and 32 <= p["T"] <= (224 if dense else 192) and p["R"] in (1, 2)
         assert p["accs"] * p["T"] <= (512 if dense else p["a_col0"]) and (dense or p["a_col0"] + 64 * p["units"] == 512)
+        assert p["ring"] % 2 == 0 and p["units"] <= p["ring"] <= 16
+        assert dense or p["accs"] * p["T"] + p["ring"] * (32 if p["T"] > 128 else 64) <= 512
         assert 1 <= p["pairs"] <= pairs
 
 
