@@ -81,6 +81,12 @@ def test_small_weights_are_split(lib, M, N, K, dense, at_most):
     assert -(-(K // 256) // (p["pairs"] // p["sk_tiles"])) <= at_most
 
 
+def elects(src):
+    """Functions of the source that elect a lane of the whole warp."""
+    functions = re.split(r"(?=__device__ __forceinline__ )", src[:src.index("__global__ ")])
+    return sorted({re.match(r"__device__ __forceinline__ \w+ (\w+)\(", f).group(1) for f in functions if "elect.sync" in f})
+
+
 def test_issuing_warps_decide_as_a_whole():
     """The issuers elect a lane of the full warp for every MMA and commit, so a lane that leaves the loop alone (its wait ran out,
     another lane's did not) would leave the rest waiting without a limit.  No wait on a GPU can be made to run out in some lanes
@@ -90,6 +96,9 @@ def test_issuing_warps_decide_as_a_whole():
     loop = issuer[issuer.index("for (int turn = 0;"):]
     assert re.match(r"for \(int turn = 0; turn < turns; \+\+turn\)", loop)            # not on the lane's own `ok`
     vote = loop.index("ok = __all_sync(0xffffffffu, ok);")
-    elections = [loop.index(f) for f in ("mma8_ss(", "mma8_ts(", "commit_leader(")]
-    assert loop.rindex("ptx::mbar_wait(") < vote < loop.index("break;") < min(elections)
+    assert set(re.findall(r"\b((?:mma|commit)\w*)\(", issuer)) <= set(elects(src))
+    elections = [m.start() for m in re.finditer(r"\b(?:%s)\(" % "|".join(elects(src)), loop)]
+    # the commit behind the loop stands behind the voted `ok` itself
+    assert len(elections) >= 7 and loop.rindex("ptx::mbar_wait(") < vote < loop.index("break;") < min(elections)
+    assert re.search(r"if \(ok\) commit_pair\(tfull0", loop) and "ok =" not in loop[loop.index("break;"):]
     assert loop.count("break;") == 1 and "return" not in loop and "continue" not in loop
