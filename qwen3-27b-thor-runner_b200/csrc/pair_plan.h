@@ -92,12 +92,23 @@ struct Work {          // of pair `id` of `pairs`
     }
 };
 
-// The kernel's ring of A units.  Above kCoarseT tokens a tile, and for BF16 weights, it has two units of 64 k for each planned one, and in
-// tensor memory (NVFP4) two more in an odd 64 columns: `spare` of them.  Two groups of warps take every other unit: an even number.
+// The kernel's ring of A units: the planned ones of 128 k, or two of 64 k for each ("fine") and in tensor memory (NVFP4) two more in an odd
+// 64 columns (`spare_units` of them).  Two groups of warps take every other unit: an even number.
+// NVFP4 takes 64 k where tensor memory has room for two units of 128 k only, above 128 tokens a tile.  BF16, whose blocks lie in shared
+// memory, takes it up to 128 tokens a tile; beyond, a unit of 64 k is twice the waits and commits, but one row tile a turn takes two
+// token stages of few when its unit is 128 k.  So an item of two row tiles has 128 k (4096 x 5120 x 17408 at T = 192 530 us with 64 k,
+// 510 with 128, 4096 x 34816 x 5120 at T = 160 1145 and 1077), one of one row tile 64 k (480 x 5120 x 17408 67.9 and 78.2), which
+// goes for plans with a tenth of their tiles in parts too (20 of 168 104.0 and 105.5, 96 of 392 244 and 260, but 8 of 896 520 and 502).
+// At T = 160 and one or two token tiles the weights' stream is the bound and 64 k is 1 % ahead (320 x 34816 x 5120 87.5 and 88.3).
 constexpr int kCoarseT = 128;
 constexpr int kRingMax = 2 * kMaxUnits;
-NVFP4_HD int spare_units(const Plan& p, bool fine, bool dense) { return fine && !dense ? (p.a_col0 - p.accs * p.T) / kUnitCols * 2 : 0; }
-NVFP4_HD int ring_units(const Plan& p, bool fine, bool dense) { return fine ? 2 * p.units + spare_units(p, fine, dense) : p.units; }
+NVFP4_HD bool fine_units(const Plan& p, bool dense) {
+    if (!dense) return p.T > kCoarseT;
+    const bool parts = 10LL * p.sk_tiles >= (long long)p.items * p.R;
+    return p.T <= kCoarseT || p.R == 1 || parts || (p.T <= 160 && p.m_tiles <= 2);
+}
+NVFP4_HD int spare_units(const Plan& p, bool dense) { return !dense && fine_units(p, dense) ? (p.a_col0 - p.accs * p.T) / kUnitCols * 2 : 0; }
+NVFP4_HD int ring_units(const Plan& p, bool dense) { return fine_units(p, dense) ? 2 * p.units + spare_units(p, dense) : p.units; }
 
 // Pairs first..last hold the parts of split tile `tile`, of which pair `id` holds one; the first one holds its head (slot 1),
 // the others a middle or tail (slot 0).

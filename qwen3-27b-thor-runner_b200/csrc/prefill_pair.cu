@@ -93,8 +93,8 @@ struct Ring {
 
 // ---------------------------------------------------------------- tcgen05, CTA pairs
 // The MMAs of a unit on one accumulator, which the first clears when `accumulate` is 0, from one elected lane of a converged
-// warp: eight (128 k, B in two blocks `step` 16-byte units apart) or, without `step`, the four of one block (64 k).  A from tensor
-// memory (8 columns per MMA) or from a shared-memory block.  Election and address arithmetic sit inside one asm block: the issuing warp shares its scheduler
+// warp: eight (128 k, B in two blocks `step` 16-byte units apart) or the four of one block (64 k).  A from tensor memory (8 columns
+// per MMA) or from shared memory (two blocks 16 KB apart, or one).  Election and address arithmetic sit inside one asm block: the issuing warp shares its scheduler
 // and instruction cache with the dequantising warps, and every instruction of its loop counts.
 __device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t step, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -114,7 +114,7 @@ __device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint
         ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(step)
         : "memory");
 }
-__device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma4_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
         "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
@@ -128,7 +128,27 @@ __device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint
         ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void mma8_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma8_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t step, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 s, a1, a2, a3, a4, a5, a6, a7, b1, b2, b3, b4, b5, b6, b7;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tcvt.u64.u32 s, %5;\n\t"
+        "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\tadd.u64 a4, %1, 1024;\n\t"
+        "add.u64 a5, a4, 2;\n\tadd.u64 a6, a4, 4;\n\tadd.u64 a7, a4, 6;\n\t"
+        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\tadd.u64 b4, %2, s;\n\t"
+        "add.u64 b5, b4, 2;\n\tadd.u64 b6, b4, 4;\n\tadd.u64 b7, b4, 6;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a4, b4, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a5, b5, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a6, b6, %3, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a7, b7, %3, t;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(step)
+        : "memory");
+}
+__device__ __forceinline__ void mma4_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
         "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\t"
@@ -316,8 +336,9 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)ptx::cluster_ctarank();
     const int kstages = p.K / WK;
-    const int spare = spare_units(p, FINE, MODE == kDense), ring = ring_units(p, FINE, MODE == kDense);      // FINE: units of 64 k
+    const int spare = spare_units(p, MODE == kDense), ring = ring_units(p, MODE == kDense);
     constexpr uint32_t kRingCols = FINE ? kUnitCols / 2 : kUnitCols;
+    constexpr int kUnitK = FINE ? BK : XK, kLoadBytes = FINE ? kDenseBlockBytes : kDenseUnitBytes;      // of a unit (the latter: BF16, a CTA's)
 
     if (tid == 0) {
         for (int i = 0; i < kRingMax; ++i) { ptx::mbar_init(&afull[i], MODE == kDense ? 1 : 2 * kGroupWarps); ptx::mbar_init(&aempty[i], 1); }
@@ -353,12 +374,13 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
             s = me;
             ptx::griddep_wait();           // a BF16 weight may come from the kernel right before; there is no pre-pass to stream behind
             while (work.next(p, it)) {
-                const int row = ((it.rt + (it.rows == 2 ? me : 0)) * 2 + rank) * TR, step = it.rows == 2 ? BK : 2 * BK;
-                for (int k = it.ks0 * WK + (it.rows == 2 ? 0 : me * BK); k < it.ks1 * WK; k += step) {
+                const int row = ((it.rt + (it.rows == 2 ? me : 0)) * 2 + rank) * TR, step = it.rows == 2 ? kUnitK : 2 * kUnitK;
+                for (int k = it.ks0 * WK + (it.rows == 2 ? 0 : me * kUnitK); k < it.ks1 * WK; k += step) {
                     const bool ok = ptx::mbar_wait(&aempty[s], ph ^ 1u, s_abort, p.status, 0x410u + s);
                     if (ptx::elect_one() && ok) {
-                        if (rank == 0) ptx::mbar_arrive_expect_tx(&afull[s], 2 * kDenseBlockBytes);
-                        ptx::tma_load_2d_pair(s_w + s * kDenseBlockBytes, &tm_w, full0 + s * 8, k, row, pol);
+                        if (rank == 0) ptx::mbar_arrive_expect_tx(&afull[s], 2 * kLoadBytes);
+                        ptx::tma_load_2d_pair(s_w + s * kLoadBytes, &tm_w, full0 + s * 8, k, row, pol);
+                        if (!FINE) ptx::tma_load_2d_pair(s_w + s * kLoadBytes + kDenseBlockBytes, &tm_w, full0 + s * 8, k + BK, row, pol);
                     }
                     s += 2;
                     if (s >= ring) { s = me; ph ^= 1u; }
@@ -465,8 +487,10 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t xdesc = umma_desc_sw128(x0 + (uint32_t)(pairwise && me ? y.i : x.i) * xbytes + (second || (FINE && one && me) ? xhalf : 0u));
-                    if (MODE == kDense) mma8_ss(d, umma_desc_sw128(ptx::smem_u32(s_w) + (uint32_t)u.i * kDenseBlockBytes), xdesc, p.idesc, (uint32_t)turn);
-                    else if (FINE) mma8_ts(d, a_col0 + (uint32_t)u.i * kRingCols, xdesc, p.idesc, (uint32_t)turn);
+                    const uint64_t wdesc = umma_desc_sw128(ptx::smem_u32(s_w) + (uint32_t)u.i * kLoadBytes);
+                    if (MODE == kDense && FINE) mma4_ss(d, wdesc, xdesc, p.idesc, (uint32_t)turn);
+                    else if (MODE == kDense) mma8_ss(d, wdesc, xdesc, xhalf >> 4, p.idesc, (uint32_t)turn);
+                    else if (FINE) mma4_ts(d, a_col0 + (uint32_t)u.i * kRingCols, xdesc, p.idesc, (uint32_t)turn);
                     else mma8_ts(d, a_col0 + (uint32_t)u.i * kRingCols, xdesc, xhalf >> 4, p.idesc, (uint32_t)turn);
                     commit_pair(aempty0 + (uint32_t)u.i * 8, other);
                     u.advance(2);
@@ -780,23 +804,29 @@ cudaError_t launch_as(const PairParams& p, int grid, int smem, const CUtensorMap
     return cudaLaunchKernelEx(&cfg, prefill_pair_kernel<MODE, FINE, SPLIT>, tma, tmw, tms, p);
 }
 
+template <int MODE, bool FINE>
+cudaError_t launch_split(const PairParams& p, int grid, int smem, const CUtensorMap& tma, const CUtensorMap& tmw, const CUtensorMap& tms,
+                   cudaStream_t s) {
+    if (p.sk_tiles == 0) return launch_as<MODE, FINE, kWhole>(p, grid, smem, tma, tmw, tms, s);
+    if (p.dp_items == 0) {
+        if constexpr (MODE == kDense && !FINE) return cudaErrorInvalidValue;      // two row tiles an item: never split all over
+        else return launch_as<MODE, FINE, kAllSplit>(p, grid, smem, tma, tmw, tms, s);
+    }
+    return launch_as<MODE, FINE, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
+}
+
 template <int MODE>
 cudaError_t launch(const PairParams& p, int grid, int smem, const CUtensorMap& tma, const CUtensorMap& tmw, const CUtensorMap& tms,
                    cudaStream_t s) {
-    const int split = p.sk_tiles == 0 ? kWhole : (p.dp_items == 0 ? kAllSplit : kTailSplit);
-    if (MODE == kDense || p.T > kCoarseT)
-        return split == kWhole ? launch_as<MODE, true, kWhole>(p, grid, smem, tma, tmw, tms, s)
-               : split == kAllSplit ? launch_as<MODE, true, kAllSplit>(p, grid, smem, tma, tmw, tms, s)
-                                    : launch_as<MODE, true, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
-    return split == kWhole ? launch_as<MODE, MODE == kDense, kWhole>(p, grid, smem, tma, tmw, tms, s)
-           : split == kAllSplit ? launch_as<MODE, MODE == kDense, kAllSplit>(p, grid, smem, tma, tmw, tms, s)
-                                : launch_as<MODE, MODE == kDense, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
+    return fine_units(p, MODE == kDense) ? launch_split<MODE, true>(p, grid, smem, tma, tmw, tms, s)
+                                         : launch_split<MODE, false>(p, grid, smem, tma, tmw, tms, s);
 }
 
 template <int MODE, bool FINE>
 cudaError_t configure() {
     cudaError_t e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kWhole>, kSmemMax);
-    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kAllSplit>, kSmemMax);
+    if constexpr (MODE != kDense || FINE)
+        if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kAllSplit>, kSmemMax);
     if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kTailSplit>, kSmemMax);
     return e;
 }
@@ -825,6 +855,7 @@ cudaError_t configure_prefill_umma(nvfp4_device_info& dev) {
     if (e == cudaSuccess) e = configure<kExact, true>();
     if (e == cudaSuccess) e = configure<kRounded, false>();
     if (e == cudaSuccess) e = configure<kRounded, true>();
+    if (e == cudaSuccess) e = configure<kDense, false>();
     if (e == cudaSuccess) e = configure<kDense, true>();
     if (e != cudaSuccess) return e;
     // The split tiles need every pair resident at once: no more pairs than the device can place.

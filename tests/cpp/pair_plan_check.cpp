@@ -14,8 +14,17 @@ void pair_plan(int M, int N, int K, int pairs, int stream_k, int dense, int* out
     int smem = 0;
     const int used = make_plan(p, pairs, stream_k != 0, dense != 0, &smem);
     const int v[] = {p.T, p.R, p.m_tiles, p.row_tiles, p.items, p.dp_items, p.sk_tiles, p.w_stages, p.x_stages, p.units, p.accs, p.a_col0, smem, used,
-                     ring_units(p, dense || p.T > kCoarseT, dense != 0)};
+                     ring_units(p, dense != 0)};
     for (int i = 0; i < (int)(sizeof v / sizeof v[0]); ++i) out[i] = v[i];
+}
+
+// Whether the plan's units are 64 k.
+int pair_fine(int M, int N, int K, int pairs, int dense) {
+    Plan p{};
+    p.M = M; p.N = N; p.K = K;
+    int smem = 0;
+    make_plan(p, pairs, true, dense != 0, &smem);
+    return fine_units(p, dense != 0);
 }
 
 // Walks all pairs' lists.  0: every (row tile, token tile, k stage) that holds outputs is worked on exactly once, no pair writes a

@@ -29,6 +29,14 @@ FP4 = [
 BF16 = [
     (163, 19000, 256, 192, 2, "whole"),
     (194, 19048, 256, 224, 2, "whole"),
+    (129, 19584, 1024, 160, 2, "whole"),      # units of 64 k, several stages, an odd number of row tiles
+    (391, 9232, 1024, 160, 2, "whole"),       # units of 128 k from here on
+    (484, 19488, 1024, 192, 2, "whole"),
+    (649, 19144, 1024, 224, 2, "whole"),
+    (327, 19152, 5376, 192, 2, "tail"),       # 4 of 152 tiles in parts
+    (387, 19136, 6656, 224, 2, "tail"),
+    (327, 21080, 6400, 192, 2, "tail"),       # 20 of 168: units of 64 k
+    (643, 15208, 5120, 224, 2, "tail"),
     (86, 552, 7424, 32, 1, "parts"),
     (194, 616, 4096, 64, 1, "parts"),
     (150, 1784, 4096, 96, 1, "parts"),

@@ -64,9 +64,12 @@ def test_plans_stay_within_the_chip(lib):
         assert p["units"] in (2, 4, 6, 8) and p["accs"] in (2, 4)
         assert p["T"] % 32 == 0 and 32 <= p["T"] <= (224 if dense else 192) and p["R"] in (1, 2)
         assert p["accs"] * p["T"] <= (512 if dense else p["a_col0"]) and (dense or p["a_col0"] + 64 * p["units"] == 512)
-        assert p["ring"] % 2 == 0 and p["units"] <= p["ring"] <= 16
-        assert dense or p["accs"] * p["T"] + p["ring"] * (32 if p["T"] > 128 else 64) <= 512
+        fine = lib.pair_fine(M, N, K, pairs, int(dense))
+        assert p["ring"] % 2 == 0 and p["units"] << fine <= p["ring"] <= 16
+        assert dense or p["accs"] * p["T"] + p["ring"] * (32 if fine else 64) <= 512
+        assert not dense or p["ring"] * (16384 if fine else 32768) == p["units"] * 32768      # the loaders' blocks fill the ring exactly
         assert 1 <= p["pairs"] <= pairs
+        assert not dense or fine or p["dp_items"] > 0               # the kernel has no such form
 
 
 @pytest.mark.parametrize("M,N,K,dense,at_most", [
