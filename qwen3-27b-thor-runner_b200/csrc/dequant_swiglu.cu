@@ -42,7 +42,8 @@ dequant_bf16_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restric
 // Few tokens: bound by the launch, so it starts while the kernel before it finishes and lets the one behind it start its
 // prologue (a few-token linear: its weight stream).  With the norm below: an MLP of 5120 x 17408 on 40 tokens 69.8 -> 64.9 us,
 // two decode layers of 4 tokens 132.8 -> 131.0 (replayed from a graph, where plain launches follow each other faster).
-constexpr int kSwigluHeld = 2;         // vectors of eight outputs a thread has in flight
+// One vector of eight outputs a thread and step: two in flight took 53 registers instead of 34, and so half as many threads on an SM
+// (149 x 17408 4.3 us, with two 5.2; 1024 x 5120 7.4 and 8.9; 8192 x 17408 166 and 167).
 
 __global__ void __launch_bounds__(256)
 swiglu_kernel(const __nv_bfloat16* gate, const __nv_bfloat16* up,
@@ -55,30 +56,24 @@ swiglu_kernel(const __nv_bfloat16* gate, const __nv_bfloat16* up,
     const long long stride = (long long)gridDim.x * blockDim.x;
     long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v < total) {
-        // row and column of vector v, carried along instead of divided out each time
-        const int dm = (int)(stride / vec_per_row), dc = (int)(stride % vec_per_row);
-        int m = (int)(v / vec_per_row), c = (int)(v % vec_per_row);
-        while (v < total) {
-            uint4 g4[kSwigluHeld], u4[kSwigluHeld];
-            size_t to[kSwigluHeld];
-            bool live[kSwigluHeld];
-#pragma unroll
-            for (int j = 0; j < kSwigluHeld; ++j) {
-                live[j] = v < total;
-                to[j] = (size_t)m * row_stride_out + c * 8;
-                if (live[j]) {
-                    const size_t from = (size_t)m * row_stride_in + (interleaved ? 16 : 8) * c;
-                    g4[j] = *reinterpret_cast<const uint4*>(gate + from);
-                    u4[j] = *reinterpret_cast<const uint4*>(up + from);
-                }
-                v += stride;
+        const unsigned vec = (unsigned)vec_per_row;
+        int m = total <= 0xffffffffLL ? (int)((unsigned)v / vec) : (int)(v / vec_per_row);
+        int c = (int)(v - (long long)m * vec_per_row);
+        auto one = [&]() {
+            const size_t from = (size_t)m * row_stride_in + (interleaved ? 16 : 8) * c;
+            const uint4 g4 = *reinterpret_cast<const uint4*>(gate + from), u4 = *reinterpret_cast<const uint4*>(up + from);
+            *reinterpret_cast<uint4*>(out + (size_t)m * row_stride_out + c * 8) = swiglu_bf16x8(g4, u4);
+        };
+        one();
+        if ((v += stride) < total) {
+            // row and column carried along instead of divided out each time (the grid is small: 32 bits hold the stride)
+            const int dm = (int)((unsigned)stride / vec), dc = (int)((unsigned)stride - (unsigned)dm * vec);
+            do {
                 m += dm;
                 c += dc;
                 if (c >= vec_per_row) { c -= vec_per_row; ++m; }
-            }
-#pragma unroll
-            for (int j = 0; j < kSwigluHeld; ++j)
-                if (live[j]) *reinterpret_cast<uint4*>(out + to[j]) = swiglu_bf16x8(g4[j], u4[j]);
+                one();
+            } while ((v += stride) < total);
         }
     }
     // I % 8 tail columns, scalar.
