@@ -215,8 +215,16 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
     *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
+// SPLIT: what the plan left to split by k.  An instantiation each, because the registers run out (96 a thread): with the code of
+// parts and reduction in one kernel every call paid for its spills, 0.5-1 us (149 x 5120 x 17408 35.7 -> 34.4 us, BF16 100 x 5120 x 5120
+// 19.1 -> 17.9), and whole items had none left to ask for the residual a chunk ahead (2048 x 5120 x 5120 with a residual 92 -> 83.4).
+// Split tiles behind whole waves have it all, hence one for calls with a residual (which have neither SwiGLU nor FP32 outputs) and one for
+// those without: in one, the residual was waited for element by element (2048 x 17408 x 5120 with one 385 us).
+enum Split { kWhole = 0, kAllSplit = 1, kTailSplit = 2, kTailSplitRes = 3 };
+
 // Every participant calls this once its own parts are stored: it waits (bounded) for the parts of the others -- the CTAs of
 // the same rank in their pairs, which hold the same 128 rows -- and sums its own 1/P of the tile in pair order.
+template <int SPLIT>
 __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int epoch, int tile, int kstages, int t, int nthreads,
                                              volatile int* s_abort) {
     int first, last;
@@ -247,7 +255,8 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
     const int e0 = (int)((long long)me * total / P), e1 = (int)((long long)(me + 1) * total / P);
     const float4* parts = reinterpret_cast<const float4*>(p.partials);
     const float4* head = parts + ((size_t)(2 * first + rank) * 2 + 1) * (kSlotFloats / 4);
-    const int shift = p.swiglu_out ? 2 : 0;      // an up chunk lies two chunks behind its gate chunk
+    const bool has_residual = SPLIT == kTailSplitRes || (SPLIT != kTailSplit && p.residual);
+    const int shift = SPLIT != kTailSplitRes && p.swiglu_out ? 2 : 0;      // an up chunk lies two chunks behind its gate chunk
     constexpr int U = 4;                         // loads of four chunks in flight: the reduction is L2 round trips
     for (int b = e0 + t; b < e1; b += U * nthreads) {
         float4 s[U], g[U];
@@ -288,12 +297,12 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
                 continue;
             }
             const size_t o = (size_t)m * p.N + n;
-            if (p.out_f32) {
+            if (SPLIT != kTailSplitRes && p.out_f32) {
                 *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C) + o) = make_float4(v[0], v[1], v[2], v[3]);
                 continue;
             }
             float r[4] = {0.f, 0.f, 0.f, 0.f};
-            if (p.residual) {
+            if (has_residual) {
                 const uint2 rr = *reinterpret_cast<const uint2*>(p.residual + o);
                 r[0] = bf16_bits_to_float(rr.x & 0xFFFFu);
                 r[1] = bf16_bits_to_float(rr.x >> 16);
@@ -305,15 +314,13 @@ __device__ __forceinline__ void reduce_split(const PairParams& p, unsigned int e
     }
 }
 
-// SPLIT: what the plan left to split by k.  An instantiation each, because the registers run out (96 a thread): with the code of
-// parts and reduction in one kernel every call paid for its spills, 0.5-1 us (149 x 5120 x 17408 35.7 -> 34.4 us, BF16 100 x 5120 x 5120
-// 19.1 -> 17.9), and whole items had none left to ask for the residual a chunk ahead (2048 x 5120 x 5120 with a residual 92 -> 83.4).
-enum Split { kWhole = 0, kAllSplit = 1, kTailSplit = 2 };
-
 template <int MODE, bool FINE, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_scale, const PairParams p) {
+    constexpr bool kTail = SPLIT == kTailSplit || SPLIT == kTailSplitRes;
+    const bool has_residual = SPLIT == kTailSplitRes || (SPLIT != kTailSplit && p.residual);
+    const bool swiglu_out = SPLIT != kTailSplitRes && p.swiglu_out, out_f32 = SPLIT != kTailSplitRes && p.out_f32;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const int xbytes = p.T / 2 * (XK * 2);                           // this CTA's T/2 tokens x 128 k, two blocks of 64 k
@@ -629,13 +636,13 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                 ptx::named_barrier_sync(1, 2 * kEpiWarps * 32);
             }
             const float* factor = s_factor;
-            const bool complete = SPLIT == kWhole || (SPLIT == kTailSplit && it.ks0 == 0 && it.ks1 == kstages);      // all split: no part is a whole tile
+            const bool complete = SPLIT == kWhole || (kTail && it.ks0 == 0 && it.ks1 == kstages);      // all split: no part is a whole tile
             const int which = it.ks0 == 0 ? 1 : 0;        // head of a tile (span end) or tail (span start)
             const bool two = it.rows == 2;
             // Both groups wait for and free both accumulators (accs is even: a pair never wraps).
             const int begin = two ? 0 : eg * (p.T / 2), end = two ? tokens : min(tokens, (eg + 1) * (p.T / 2));
             const int n = ((it.rt + (two ? eg : 0)) * 2 + rank) * TR + te;
-            if (p.residual && complete && n - lane < p.N) {    // its way from memory goes behind the MMAs: 64 bytes a token and warp into L2
+            if (has_residual && complete && n - lane < p.N) {    // its way from memory goes behind the MMAs: 64 bytes a token and warp into L2
                 const __nv_bfloat16* src = p.residual + (size_t)m0 * p.N;
                 for (int i = 2 * begin + lane; i < 2 * end; i += 32)
                     ptx::prefetch_l2(src + (size_t)(i >> 1) * p.N + min(n - lane + 16 * (i & 1), p.N - 1));
@@ -647,30 +654,36 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
 #pragma unroll
                 for (int i = 0; i < 16; ++i) res[i] = c0 + i < end ? src[(size_t)i * p.N] : (unsigned short)0;
             };
-            if (SPLIT == kWhole && p.residual && n < p.N) ask(begin);
+            if (SPLIT != kAllSplit && has_residual && complete && n < p.N) ask(begin);
             for (int i = t.i; i < t.i + 2; ++i) ptx::mbar_wait(&tfull[i], t.phase, s_abort, p.status, 0x470u + i);
             __syncwarp();
             tc_fence_after();
             {
                 const uint32_t t_addr = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)((t.i + (two ? eg : 0)) * p.T);
                 float* slot = p.partials + ((size_t)blockIdx.x * 2 + which) * kSlotFloats + te;
-                for (int c0 = begin; c0 < end; c0 += 16) {
-                    uint32_t v[16];
-                    __syncwarp();                  // lanes beyond the weight left the last chunk early
+                // The sums of sixteen tokens; called by the whole warp (lanes beyond the weight left the last chunk early).
+                auto sums = [&](int c0, uint32_t (&v)[16]) {
+                    __syncwarp();
                     tmem_ld16(t_addr + c0, v);
-                    if (!two) {
-                        uint32_t w[16];
-                        tmem_ld16(t_addr + p.T + c0, w);
+                    if (two) return;
+                    uint32_t w[16];
+                    tmem_ld16(t_addr + p.T + c0, w);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
-                    }
+                    for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(w[i]));
+                };
+                // A loop each for parts and for whole tiles: registers again.
+                for (int c0 = begin; SPLIT != kWhole && !complete && c0 < end; c0 += 16) {
+                    uint32_t v[16];
+                    sums(c0, v);
                     const int cnt = min(16, end - c0);
-                    if (!complete) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)           // [token][row]: a warp stores 128 contiguous bytes
-                            if (i < cnt) __stcg(slot + (c0 + i) * TR, __uint_as_float(v[i]));
-                        continue;
-                    }
+                    for (int i = 0; i < 16; ++i)           // [token][row]: a warp stores 128 contiguous bytes
+                        if (i < cnt) __stcg(slot + (c0 + i) * TR, __uint_as_float(v[i]));
+                }
+                for (int c0 = begin; SPLIT != kAllSplit && complete && c0 < end; c0 += 16) {
+                    uint32_t v[16];
+                    sums(c0, v);
+                    const int cnt = min(16, end - c0);
                     float f[16];
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
@@ -680,7 +693,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                         f[i + 2] = __uint_as_float(v[i + 2]) * k4.z;
                         f[i + 3] = __uint_as_float(v[i + 3]) * k4.w;
                     }
-                    if (p.swiglu_out) {
+                    if (swiglu_out) {
                         // A gate lane and its up lane (eight rows on) hold both halves of sixteen outputs: the gate lane finishes
                         // the first eight tokens, the up lane the others, one exchange and one SiLU each.
                         const int late = n & 8;
@@ -695,17 +708,16 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                     }
                     if (n >= p.N) continue;
                     const size_t o = (size_t)(m0 + c0) * p.N + n;
-                    if (p.out_f32) {
+                    if (out_f32) {
                         float* dst = reinterpret_cast<float*>(p.C) + o;
 #pragma unroll
                         for (int i = 0; i < 16; ++i) if (i < cnt) dst[(size_t)i * p.N] = f[i];
                         continue;
                     }
-                    if (p.residual) {
-                        if (SPLIT != kWhole) ask(c0);
+                    if (has_residual) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i) f[i] += bf16_bits_to_float(res[i]);
-                        if (SPLIT == kWhole && c0 + 16 < end) ask(c0 + 16);
+                        if (c0 + 16 < end) ask(c0 + 16);
                     }
                     __nv_bfloat16* dst = p.C + o;
                     if (cnt == 16) {
@@ -733,10 +745,10 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
             more = work.next(p, it);
             // Whole items follow the split ones: these warps reduce the split tiles they stored now, behind the MMAs
             // of the next items.  (With no whole items all warps do it at the end.)
-            if (SPLIT == kTailSplit && (pend[0] >= 0 || pend[1] >= 0) && (!more || it.sk < 0)) {
+            if (kTail && (pend[0] >= 0 || pend[1] >= 0) && (!more || it.sk < 0)) {
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
-                    if (pend[w] >= 0) reduce_split(p, epoch, pend[w], kstages, tt, 2 * kEpiWarps * 32, s_abort);
+                    if (pend[w] >= 0) reduce_split<SPLIT>(p, epoch, pend[w], kstages, tt, 2 * kEpiWarps * 32, s_abort);
                     pend[w] = -1;
                 }
             }
@@ -762,8 +774,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
         const long long u0 = (long long)id * units / pairs, u1 = (long long)(id + 1) * units / pairs;
         if (u0 < u1) {
             const int t0 = (int)(u0 / kstages), t1 = (int)((u1 - 1) / kstages);
-            if (u0 % kstages != 0 || u1 - u0 < kstages) reduce_split(p, epoch, t0, kstages, tid, kThreads, s_abort);
-            if (t1 != t0 && u1 - (long long)t1 * kstages < kstages) reduce_split(p, epoch, t1, kstages, tid, kThreads, s_abort);
+            if (u0 % kstages != 0 || u1 - u0 < kstages) reduce_split<SPLIT>(p, epoch, t0, kstages, tid, kThreads, s_abort);
+            if (t1 != t0 && u1 - (long long)t1 * kstages < kstages) reduce_split<SPLIT>(p, epoch, t1, kstages, tid, kThreads, s_abort);
         }
     }
 }
@@ -812,7 +824,8 @@ cudaError_t launch_split(const PairParams& p, int grid, int smem, const CUtensor
         if constexpr (MODE == kDense && !FINE) return cudaErrorInvalidValue;      // two row tiles an item: never split all over
         else return launch_as<MODE, FINE, kAllSplit>(p, grid, smem, tma, tmw, tms, s);
     }
-    return launch_as<MODE, FINE, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
+    return p.residual ? launch_as<MODE, FINE, kTailSplitRes>(p, grid, smem, tma, tmw, tms, s)
+                      : launch_as<MODE, FINE, kTailSplit>(p, grid, smem, tma, tmw, tms, s);
 }
 
 template <int MODE>
@@ -828,6 +841,7 @@ cudaError_t configure() {
     if constexpr (MODE != kDense || FINE)
         if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kAllSplit>, kSmemMax);
     if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kTailSplit>, kSmemMax);
+    if (e == cudaSuccess) e = configure_large_smem(prefill_pair_kernel<MODE, FINE, kTailSplitRes>, kSmemMax);
     return e;
 }
 

@@ -26,8 +26,8 @@ def test_warps_are_whole_at_tensor_memory_accesses(name):
         before = src[:at]
         whole = max(before.rfind("__syncwarp();"), before.rfind("WHOLE"))
         assert whole > max(before.rfind(f) for f in ("mbar_wait(", "mbar_test_wait(", "continue;", "elect_one("))
-        # a loop whose lanes may leave a turn early meets a __syncwarp() before the next turn's load
-        turn = re.search(r"for \(int c0 = (?:begin|0); c0 < (?:end|p\.NT); c0 \+= 16\) \{[^}]*$", before)
+        # a loop whose lanes may leave a turn early meets a __syncwarp() before the next turn's load; so does a function it calls
+        turn = re.search(r"(?:for \(int c0 = 0; c0 < p\.NT; c0 \+= 16\)|auto sums = \[&\]\([^{]*\)) \{[^}]*$", before)
         assert not turn or "__syncwarp();" in turn.group(0)
 
 
