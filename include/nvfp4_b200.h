@@ -103,7 +103,8 @@ const char* nvfp4_status_string(int status);
  *   "wide_gemv": 1 (default) = 9..16 tokens take one launch of the wide GEMV kernel (two
  *                   8-token MMA tiles, activations streamed with the weights); 0 = off
  *   "skinny_min_m", "skinny_max_m": token counts (default 9..80) routed to the few-token
- *                   kernel that keeps the dequantised weights in tensor memory; min 129 or
+ *                   kernel that keeps the dequantised weights in tensor memory (with the default
+ *                   limit, above 64 where it is ahead of the tcgen05 GEMM); min 129 or
  *                   max 0 turns it off.  "skinny_split_cost": stage-times charged to
  *                   splitting row tiles along K when that kernel plans its work.
  *   "prefill_stream_k": 1 (default) = output tiles left over after whole waves of tiles are

@@ -15,6 +15,8 @@
 
 using namespace nvfp4;
 
+constexpr int kSkinnyMaxDefault = 80;
+
 struct nvfp4_handle {
     nvfp4_device_info dev{};
     char* workspace = nullptr;
@@ -23,10 +25,8 @@ struct nvfp4_handle {
     int prefill_impl = 0;
     int decode_max_m = 16;
     int wide_gemv = 1;                           // 9..16 tokens: one launch of the wide GEMV kernel
-    // Token counts routed to the few-token kernel.  80: with the weights following the stream it is ahead of the prefill kernel on every
-    // shape measured at 65 and 80 tokens (34816 x 5120 38.4 -> 33.1 us, 5120 x 17408 31.6 -> 26.6, 7168 x 5120 20.8 -> 18.5, 2048 x 2048
-    // 10.9 -> 10.2), at 96 behind on some (5120 x 6144 20.0 -> 22.0).
-    int skinny_min_m = 9, skinny_max_m = 80;
+    // Token counts routed to the few-token kernel; from 65 on, with the default limit, where skinny_umma_ahead() says so.
+    int skinny_min_m = 9, skinny_max_m = kSkinnyMaxDefault;
     int fp4_native = 1;                          // the NVFP4 tensor-core GEMV (weights untouched, activations as NVFP4 terms) ...
     int fp4_min_m = 1;                           // ... from this token count on (up to 16)
     int fp4_stream_min_m = 10;                   // from this token count on its activations travel through the ring (decode_fp4_stream.cu)
@@ -173,9 +173,11 @@ int run_linear(nvfp4_handle* h, const LinearArgs& a, cudaStream_t s, size_t ws_b
         h->launches += (unsigned long long)nl;
         return cuda_status(e);
     }
-    // Above 64 tokens only by default: a caller who names the tcgen05 GEMM, or whole tiles, gets that kernel and what it refuses.
-    const bool prefill_named = a.M > 64 && (h->prefill_impl == 2 || !h->dev.prefill_stream_k);
-    if (fast_path_wanted && !prefill_named && a.M >= h->skinny_min_m && a.M <= h->skinny_max_m && skinny_umma_supported(a) &&
+    // Above 64 tokens only by default: a caller who names the tcgen05 GEMM, or whole tiles, gets that kernel and what it refuses.  A limit
+    // that the caller sets is taken as it is.
+    const bool to_prefill = a.M > 64 && (h->prefill_impl == 2 || !h->dev.prefill_stream_k ||
+                                         (h->skinny_max_m == kSkinnyMaxDefault && prefill_umma_supported(a) && !skinny_umma_ahead(a, h->dev)));
+    if (fast_path_wanted && !to_prefill && a.M >= h->skinny_min_m && a.M <= h->skinny_max_m && skinny_umma_supported(a) &&
         kDecodeScratchBytes + (a.M > 64 ? prefill_umma_scratch_bytes(a.M, a.N, a.K) : prefill_umma_reserved_bytes()) <= ws_bytes) {
         int nl = 0;
         cudaError_t e = launch_skinny_umma(a, h->dev, h->workspace, ws_bytes, kDecodeScratchBytes, &nl, s);

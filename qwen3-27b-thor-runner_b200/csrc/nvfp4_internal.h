@@ -196,6 +196,8 @@ cudaError_t launch_decode_wide(const LinearArgs& a, nvfp4_device_info& dev, void
 
 // --- skinny_umma.cu: 1 <= M <= 128, dequantised weights as the TMEM A operand of tcgen05.mma.
 bool skinny_umma_supported(const LinearArgs& a);
+// 65 to 80 tokens: whether it is ahead of the prefill kernel.
+bool skinny_umma_ahead(const LinearArgs& a, const nvfp4_device_info& dev);
 cudaError_t configure_skinny_umma();
 cudaError_t launch_skinny_umma(const LinearArgs& a, nvfp4_device_info& dev, void* scratch, size_t scratch_bytes,
                                size_t offset, int* launches, cudaStream_t s);

@@ -513,6 +513,19 @@ bool skinny_umma_supported(const LinearArgs& a) {
     return true;
 }
 
+// At 65 to 80 tokens tensor memory holds one item's accumulators: a CTA with parts of two row tiles drains the first before it sums the
+// second, and each tile of few rows on a long k is shared by many CTAs.  Behind the prefill kernel are few row tiles with a middling share of
+// stages a CTA (with it / here, us, 65 tokens: 640 x 17408 18.9 / 27.6, 2048 x 5120 14.4 / 17.0, 2048 x 4096 14.0 / 16.3, 5120 x 5120
+// 17.5 / 19.6, 6144 x 5120 18.4 / 20.8); ahead are tiles shared by three CTAs or fewer (7168 x 5120 19.3 / 18.2, 34816 x 5120 38.8 / 33.3),
+// long shares (5120 x 17408 30.7 / 27.9, 2560 x 17408 21.9 / 21.3), a stage a CTA (1024 x 4096 13.9 / 12.0, 512 x 5120 12.9 / 12.5) and
+// tiles of four CTAs on a short k (5120 x 3072 14.9 / 13.7).
+bool skinny_umma_ahead(const LinearArgs& a, const nvfp4_device_info& dev) {
+    const int grid = dev.sm_count < 160 ? dev.sm_count : 160;
+    const int tiles = (a.N + TR - 1) / TR, kstages = a.K / WK;
+    const long long units = (long long)tiles * kstages;
+    return 3LL * tiles >= grid || units >= 8LL * grid || units <= grid || (4LL * tiles >= grid && kstages <= 12);
+}
+
 cudaError_t configure_skinny_umma() {
     return configure_large_smem(skinny_umma_kernel, 1024 + kSmemBudget + 1536);
 }

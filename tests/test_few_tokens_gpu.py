@@ -17,6 +17,13 @@ def handle():
     h.close()
 
 
+@pytest.fixture
+def few(handle):
+    """65 to 80 tokens to this kernel whatever the shape."""
+    with util.options(handle, skinny_max_m=128):
+        yield handle
+
+
 @pytest.mark.parametrize("M,N,K,res", [
     (17, 128, 256, False),        # one stage: a unit for each issuer
     (33, 130, 512, True),         # two rows in the second tile, N % 4 != 0
@@ -27,8 +34,9 @@ def handle():
     (80, 19208, 768, False),      # the same with more tiles than CTAs, the last one cut
     (80, 640, 17408, True),       # deep split
 ])
-def test_against_the_oracle(handle, M, N, K, res):
+def test_against_the_oracle(few, M, N, K, res):
     import torch
+    handle = few
     packed, scale = util.make_weight(N, K, seed=M + N, sigma=0.14)
     A, R = util.make_bf16((M, K), seed=M), util.make_bf16((M, N), seed=N)
     dA, dP, dS = util.to_dev(A), util.to_dev(packed), util.to_dev(scale)
@@ -46,10 +54,11 @@ def test_against_the_oracle(handle, M, N, K, res):
 
 @pytest.mark.parametrize("writer", ["linear", "swiglu"])
 @pytest.mark.parametrize("M", [65, 80])
-def test_weights_follow_a_kernel_that_lets_its_successor_start(handle, M, writer):
+def test_weights_follow_a_kernel_that_lets_its_successor_start(few, M, writer):
     """The codes are the BF16 output of a library call right before, which leaves most SMs idle and lets its successor start early
     (SwiGLU at its first instruction); a copy, as below, never does.  The bits of the synchronised sequence."""
     import torch
+    handle = few
     N, K = 2048, 1024                                    # N * K / 2 bytes of codes: an output of [T, 256]
     T, K1 = 2048, 2560
     A, A1 = util.to_dev(util.make_bf16((M, K), seed=M)), util.to_dev(util.make_bf16((T, K1), seed=M + 1))
@@ -82,9 +91,10 @@ def test_weights_follow_a_kernel_that_lets_its_successor_start(handle, M, writer
 
 
 @pytest.mark.parametrize("M", [65, 80])
-def test_weights_follow_the_stream_beyond_64_tokens(handle, M):
+def test_weights_follow_the_stream_beyond_64_tokens(few, M):
     """A weight copied into place right before the call, on the same stream, is the one that is used."""
     import torch
+    handle = few
     N, K = 4096, 2048
     sets = [tuple(util.to_dev(a) for a in util.make_weight(N, K, seed=s)) for s in (1, 2)]
     A = util.to_dev(util.make_bf16((M, K), seed=3))
@@ -147,3 +157,29 @@ def test_options_that_name_the_prefill_kernel_reach_it(handle, M, option, value)
     if option == "prefill_impl":
         with util.options(handle, prefill_impl=value), pytest.raises(nvfp4.Nvfp4Error, match="shape"):
             handle.linear(A, M, p, s, 1.0, N - 1, K, torch.zeros((M, N - 1), dtype=torch.int16, device="cuda"))
+
+
+@pytest.mark.parametrize("N,K,here", [
+    (6272, 5120, False), (6400, 5120, True),             # 49 and 50 row tiles on 148 CTAs: the latter three CTAs a tile or fewer
+    (640, 17408, False), (2048, 5120, False), (640, 5120, True),      # 2.3, 2.2 and less than one stage a CTA
+    (4736, 3072, True), (4608, 3072, False), (4736, 3328, False),     # four CTAs a tile, or a few more; twelve stages, thirteen
+    (4096, 9472, True), (4096, 9216, False),             # eight stages a CTA
+])
+def test_route_at_65_tokens(handle, N, K, here):
+    """Which kernel takes the call, by its bits: the limit of 128 names this kernel, 0 the prefill kernel."""
+    import torch
+    M = 65
+    if handle.get_option("sm_count") != 148:
+        pytest.skip("shapes chosen for 148 SMs")
+    p, s = (util.to_dev(a) for a in util.make_weight(N, K, seed=M))
+    A = util.to_dev(util.make_bf16((M, K), seed=M + 1))
+
+    def call(**settings):
+        C = torch.zeros((M, N), dtype=torch.bfloat16, device="cuda")
+        with util.options(handle, **settings):
+            handle.linear(A, M, p, s, 1.0, N, K, C)
+        return C
+
+    mine, other = call(skinny_max_m=128), call(skinny_max_m=0)
+    assert not torch.equal(mine, other)
+    assert torch.equal(call(), mine if here else other)
