@@ -76,8 +76,9 @@ __device__ __forceinline__ uint32_t absmax_bf16x8(uint4 x) {
 // Columns beyond tokens x terms are never written: whatever an earlier call left there only reaches
 // accumulator columns the GEMV's epilogue does not read (stale codes and scales are finite).
 //
-// Row loads a thread has in flight: 9 take 18432 columns in one trip (with 4 a row of 17408 took three), as many as leave the
-// CTA room beside a GEMV's.  SwiGLU and RMSNorm load a second vector with each.
+// Row loads a thread asks for in a turn: 9 cover 18432 columns (with 4 a row of 17408 took three turns, each behind the maximum of the
+// one before).  They are not all in flight together: the plain and the norm form compile to 32 registers, of which nine loads would
+// take 36, so they go out in batches.  SwiGLU and RMSNorm load a second vector with each.
 template <int TERMS, int MODE>
 __global__ void __launch_bounds__(kPreThreads)
 act_to_fp4_kernel(const ActParams p) {

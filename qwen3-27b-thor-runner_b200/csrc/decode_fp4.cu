@@ -236,7 +236,7 @@ decode_fp4_kernel(const __grid_constant__ CUtensorMap tm_packed, const __grid_co
                 *reinterpret_cast<uint16_t*>(row0 + col * 128 + (((bl >> 1) ^ (col & 7)) << 4) + (bl & 1) * 8 + part * 2) = (uint16_t)w;
                 if (part == 0) sf0[(col & 31) * 16] = (uint8_t)ue4m3_pow2(pw);
             }
-            }
+        }
         ptx::fence_proxy_async_smem();                        // the tensor core reads the codes through the asynchronous proxy
         ptx::named_barrier_sync(2, kOwnThreads);
         if (tq == 0) {

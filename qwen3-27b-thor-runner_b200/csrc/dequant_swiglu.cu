@@ -159,7 +159,7 @@ namespace {
 // came as, and reads the row again beyond that.  1/sqrtf and a true division, not the fast-math forms.
 // Bound by latency: a launch, one trip to memory, two barriers.  So all loads (without a bias the weight's too) go out before the
 // first use, the kernel starts while the one before it finishes and lets the one behind it do the same; for that a CTA has to
-// fit beside a persistent GEMV's (123 registers x 384 threads), hence at most 64 registers.
+// fit beside a persistent GEMV's (128 registers x 384 threads), hence at most 64 registers, at 20 (8 with a bias) bytes of spills.
 constexpr int kNormThreads = 256;
 constexpr int kNormCache = 4, kNormBiasCache = 3;   // x 256 threads x 8 elements: 8192 (6144 with a bias) columns from registers
 

@@ -84,7 +84,10 @@ __device__ __forceinline__ void fp4_publish(const float (&v)[KTOK], unsigned cha
         if (g * kQuadTokens >= M) break;
         uint32_t w[kQuadTokens];
 #pragma unroll
-        for (int i = 0; i < kQuadTokens; ++i) w[i] = g * kQuadTokens + i < KTOK ? __float_as_uint(v[g * kQuadTokens + i < KTOK ? g * kQuadTokens + i : 0]) : tag;
+        for (int i = 0; i < kQuadTokens; ++i) {
+            const int m = g * kQuadTokens + i;
+            w[i] = m < KTOK ? __float_as_uint(v[m < KTOK ? m : 0]) : tag;
+        }
         ptx::st_relaxed_b128(slot + (g * 128 + te) * 16, w[0], w[1], w[2], tag);
     }
 }
@@ -139,9 +142,10 @@ __device__ __forceinline__ bool fp4_gather_block(float (&v)[KTOK], const unsigne
 
 // Adds to v the FP32 partial sums the CTAs first .. last published for this row tile (slot_bytes per CTA), in CTA order per
 // token (a fixed summation order).  Each trip to L2 costs the owner ~0.7 us at the end of its call, so as many accesses travel
-// together as the registers hold: eight with nine tokens, twelve with sixteen.  {value, tag} pairs before, sixteen accesses a trip and
-// four trips for two contributors of sixteen tokens: 7168 x 5120 at 16 tokens 12.7 -> 10.0 us, 5120 x 17408 18.9 -> 16.4 (with the
-// stores above), 5120 x 6144 at 12 12.0 -> 10.1; two decode layers of sixteen tokens 159.5 -> 140.4, of four 120.8 -> 118.3.
+// together as the registers hold: up to 3 / 6 / 9 tokens four of one group / eight of two / six of three, in the sixteen-token kernel above
+// six tokens twelve of six.  {value, tag} pairs before, sixteen accesses a trip and four trips for two contributors of sixteen
+// tokens: 7168 x 5120 at 16 tokens 12.7 -> 10.0 us, 5120 x 17408 18.9 -> 16.4 (with the stores above), 5120 x 6144 at 12 12.0 -> 10.1;
+// two decode layers of sixteen tokens 159.5 -> 140.4, of four 120.8 -> 118.3.
 template <int KTOK>
 __device__ __forceinline__ bool fp4_gather(float (&v)[KTOK], const unsigned char* pairs, size_t slot_bytes, int first, int last,
                                            int M, int te, unsigned int tag, volatile int* abort_flag, unsigned int* status,

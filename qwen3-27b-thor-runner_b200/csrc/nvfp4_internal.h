@@ -59,7 +59,8 @@ struct nvfp4_device_info {
     int cc_major, cc_minor;
     size_t smem_optin;
     int prefill_stream_k = 1;    // split the tiles left after whole waves by k over all CTAs
-    int skinny_split_cost = 12;  // stage-times charged to splitting row tiles by k in the few-token kernel
+    int skinny_split_cost = 12;  // stage-times charged to splitting row tiles by k in the few-token kernel; set when a stage took 1650
+                                 // clocks (920 now) and the reduction read one element at a time (four now), not fitted again since
     int fp4_own_quant = 1;       // one or two tokens: the tensor-core GEMV expands its activations itself, no pre-pass launch
     size_t gemv_pairs_offset = 6u << 20;   // where the 8-token GEMV's {value, epoch} partial pairs start in its scratch
     int max_pairs = 0;                     // CTA pairs of the prefill kernel the device can hold at once (set at creation)

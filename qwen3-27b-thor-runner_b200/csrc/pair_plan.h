@@ -120,7 +120,9 @@ NVFP4_HD void participants(const Plan& p, int kstages, int pairs, int id, int ti
     while (last + 1 < pairs && (long long)(last + 1) * units / pairs < e) ++last;
 }
 
-// Clocks, fitted to the times of all plans for each weight form alone.
+// Clocks, fitted to the times of all plans for each weight form alone, with the kernel as it was when its groups of dequantising warps took
+// a half of every unit: an MMA took 100 to 120 clocks then and takes 75 (T = 128), 81 (160) or 110 (192) now, and drains and parts
+// cost less.  They were not fitted again since; how far the plans they choose are from the best ones today has not been measured.
 struct Prices {
     double mma;            // one MMA at least (alone 65: the issuing warps share their schedulers with the dequantising ones)
     double rate;           // bytes a clock of both operand streams of an SM
@@ -140,15 +142,15 @@ constexpr Prices kPricesBf16 = {73.5, 68.0, 16384.0, 6.2, 18.8, 1060.0, 7900.0, 
 inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem, const Prices* prices = nullptr) {
     const int kst = p.K / WK;
     p.row_tiles = (p.N + 2 * TR - 1) / (2 * TR);
-    // T up to 192: two accumulators and two 64-column A units (four of 64 k in the kernel) fill tensor memory.  BF16 weights: up to 224, four 32 KB A units
-    // and three token stages; from 192 on only with two row tiles an item (one row tile takes two token stages a turn: 512 x 5120
-    // x 8192 at T = 192 64 us, at T = 128 40) and never split all over.
+    // T up to 192: two accumulators and two 64-column A units (four of 64 k in the kernel) fill tensor memory.  BF16 weights: up to 224,
+    // four 32 KB A units and three token stages; from 192 on only with two row tiles an item (one row tile takes two token stages a
+    // turn: 512 x 5120 x 8192 at T = 192 64 us, at T = 128 40) and never split all over.
     const int t_max = dense ? 224 : 192;
     // Every plan -- T, row tiles per item (R), items left over after whole waves run whole or split by k -- is priced in clocks,
     // with constants fitted to all plans of some 300 shapes of each weight form (17 to 2048 tokens, N 512 to 34816, K 1024 to
-    // 17408, weights from memory): the plan chosen is 0.2 (BF16 1.0) % slower than the best one on average, 1.4 (5.6) at the 95th
-    // percentile.  The list before it was fitted to large weights only, charged 23,500 clocks for any split and had none for
-    // fewer stages than pairs: 65 x 512 x 5120 ran whole in 25 us, 14 split.
+    // 17408, weights from memory): the plan chosen was 0.2 (BF16 1.0) % slower than the best one on average, 1.4 (5.6) at the 95th
+    // percentile, for the kernel they were fitted to.  The list before it was fitted to large weights only, charged 23,500 clocks for
+    // any split and had none for fewer stages than pairs: 65 x 512 x 5120 ran whole in 25 us, 14 split.
     const Prices& c = prices ? *prices : dense ? kPricesBf16 : kPricesFp4;
     double best = 1e30;
     int used = 1;
@@ -159,7 +161,8 @@ inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem, c
             const long long items = (long long)((p.row_tiles + R - 1) / R) * mt;
             // clocks of one 64-k block of an item, of one row tile: the MMAs, or the bytes of both streams
             const double mma = 4.0 * (T / 2 > c.mma ? T / 2 : c.mma);
-            const double blk = std::fmax(R * mma, (T * 64.0 + R * c.block_bytes) / c.rate), blk1 = std::fmax(mma, (T * 64.0 + c.block_bytes) / c.rate);
+            const double blk = std::fmax(R * mma, (T * 64.0 + R * c.block_bytes) / c.rate);
+            const double blk1 = std::fmax(mma, (T * 64.0 + c.block_bytes) / c.rate);
             const long long full = items / pairs, left = items % pairs, sk = left * R;
             const double item = kst * kBlocks * blk + c.item_token * tokens * R + c.item;
             auto take = [&](double cost, bool split, long long on) {
@@ -197,7 +200,8 @@ inline int make_plan(Plan& p, int pairs, bool stream_k, bool dense, int* smem, c
             }
             const long long on = sk * kst < pairs ? sk * kst : pairs;
             if ((sk * kst + on - 1) / on < kst)                    // no part is a whole tile: the kernel for plans split all over has none
-                take((double)((sk * kst + on - 1) / on) * kBlocks * blk1 + c.split + 2.0 * c.split_token * tokens + c.part * on / sk + c.straddle + c.pair * on,
+                take((double)((sk * kst + on - 1) / on) * kBlocks * blk1 + c.split + 2.0 * c.split_token * tokens + c.part * on / sk +
+                         c.straddle + c.pair * on,
                      true, on);
         }
     }

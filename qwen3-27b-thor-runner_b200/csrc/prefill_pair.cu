@@ -25,9 +25,10 @@
 // units of 64 k, and commits reach both CTAs' barriers themselves (a warp that passed them on came 200 clocks later).  Issuers at
 // T = 128 / 160 / 192: 100 / 100 / 120 clocks an MMA -> 75 / 81 / 110.  What bounds it now is the issue of the MMAs for T <= 128, the way
 // around the A ring at T = 192, draining the accumulators (5-8 thousand clocks an item), and the power cap for long runs.
-// Measured, before -> now, pre-pass included, weights from memory, calls back to back in short bursts: 34816 x 5120 at 100 / 149 / 256 /
-// 512 / 1111 / 2048 tokens 43.7 -> 38.8, 46.5 -> 43.8, 78.1 -> 70.5, 136 -> 133, 274 -> 266, 497 -> 483 us; 5120 x 17408 with a residual at
-// 100 / 256 / 1111 34.7 -> 32.4, 54.9 -> 51.2, 149 -> 143; BF16 5120 x 5120 at 512 34.7 -> 30.3 (two warps stream its blocks).
+// Measured, before whole units in turn -> now, pre-pass included, weights from memory, calls back to back in short bursts on one box:
+// 34816 x 5120 at 100 / 149 / 256 / 512 / 1111 / 2048 tokens 50.2 -> 45.2, 54.6 -> 49.8, 90.5 -> 80.8, 151 -> 146, 282 -> 267, 497 -> 476 us;
+// 5120 x 17408 with a residual at 149 / 256 / 1111 40.3 -> 37.5, 59.7 -> 54.2, 165 -> 146; BF16 5120 x 5120 at 100 / 512 20.3 -> 19.2,
+// 37.4 -> 32.6, 34816 x 5120 at 4096 1107 -> 1054, with a residual 1247 -> 1123.
 //
 // Operands are FP16 because the hardware E2M1 conversion produces FP16 and every e2m1 x ue4m3 product is exact in FP16
 // (kind::f16 takes both operands in ONE 16-bit format).  A pre-pass turns the BF16 activations into FP16 with an exact
@@ -92,16 +93,18 @@ struct Ring {
 };
 
 // ---------------------------------------------------------------- tcgen05, CTA pairs
-// The MMAs of a unit on one accumulator, which the first clears when `accumulate` is 0, from one elected lane of a converged
-// warp: eight (128 k, B in two blocks `step` 16-byte units apart) or the four of one block (64 k).  A from tensor memory (8 columns
-// per MMA) or from shared memory (two blocks 16 KB apart, or one).  Election and address arithmetic sit inside one asm block: the issuing warp shares its scheduler
-// and instruction cache with the dequantising warps, and every instruction of its loop counts.
+// The MMAs of a unit on one accumulator, which the first clears when `accumulate` is 0, from one elected lane of a converged warp: eight
+// (128 k, B in two blocks `step` 16-byte units apart) or the four of one block (64 k).  A from tensor memory (8 columns per MMA) or from
+// shared memory (two blocks 16 KB apart, or one).  Election and address arithmetic sit inside one asm block: the issuing warp
+// shares its scheduler and instruction cache with the dequantising warps, and every instruction of its loop counts.
 __device__ __forceinline__ void mma8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t step, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a1, a2, a3, a4, a5, a6, a7;\n\t.reg .b64 s, b1, b2, b3, b4, b5, b6, b7;\n\t"
         "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tcvt.u64.u32 s, %5;\n\t"
-        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\tadd.u32 a4, %1, 32;\n\tadd.u32 a5, %1, 40;\n\tadd.u32 a6, %1, 48;\n\tadd.u32 a7, %1, 56;\n\t"
-        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\tadd.u64 b4, %2, s;\n\tadd.u64 b5, b4, 2;\n\tadd.u64 b6, b4, 4;\n\tadd.u64 b7, b4, 6;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\tadd.u32 a4, %1, 32;\n\t"
+        "add.u32 a5, %1, 40;\n\tadd.u32 a6, %1, 48;\n\tadd.u32 a7, %1, 56;\n\t"
+        "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\tadd.u64 b4, %2, s;\n\t"
+        "add.u64 b5, b4, 2;\n\tadd.u64 b6, b4, 4;\n\tadd.u64 b7, b4, 6;\n\t"
         "elect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, t;\n\t"
@@ -493,7 +496,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_con
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint64_t xdesc = umma_desc_sw128(x0 + (uint32_t)(pairwise && me ? y.i : x.i) * xbytes + (second || (FINE && one && me) ? xhalf : 0u));
+                    const uint32_t xstage = x0 + (uint32_t)(pairwise && me ? y.i : x.i) * xbytes;
+                    const uint64_t xdesc = umma_desc_sw128(xstage + (second || (FINE && one && me) ? xhalf : 0u));
                     const uint64_t wdesc = umma_desc_sw128(ptx::smem_u32(s_w) + (uint32_t)u.i * kLoadBytes);
                     if (MODE == kDense && FINE) mma4_ss(d, wdesc, xdesc, p.idesc, (uint32_t)turn);
                     else if (MODE == kDense) mma8_ss(d, wdesc, xdesc, xhalf >> 4, p.idesc, (uint32_t)turn);

@@ -60,7 +60,7 @@ using namespace umma;
 constexpr int TR = 128;            // weight rows per tile (UMMA M = TMEM lanes)
 constexpr int BK = 64;             // k per activation operand block (128 bytes of BF16)
 constexpr int WK = 256;            // k per stage
-constexpr int kMaxTokens = 128;    // UMMA N <= 128 here: two accumulators + the A ring = 512 TMEM columns
+constexpr int kMaxTokens = 128;    // UMMA N <= 128 here: two accumulators an item + the A ring = 512 TMEM columns
 constexpr int kWPackedBytes = TR * WK / 2;     // 16 KB
 constexpr int kWScaleBytes = TR * WK / 16;     // 2 KB
 constexpr int kMaxWStages = 8, kMaxXStages = 4, kMaxAUnits = 4, kMaxItems = 2;
