@@ -53,6 +53,7 @@ struct DenseParams {
     int units, kchunks;       // units in all, units per row tile
     int stages;
     int act_slots, act_all;   // resident activation slots (units of 128 k); 1 = slot index is the k-chunk
+    int ahead;                // the call is one launch
     unsigned int epoch;
 };
 
@@ -92,13 +93,21 @@ dense_gemv_kernel(const __grid_constant__ CUtensorMap tm_w, const DenseParams p)
         if (lane == 0) {
             ptx::prefetch_tensormap(&tm_w);
             // W follows the stream.  A kernel before this one may trigger its dependents at its first instruction (RMSNorm and SwiGLU do),
-            // so without this wait the loads could run beside whatever writes W, two kernels back or more.  Calls back to back pay for
-            // it: 2048 x 2048 at one token 6.7 -> 7.6 us, 16384 x 5120 26.0 -> 27.5, a head of 248320 x 5120 none of 355.
+            // so without this wait the loads could run beside whatever writes W, two kernels back or more.  Calls back to back paid
+            // for it: 2048 x 2048 at one token 6.7 -> 7.6 us, 5120 x 5120 10.9 -> 11.9, 16384 x 5120 26.4 -> 27.9.  What the ring takes
+            // first is therefore asked for into L2 in front of the wait, where it costs no ordering: a write that comes later meets
+            // it there.  6.9, 10.6, 26.5; a head of 248320 x 5120 364 -> 361.  Not for 9 to 16 tokens, whose second launch reads the
+            // weight from L2, where the next call's request would displace it (5120 x 5120 at 16 20.8, with it 21.7).
+            int tile = u_begin / p.kchunks, kc = kc_begin;
+            for (int i = 0, t = tile, k = kc; p.ahead && i < stages && u_begin + i < u_end; ++i) {
+                ptx::tma_prefetch_l2_2d(&tm_w, k * kUK, t * kRT);
+                ptx::tma_prefetch_l2_2d(&tm_w, k * kUK + 64, t * kRT);
+                if (++k == p.kchunks) { k = 0; ++t; }
+            }
             ptx::griddep_wait();
             const uint64_t pol = ptx::policy_evict_first();
             int stage = 0;
             uint32_t ph = 0;
-            int tile = u_begin / p.kchunks, kc = kc_begin;
             for (int u = u_begin; u < u_end; ++u) {
                 ptx::mbar_wait(&empty_bar[stage], ph ^ 1u, s_abort, status, 0x800u + (unsigned)stage);
                 ptx::mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)kUnitBytes);
@@ -349,6 +358,7 @@ cudaError_t launch_dense_gemv(const DenseArgs& a, nvfp4_device_info& dev, void* 
         if (a.residual) b.residual = static_cast<const char*>(a.residual) + (size_t)m0 * a.N * 2;
         DensePlan pl;
         if (!plan_dense(b, m, dev, scratch, &pl)) return cudaErrorInvalidValue;
+        pl.p.ahead = a.M <= per ? 1 : 0;
         pl.p.epoch = next_launch_tag();
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(pl.grid);
